@@ -11,29 +11,59 @@
 
 namespace fpp {
 
+int ozaki_split(OzakiOperand &op, int rows, int K, const double *X, long long ldx,
+                cudaStream_t st) {
+  const OzakiShape sh = ozaki_shape(rows, K);
+  FPP_TRY(op.planes.reserve(std::max<size_t>(sh.plane_bytes, 16)));
+  FPP_TRY(op.exps.reserve(sizeof(int) * std::max(rows, 1)));
+  op.rows = rows;
+  op.K = K;
+  if (launch_ozaki_split(rows, K, X, ldx, op.planes.as<__half>(), op.exps.as<int>(), st) != 0)
+    return fail(FPP_ERR_CUDA, "digit-plane split launch failed");
+  return FPP_OK;
+}
+
+int ozaki_const(OzakiOperand &op, int rows, int K, const double *X, long long ldx,
+                cudaStream_t st) {
+  if (op.ready && op.rows == rows && op.K == K) return FPP_OK;
+  op.ready = false;
+  FPP_TRY(ozaki_split(op, rows, K, X, ldx, st));
+  FPP_CUDA(cudaStreamSynchronize(st));  // later calls may run on other streams
+  op.ready = true;
+  return FPP_OK;
+}
+
+OzakiMat ozaki_mat(const OzakiOperand &op) {
+  return OzakiMat{op.planes.as<__half>(), op.exps.as<int>(), op.rows, op.K};
+}
+
+int ozaki_run(const OzakiProblem *probs, int n, DeviceStatus *status, cudaStream_t st) {
+  const int rc = launch_ozaki_gemm(probs, n, status, st);
+  if (rc != 0) return fail(FPP_ERR_CUDA, "tensor-core FP64 GEMM launch failed (" +
+                                             std::to_string(rc) + ")");
+  return FPP_OK;
+}
+
+int ozaki_status(OzakiWork &w, cudaStream_t st, DeviceStatus **out) {
+  if (w.status.bytes < sizeof(DeviceStatus)) {  // cleared once, then by each check
+    FPP_TRY(w.status.reserve(sizeof(DeviceStatus)));
+    FPP_CUDA(cudaMemsetAsync(w.status.ptr, 0, sizeof(DeviceStatus), st));
+  }
+  *out = w.status.as<DeviceStatus>();
+  return FPP_OK;
+}
+
 int ozaki_dgemm_nt(int M, int N, int K, const double *A, long long lda, const double *B,
                    long long ldb, double *C, long long ldc, OzakiWork &w, cudaStream_t st,
                    bool b_lower) {
   if (M <= 0 || N <= 0) return FPP_OK;
   if (K <= 0) return fail(FPP_ERR_INVALID, "GEMM with K <= 0");
-  const OzakiShape sa = ozaki_shape(M, K), sb = ozaki_shape(N, K);
-  FPP_TRY(w.a.reserve(sa.plane_bytes));
-  FPP_TRY(w.b.reserve(sb.plane_bytes));
-  FPP_TRY(w.pa.reserve(sizeof(double) * M));
-  FPP_TRY(w.pb.reserve(sizeof(double) * N));
-  if (w.status.bytes < sizeof(DeviceStatus)) {  // cleared once, then by each check
-    FPP_TRY(w.status.reserve(sizeof(DeviceStatus)));
-    FPP_CUDA(cudaMemsetAsync(w.status.ptr, 0, sizeof(DeviceStatus), st));
-  }
-  if (launch_ozaki_split(M, K, A, lda, w.a.as<__half>(), w.pa.as<double>(), st) != 0 ||
-      launch_ozaki_split(N, K, B, ldb, w.b.as<__half>(), w.pb.as<double>(), st) != 0)
-    return fail(FPP_ERR_CUDA, "digit-plane split launch failed");
-  const int rc = launch_ozaki_gemm(M, N, K, w.a.as<__half>(), w.pa.as<double>(),
-                                   w.b.as<__half>(), w.pb.as<double>(), C, ldc,
-                                   w.status.as<DeviceStatus>(), st, b_lower);
-  if (rc != 0) return fail(FPP_ERR_CUDA, "tensor-core FP64 GEMM launch failed (" +
-                                             std::to_string(rc) + ")");
-  return FPP_OK;
+  DeviceStatus *status;
+  FPP_TRY(ozaki_status(w, st, &status));
+  FPP_TRY(ozaki_split(w.a, M, K, A, lda, st));
+  FPP_TRY(ozaki_split(w.b, N, K, B, ldb, st));
+  const OzakiProblem q{ozaki_mat(w.a), ozaki_mat(w.b), 0, M, N, C, ldc, b_lower};
+  return ozaki_run(&q, 1, status, st);
 }
 
 int ozaki_check_status(OzakiWork &w, cudaStream_t st) {

@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "b2_kernels.h"
+#include "gemm_ozaki.h"
 #include "internal.h"
 
 struct fpp_structure {
@@ -125,4 +126,15 @@ int ozaki_dgemm_nt(int M, int N, int K, const double *A, long long lda, const do
                    long long ldb, double *C, long long ldc, OzakiWork &w, cudaStream_t st,
                    bool b_lower = false);
 int ozaki_check_status(OzakiWork &w, cudaStream_t st);
+// The steps of it: digit planes of a matrix (rows x K, row stride ldx), the
+// same for a constant of a model (split once; ready is reset where the matrix
+// changes), and several products in one launch.
+int ozaki_split(OzakiOperand &op, int rows, int K, const double *X, long long ldx,
+                cudaStream_t st);
+int ozaki_const(OzakiOperand &op, int rows, int K, const double *X, long long ldx,
+                cudaStream_t st);
+OzakiMat ozaki_mat(const OzakiOperand &op);
+int ozaki_run(const OzakiProblem *probs, int n, DeviceStatus *status, cudaStream_t st);
+// the workspace's status word, allocated and cleared on first use
+int ozaki_status(OzakiWork &w, cudaStream_t st, DeviceStatus **out);
 }  // namespace fpp

@@ -3,30 +3,53 @@
 // "Error-free transformations of matrix multiplication by using fast routines
 // of matrix multiplication and its applications", Numer. Algorithms 59, 2012).
 //
-// Each row of A (and of B) is scaled by a power of two 2^e so that its
-// entries lie in (-1, 1), then cut into kOzakiDigits signed digits of
-// kOzakiBits bits:  a = 2^e sum_s d_s 2^(-5 (s + 1)),  |d_s| <= 31,
-// which fp16 holds exactly.  For one pair of digit planes (s, t) the products
-// d_s d_t are integers of at most 961 and a K-sum of them stays an integer; all
-// the pairs of one level L = s + t summed over at most kOzakiChunkK columns
-// stay below 11 * 1536 * 961 < 2^24, so the FP32 TMEM accumulator holds them
-// EXACTLY whatever order or truncation the tensor cores use.  The epilogue
-// adds each level into C in FP64:
-//   C = 2^(e_a + e_b) sum_{L <= 10} 2^(-5 (L + 2)) (sum_{s + t = L} A_s B_t^T),
-// which keeps about 55 bits of every operand relative to its row's largest
-// entry (the pairs of levels 11 and above, dropped, weigh below 2^-55 of it).
+// Each row of A (and of B) is scaled by a power of two 2^(e + 1) so that its
+// entries lie in (-1/2, 1/2), then cut into kOzakiDigits balanced digits of
+// kOzakiBits bits:  a = 2^(e + 1) sum_s d_s 2^(-7 (s + 1)),  |d_s| <= 64, which
+// fp16 holds exactly.  For one pair of digit planes (s, t) the products
+// d_s d_t are integers of at most 2^12 and a K-sum of them stays an integer;
+// the pairs of one level L = s + t (at most 8) summed over a chunk of columns (512
+// for 8 pairs, more for fewer) stay within 8 * 512 * 2^12 = 2^24, so the FP32 TMEM
+// accumulator holds them EXACTLY whatever order or truncation the tensor cores
+// use.  Groups of four levels L0..L1 are then added exactly in 64-bit integers,
+//   G = sum_{L0 <= L <= L1} 2^(7 (L1 - L)) S_L,   weight 2^(-14 - 7 L1),
+// and the groups, lowest first, by one FP64 multiply-add each.  The operands keep
+// 55 bits relative to their row's largest entry, rounded to nearest.  With levels
+// 0..7 (36 pairs) the dropped pairs are the largest error, about 2^-55 sqrt(K) of
+// the row maxima's product (the digits being balanced they have no common sign);
+// with level 8 too (43 pairs) they are below the operands' rounding.
 //
-// Kernel layout (one persistent CTA per SM, 320 threads):
-//   warp 0 lane 0  TMA producer: 128B-swizzled 128 x 64 tiles of the A and B
-//                  digit planes into a 6-stage ring
-//   warp 1 lane 0  MMA issuer: per unit (tile, level, K chunk) the pairs of
-//                  the level into one 128-column TMEM accumulator; four
-//                  accumulators rotate between units
-//   warps 2-9      epilogue: two warps per TMEM lane quarter, each owning 64
-//                  columns of its 32 rows: tcgen05.ld, then the level times
-//                  2^(-5 (L + 2)) added to FP64 sums held in registers for the
-//                  whole tile; after the last level the row and column powers
-//                  of two are applied and the tile is stored once
+// Eleven truncated 5-bit digits held the same bits with 66 pairs instead of 36
+// (their level sums could run over 1536 columns, which FP64 epilogue sums need:
+// FP64 issues 2 per clock and SM; the integer ones do not).
+//
+// What bounds it: shared memory.  An N = 128 MMA takes 64 cycles and reads 8 KB, all
+// of the SM's 128 bytes per cycle, and TMA writes there too.  So
+//  - a K block's digit tiles are loaded once per group of levels and used in all its
+//    pairs: the pairs of levels L0..L1 run by ascending A digit s, whose partners
+//    t = L0-s .. L1-s are a window sliding down the B digits; A tiles live one step,
+//    B tiles four or five (24 tile loads feed 36 pairs; one A and one B tile per
+//    pair before);
+//  - two neighboring partners make one N = 256 MMA, which reads A once.
+// The issuing thread comes next: its loops are unrolled per group (376 cycles per
+// pair with the slots worked out at run time, where the pair's MMAs take 256) and
+// its tcgen05 instructions stand under elect.sync.  Measured at 4096 x 2048 x 1500:
+// 13.8 TFLOP/s FP64-equivalent with the 5-bit digits, 17.7 with these and run-time
+// slots, 26.6 unrolled, 28.9 with elect.sync and N = 256, 34.2 with integer group
+// sums in place of FP64 conversions and 32-byte accesses to C (36 pairs, one
+// launch; the MMAs alone would take 52).
+//
+// Kernel layout (one persistent CTA per SM, 576 threads):
+//   warp 0 lane 0  TMA producer: 128B-swizzled 128 x 64 digit tiles into two
+//                  rings (A: 6 slots, B: 8 slots)
+//   warp 1         MMA issuer (one elected lane): per unit (tile, group of
+//                  levels, K chunk) the pairs of its four levels into four
+//                  128-column accumulators (all of TMEM); a level is handed to the epilogue as soon as
+//                  its last pair of the chunk is issued
+//   warps 2-17     epilogue: four warps per TMEM lane quarter, each owning 32
+//                  columns of its 32 rows: tcgen05.ld, then the level's integer
+//                  into 64-bit sums held in registers over all chunks.  The
+//                  lowest group comes first; its sum waits in C.
 // Every wait is bounded; a wait that runs out records FPP_ERR_TIMEOUT in the
 // status word and the CTA skips to its exit.
 #include <cuda.h>
@@ -44,31 +67,143 @@
 namespace fpp {
 
 namespace {
-constexpr int OBM = 128, OBN = 128, OBK = kTmaBoxK, OSTAGES = 6;
-constexpr int OA_TILE = OBM * OBK * 2, OB_TILE = OBN * OBK * 2;
-constexpr int OSTAGE_BYTES = OA_TILE + OB_TILE;
-constexpr int OACC = 4;                 // TMEM accumulators (units in flight)
-constexpr int OTMEM_COLS = OACC * OBN;
-constexpr int OEPI = 8;                 // epilogue warps
+constexpr int OBM = 128, OBN = 128, OBK = kTmaBoxK;
+constexpr int OTILE = OBM * OBK * 2;    // bytes of one digit tile (A or B)
+constexpr int ONA = 6, ONB = 8;         // ring slots
+constexpr int OLEV = 4;                 // levels per half (TMEM accumulators)
+constexpr int OTMEM_COLS = OLEV * OBN;
+constexpr int OEPI = 16;                // epilogue warps
+constexpr int OCOLS = 4 * OBN / OEPI;   // columns of an epilogue warp
 constexpr int OTHREADS = 32 * (2 + OEPI);
-constexpr int OSMEM_BYTES = OSTAGES * OSTAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
-constexpr int kChunkBlocks = kOzakiChunkK / OBK;
-static_assert(kOzakiChunkK % OBK == 0, "K chunks are whole TMA boxes");
-// exactness of one level's sum: (pairs per level) * chunk * 31^2 < 2^24
-static_assert((long long)kOzakiDigits * kOzakiChunkK * 961 < (1ll << 24),
-              "a level's integer sum must fit the FP32 significand");
+constexpr int OSMEM_BYTES = (ONA + ONB) * OTILE + 1024 /*align*/ + 512 /*barriers*/;
+static_assert(OTMEM_COLS == 512, "four levels of a group fill TMEM");
+static_assert(ONB > OLEV + 1, "the live B digits of a step and a slot to fill");
 }  // namespace
 
-struct OzakiParams {
-  CUtensorMap a, b;          // digit planes: rows s * Mp + m (s * Np + n), inner Kp
-  int M, N, Mp, Np;
-  int kblocks, n_chunks, tiles_n, n_tiles;
+struct OzakiGroup {
+  int M, N, Mp, Np, a_row0, kblocks, tiles_n, tile0;
   int b_lower;               // B lower triangular: tile n0 needs K < n0 + OBN only
-  const double *pa, *pb;     // 2^e of each row of A and of B
+  const int *ea, *eb;        // row exponents of A and of B
   double *C;
   long long ldc;
+};
+
+struct OzakiParams {
+  // digit planes: rows s * Mp + m (s * Np + n), inner k_pad
+  CUtensorMap a[kOzakiMaxGroups], b[kOzakiMaxGroups];
+  OzakiGroup g[kOzakiMaxGroups];
+  int n_groups, n_tiles;
+  int n_levels;              // levels 0 .. n_levels - 1 (8 or 9)
   DeviceStatus *status;
 };
+
+// Group sums are at most K 2^34.1 (levels 1-4): below 2^51 up to this K.
+constexpr int kLongK = 1 << 16;
+
+// A 64-bit integer below 2^51 in magnitude as FP64, by its bit pattern.
+__device__ __forceinline__ double exact_double(long long v) {
+  return __longlong_as_double(0x4338000000000000ll + v) - 6755399441055744.0;
+}
+
+// hi 2^28 + lo rounded once, for |hi| < 2^50 and |lo| < 2^62: two FP64
+// instructions (a 64-bit integer conversion alone takes three).
+__device__ __forceinline__ double combine(long long hi, long long lo) {
+  constexpr int kB = kOzakiBits * OLEV;
+  static_assert(kB == 28, "the constants below");
+  hi += lo >> kB;                                  // lo = 2^28 (lo >> 28) + rem, rem >= 0
+  const long long rem = lo & ((1ll << kB) - 1);
+  const double h = exact_double(hi - (1ll << 24));
+  const double r = __longlong_as_double(0x4330000000000000ll | rem);
+  return fma(h, 268435456.0, r);
+}
+
+// The same where the group sums may leave that range (K above kLongK).
+static __device__ __noinline__ double combine_long(long long hi, long long lo) {
+  return fma(__ll2double_rn(hi), 268435456.0, __ll2double_rn(lo));
+}
+
+// Four consecutive entries of a row of C, of which the first nc are there:
+// one 32-byte access where rows are 32-byte aligned (vec).
+__device__ __forceinline__ void store4(double *dst, const double (&o)[4], int nc, bool vec) {
+  if (vec && nc == 4) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(dst), "d"(o[0]), "d"(o[1]),
+                 "d"(o[2]), "d"(o[3])
+                 : "memory");
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    if (k < nc) dst[k] = o[k];
+}
+__device__ __forceinline__ void load4(const double *src, double (&o)[4], int nc, bool vec) {
+  if (vec && nc == 4) {
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3])
+                 : "l"(src)
+                 : "memory");
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) o[k] = k < nc ? src[k] : 0.0;
+}
+
+// The levels L0..L1 of one pass over a tile and their pairs (s, t) by steps s:
+// the partners of A digit s are B digits hi(s) .. lo(s), loaded from top down.
+struct LevelGroup {
+  int L0, L1;
+  // groups of four from the highest level down; the last takes what remains
+  __host__ __device__ constexpr LevelGroup(int n_levels, int gr)
+      : L0(n_levels - OLEV * (gr + 1) > 0 ? n_levels - OLEV * (gr + 1) : 0),
+        L1(n_levels - 1 - OLEV * gr) {}
+  static constexpr int D = kOzakiDigits;
+  __host__ __device__ constexpr int top() const { return L1 < D ? L1 : D - 1; }
+  __host__ __device__ constexpr int steps() const { return top() + 1; }
+  __host__ __device__ constexpr int hi(int s) const { return L1 - s < D ? L1 - s : D - 1; }
+  __host__ __device__ constexpr int lo(int s) const { return L0 > s ? L0 - s : 0; }
+  // K blocks whose level sums stay exact: pairs of one level * K * 64^2 <= 2^24
+  __host__ __device__ constexpr int chunk() const { return 4096 / (OBK * (top() + 1)); }
+  // first and last step with a pair of level L
+  __host__ __device__ static constexpr int first_step(int L) { return L < D ? 0 : L - (D - 1); }
+  __host__ __device__ static constexpr int last_step(int L) { return L < D ? L : D - 1; }
+};
+
+template <int NL, int GR> struct GroupConst {
+  __host__ __device__ static constexpr LevelGroup value() { return LevelGroup(NL, GR); }
+};
+
+// A position in a ring of N slots: slot and phase parity without divisions
+// (one thread walks the rings, its instruction latency is the kernel's rate).
+template <int N> struct RingPos {
+  int slot = 0;
+  uint32_t parity = 0;
+  __device__ __forceinline__ RingPos ahead(int k) const {  // k < N
+    RingPos r = *this;
+    r.slot += k;
+    if (r.slot >= N) {
+      r.slot -= N;
+      r.parity ^= 1u;
+    }
+    return r;
+  }
+  __device__ __forceinline__ void advance(int k) { *this = ahead(k); }
+};
+// TMEM column of the accumulator of a group's level L0 + l: descending, as the
+// B digits of a step (largest first) meet the levels.
+__host__ __device__ constexpr int acc_col(int l) { return (OLEV - 1 - l) * OBN; }
+__device__ __forceinline__ int level_groups(int n_levels) { return (n_levels + OLEV - 1) / OLEV; }
+
+// v 2^k for a finite v, exactly where the result is a normal number (the
+// exponent field is moved by an integer add; FP64 instructions are scarce).
+__device__ __forceinline__ double scale_pow2(double v, int k) {
+  const long long b = __double_as_longlong(v);
+  const int ex = (int)((b >> 52) & 0x7ff);
+  if (ex != 0 && ex + k > 0 && ex + k < 0x7ff)
+    return __longlong_as_double(b + ((long long)k << 52));
+  // zero, or a result at the ends of the range: |k| < 3 * 1000
+  auto p2 = [](int n) { return __longlong_as_double((long long)(1023 + n) << 52); };
+  const int k1 = k / 3, k2 = (k - k1) / 2;
+  return v * p2(k1) * p2(k2) * p2(k - k1 - k2);
+}
 
 __global__ void __launch_bounds__(OTHREADS, 1)
 k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
@@ -76,26 +211,37 @@ k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char *gbase = smem_raw + (base - raw);
-  const uint32_t bars = base + OSTAGES * OSTAGE_BYTES;
-  uint64_t *bar_ptr = reinterpret_cast<uint64_t *>(gbase + OSTAGES * OSTAGE_BYTES);
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_ptr + 2 * OSTAGES + 2 * OACC);
+  constexpr int kBarOff = (ONA + ONB) * OTILE;
+  constexpr int kBars = 2 * (ONA + ONB) + 2 * OLEV;
+  const uint32_t bars = base + kBarOff;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(gbase + kBarOff + 8 * kBars);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-  auto full_bar = [&](int s) { return bars + 8u * s; };
-  auto empty_bar = [&](int s) { return bars + 8u * (OSTAGES + s); };
-  auto accf_bar = [&](int b) { return bars + 8u * (2 * OSTAGES + b); };
-  auto acce_bar = [&](int b) { return bars + 8u * (2 * OSTAGES + OACC + b); };
+  auto a_slot = [&](int s) { return base + (uint32_t)s * OTILE; };
+  auto b_slot = [&](int s) { return base + (uint32_t)(ONA + s) * OTILE; };
+  auto a_full = [&](int s) { return bars + 8u * s; };
+  auto a_empty = [&](int s) { return bars + 8u * (ONA + s); };
+  auto b_full = [&](int s) { return bars + 8u * (2 * ONA + s); };
+  auto b_empty = [&](int s) { return bars + 8u * (2 * ONA + ONB + s); };
+  auto accf_bar = [&](int l) { return bars + 8u * (2 * (ONA + ONB) + l); };
+  auto acce_bar = [&](int l) { return bars + 8u * (2 * (ONA + ONB) + OLEV + l); };
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
   const int cid = (int)blockIdx.x, ncta = (int)gridDim.x;
+  const int ngr = level_groups(p.n_levels);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < OSTAGES; s++) {
-      mbar_init(full_bar(s), 1);
-      mbar_init(empty_bar(s), 1);
+    for (int s = 0; s < ONA; s++) {
+      mbar_init(a_full(s), 1);
+      mbar_init(a_empty(s), 1);
     }
-    for (int b = 0; b < OACC; b++) {
-      mbar_init(accf_bar(b), 1);
-      mbar_init(acce_bar(b), OEPI);
+    for (int s = 0; s < ONB; s++) {
+      mbar_init(b_full(s), 1);
+      mbar_init(b_empty(s), 1);
+    }
+    for (int l = 0; l < OLEV; l++) {
+      mbar_init(accf_bar(l), 1);
+      mbar_init(acce_bar(l), OEPI);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -112,149 +258,290 @@ k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
-  // K blocks and chunks of a tile: all of K, or with a lower-triangular B
-  // (row n of B is zero beyond column n) only the blocks below n0 + OBN
-  auto tile_kb = [&](int t) {
-    if (!p.b_lower) return p.kblocks;
-    const int n0 = (t % p.tiles_n) * OBN;
-    const int e = (n0 + OBN + OBK - 1) / OBK;
-    return e < p.kblocks ? e : p.kblocks;
+  // tile t -> its product, row and column origin, K blocks (all of K, or with
+  // a lower-triangular B, whose row n is zero beyond column n, only the blocks
+  // below n0 + OBN)
+  auto locate = [&](int t, int &gi, int &mrow, int &n0, int &kbt) {
+    gi = 0;
+    while (gi + 1 < p.n_groups && t >= p.g[gi + 1].tile0) gi++;
+    const OzakiGroup &g = p.g[gi];
+    const int lt = t - g.tile0;
+    mrow = (lt / g.tiles_n) * OBM;
+    n0 = (lt % g.tiles_n) * OBN;
+    kbt = g.kblocks;
+    if (g.b_lower) kbt = min(kbt, (n0 + OBN + OBK - 1) / OBK);
   };
-  auto n_chunks_of = [&](int kbt) { return (kbt + kChunkBlocks - 1) / kChunkBlocks; };
 
   if (warp == 0 && lane == 0) {
     // ---------------- TMA producer ----------------
-    int it = 0;
+    RingPos<ONA> ia;
+    RingPos<ONB> ib;
     bool stop = false;
+    auto wait_slot = [&](uint32_t bar, uint32_t parity, int t) {
+      if (!mbar_wait(bar, parity)) {
+        set_status(p.status, FPP_ERR_TIMEOUT, 211, t);
+        *abort_flag = 1;
+      }
+      if (*abort_flag) stop = true;
+      return !stop;
+    };
     for (int t = cid; t < p.n_tiles && !stop; t += ncta) {
-      const int mrow = (t / p.tiles_n) * OBM, n0 = (t % p.tiles_n) * OBN;
-      const int kbt = tile_kb(t), nch = n_chunks_of(kbt);
-      for (int L = 0; L < kOzakiDigits && !stop; L++)
-        for (int c = 0; c < nch && !stop; c++) {
-          const int kb1 = min((c + 1) * kChunkBlocks, kbt);
-          for (int s = 0; s <= L && !stop; s++)
-            for (int kb = c * kChunkBlocks; kb < kb1; kb++, it++) {
-              const int st = it % OSTAGES;
-              const uint32_t ph = (uint32_t)((it / OSTAGES) & 1);
-              if (!mbar_wait(empty_bar(st), ph ^ 1u)) {
-                set_status(p.status, FPP_ERR_TIMEOUT, 211, t);
-                *abort_flag = 1;
-              }
-              if (*abort_flag) {
-                stop = true;
-                break;
-              }
-              const uint32_t sa = base + st * OSTAGE_BYTES;
-              mbar_expect_tx(full_bar(st), OSTAGE_BYTES);
-              tma_load_2d(sa, &p.a, full_bar(st), kb * OBK, s * p.Mp + mrow);
-              tma_load_2d(sa + OA_TILE, &p.b, full_bar(st), kb * OBK, (L - s) * p.Np + n0);
+      int gi, mrow, n0, kbt;
+      locate(t, gi, mrow, n0, kbt);
+      const CUtensorMap *ma = &p.a[gi], *mb = &p.b[gi];
+      const int Mp = p.g[gi].Mp, Np = p.g[gi].Np, arow = p.g[gi].a_row0 + mrow;
+      for (int gr = 0; gr < ngr && !stop; gr++) {
+        const LevelGroup G(p.n_levels, gr);
+        for (int kb = 0; kb < kbt && !stop; kb++) {
+          int next = G.top();  // the next B digit to load
+          for (int s = 0; s < G.steps() && !stop; s++) {
+            {
+              const int st = ia.slot;
+              if (!wait_slot(a_empty(st), ia.parity ^ 1u, t)) break;
+              mbar_expect_tx(a_full(st), OTILE);
+              tma_load_2d(a_slot(st), ma, a_full(st), kb * OBK, s * Mp + arow);
+              ia.advance(1);
             }
+            // the B digits first used at this step, largest first
+            for (; next >= G.lo(s) && !stop; next--) {
+              const int st = ib.slot;
+              if (!wait_slot(b_empty(st), ib.parity ^ 1u, t)) break;
+              mbar_expect_tx(b_full(st), OTILE);
+              tma_load_2d(b_slot(st), mb, b_full(st), kb * OBK, next * Np + n0);
+              ib.advance(1);
+            }
+          }
         }
+      }
     }
-    // drain: every stage this CTA filled has been read before it exits
-    for (int d = 0; d < OSTAGES && !*abort_flag; d++, it++) {
-      if (!mbar_wait(empty_bar(it % OSTAGES), (uint32_t)(((it / OSTAGES) & 1) ^ 1))) {
+    // drain: every slot this CTA filled has been read before it exits
+    for (int d = 0; d < ONA && !*abort_flag; d++, ia.advance(1))
+      if (!mbar_wait(a_empty(ia.slot), ia.parity ^ 1u)) {
         set_status(p.status, FPP_ERR_TIMEOUT, 215, d);
         *abort_flag = 1;
       }
-    }
-  } else if (warp == 1 && lane == 0) {
+    for (int d = 0; d < ONB && !*abort_flag; d++, ib.advance(1))
+      if (!mbar_wait(b_empty(ib.slot), ib.parity ^ 1u)) {
+        set_status(p.status, FPP_ERR_TIMEOUT, 216, d);
+        *abort_flag = 1;
+      }
+  } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    int it = 0, j = 0;
+    // ib: slot of the K block's first B digit; unit: uses of accumulator 0, of
+    // the others (a group of one level leaves them out).  Everything but the
+    // waits is unrolled per group of levels: with the slots and levels worked
+    // out at run time this thread took 376 cycles per pair, the pair's four
+    // MMAs 256.
+    RingPos<ONA> ia;
+    RingPos<ONB> ib;
+    int unit = 0, unit_rest = 0;
     bool stop = false;
-    for (int t = cid; t < p.n_tiles && !stop; t += ncta) {
-      const int kbt = tile_kb(t), nch = n_chunks_of(kbt);
-      for (int L = 0; L < kOzakiDigits && !stop; L++)
-        for (int c = 0; c < nch && !stop; c++, j++) {
-          const int kb1 = min((c + 1) * kChunkBlocks, kbt);
-          const int buf = j % OACC;
-          const uint32_t acc = tmem + (uint32_t)(buf * OBN);
-          if (!mbar_wait(acce_bar(buf), (uint32_t)(((j / OACC) & 1) ^ 1))) {
-            set_status(p.status, FPP_ERR_TIMEOUT, 212, t);
-            *abort_flag = 1;
-          }
-          if (*abort_flag) {
-            mma_commit(accf_bar(buf));  // release the epilogue of this buffer
-            stop = true;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          bool first = true;
-          for (int s = 0; s <= L && !stop; s++)
-            for (int kb = c * kChunkBlocks; kb < kb1; kb++, it++) {
-              const int st = it % OSTAGES;
-              const uint32_t ph = (uint32_t)((it / OSTAGES) & 1);
-              if (!mbar_wait(full_bar(st), ph)) {
-                set_status(p.status, FPP_ERR_TIMEOUT, 213, t);
-                *abort_flag = 1;
-                stop = true;
-                break;
-              }
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              const uint32_t sa = base + st * OSTAGE_BYTES, sb = sa + OA_TILE;
+    const uint64_t da0 = smem_desc(base), db0 = smem_desc(base + ONA * OTILE);
+    auto wait_or_abort = [&](uint32_t bar, uint32_t parity, int site, int t) {
+      if (!mbar_wait(bar, parity)) {
+        if (lane == 0) set_status(p.status, FPP_ERR_TIMEOUT, site, t);
+        *abort_flag = 1;
+      }
+    };
+    auto k_block = [&](auto lc, bool chunk_first, bool chunk_last, int t) {
+      constexpr LevelGroup G = decltype(lc)::value();
 #pragma unroll
-              for (int ks = 0; ks < OBK / 16; ks++) {
-                const uint32_t off = ks * 32;
-                mma_f16<OBN>(acc, smem_desc(sa + off), smem_desc(sb + off),
-                             (first && ks == 0) ? 0u : 1u);
-              }
-              first = false;
-              mma_commit(empty_bar(st));  // frees the stage once these MMAs read it
-            }
-          mma_commit(accf_bar(buf));
+      for (int s = 0; s < G.steps(); s++) {
+        wait_or_abort(a_full(ia.slot), ia.parity, 213, t);
+#pragma unroll
+        for (int d = s == 0 ? G.top() : G.lo(s - 1) - 1; d >= G.lo(s); d--) {
+          const RingPos<ONB> q = ib.ahead(G.top() - d);
+          wait_or_abort(b_full(q.slot), q.parity, 213, t);
         }
+        const bool fresh = chunk_first && s <= G.first_step(G.L1);
+        if (fresh) {
+          // the accumulators of the levels that start at this step
+#pragma unroll
+          for (int L = G.L0; L <= G.L1; L++)
+            if (s == G.first_step(L))
+              wait_or_abort(acce_bar(L - G.L0),
+                            (uint32_t)((L == G.L0 ? unit : unit_rest) & 1) ^ 1u, 212, t);
+        }
+        if (__any_sync(0xffffffffu, *abort_flag)) return false;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t pa = da0 + (uint64_t)(ia.slot * (OTILE >> 4));
+        // Partners two by two: B digits d and d - 1 in neighboring slots are one
+        // 256-row operand and their levels' accumulators neighboring columns, so
+        // one N = 256 MMA forms both pairs.
+#pragma unroll
+        for (int j = 0; j < OLEV; j += 2) {
+          const int d = G.hi(s) - j;
+          if (d < G.lo(s)) continue;
+          const RingPos<ONB> q0 = ib.ahead(G.top() - d);
+          const uint64_t pb = db0 + (uint64_t)(q0.slot * (OTILE >> 4));
+          const uint32_t acc = tmem + (uint32_t)(acc_col(s + d - G.L0));
+          const bool new0 = s == G.first_step(s + d), new1 = s == G.first_step(s + d - 1);
+          const uint32_t add0 = new0 && chunk_first ? 0u : 1u;
+          const uint32_t add1 = new1 && chunk_first ? 0u : 1u;
+          const bool two = d - 1 >= G.lo(s);
+          if (two && add0 == add1 && q0.slot + 1 < ONB) {
+            if (elect_one()) {
+#pragma unroll
+              for (int ks = 0; ks < OBK / 16; ks++)
+                mma_f16<2 * OBN>(acc, pa + ks * 2, pb + ks * 2, ks == 0 ? add0 : 1u);
+            }
+          } else {
+            const uint64_t pb1 = db0 + (uint64_t)(q0.ahead(1).slot * (OTILE >> 4));
+            if (elect_one()) {
+#pragma unroll
+              for (int ks = 0; ks < OBK / 16; ks++)
+                mma_f16<OBN>(acc, pa + ks * 2, pb + ks * 2, ks == 0 ? add0 : 1u);
+              if (two) {
+#pragma unroll
+                for (int ks = 0; ks < OBK / 16; ks++)
+                  mma_f16<OBN>(acc + OBN, pa + ks * 2, pb1 + ks * 2, ks == 0 ? add1 : 1u);
+              }
+            }
+          }
+        }
+        // free the slots once these MMAs read them: the A digit, and the B
+        // digits without a later partner
+        if (elect_one()) {
+          mma_commit(a_empty(ia.slot));
+#pragma unroll
+          for (int d = G.top(); d >= 0; d--) {
+            const int last = G.L1 - d < G.steps() ? G.L1 - d : G.steps() - 1;
+            if (s == last) mma_commit(b_empty(ib.ahead(G.top() - d).slot));
+          }
+          if (chunk_last) {
+#pragma unroll
+            for (int L = G.L0; L <= G.L1; L++)
+              if (s == G.last_step(L)) mma_commit(accf_bar(L - G.L0));
+          }
+        }
+        __syncwarp();
+        ia.advance(1);
+      }
+      ib.advance(G.steps());
+      if (chunk_last) {
+        unit++;
+        if (G.L1 > G.L0) unit_rest++;
+      }
+      return true;
+    };
+    for (int t = cid; t < p.n_tiles && !stop; t += ncta) {
+      int gi, mrow, n0, kbt;
+      locate(t, gi, mrow, n0, kbt);
+      for (int gr = 0; gr < ngr && !stop; gr++)
+        for (int kb = 0; kb < kbt && !stop; kb++) {
+          const int chunk = LevelGroup(p.n_levels, gr).chunk();
+          const bool first = kb % chunk == 0;
+          const bool last = kb + 1 == kbt || (kb + 1) % chunk == 0;
+          bool ok;
+          if (p.n_levels == 8)
+            ok = gr == 0 ? k_block(GroupConst<8, 0>{}, first, last, t)
+                         : k_block(GroupConst<8, 1>{}, first, last, t);
+          else
+            ok = gr == 0   ? k_block(GroupConst<9, 0>{}, first, last, t)
+                 : gr == 1 ? k_block(GroupConst<9, 1>{}, first, last, t)
+                           : k_block(GroupConst<9, 2>{}, first, last, t);
+          stop = !ok;
+        }
+    }
+    if (__any_sync(0xffffffffu, *abort_flag)) {  // release the epilogue
+      if (elect_one())
+        for (int l = 0; l < OLEV; l++) mma_commit(accf_bar(l));
     }
   } else if (warp >= 2) {
     // ---------------- epilogue ----------------
     const int q = warp & 3;                 // TMEM lane quarter this warp may access
-    const int half = (warp - 2) / 4;        // which 64 columns of the tile
+    const int colh = (warp - 2) / 4;        // which OCOLS columns of the tile
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
-    int j = 0;
+    int unit = 0, unit_rest = 0;
     bool stop = false;
     for (int t = cid; t < p.n_tiles && !stop; t += ncta) {
-      const int mrow = (t / p.tiles_n) * OBM, n0 = (t % p.tiles_n) * OBN + half * 64;
+      int gi, mrow, n0, kbt;
+      locate(t, gi, mrow, n0, kbt);
+      const OzakiGroup &g = p.g[gi];
+      n0 += colh * OCOLS;
       const int r = mrow + q * 32 + lane;
-      const int nch = n_chunks_of(tile_kb(t));
-      double acc[64];
+      double *crow = g.C + (size_t)r * g.ldc + n0;
+      const bool long_k = kbt * OBK > kLongK;
+      const bool vec = (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(g.C) & 31u) == 0;
+      for (int gr = 0; gr < ngr && !stop; gr++) {
+        const LevelGroup G(p.n_levels, gr);
+        const int nch = (kbt + G.chunk() - 1) / G.chunk();
+        long long acc[OCOLS];
 #pragma unroll
-      for (int i = 0; i < 64; i++) acc[i] = 0.0;
-      for (int L = 0; L < kOzakiDigits && !stop; L++) {
-        // 2^(-5 (L + 2)), exact
-        const double sL = __longlong_as_double((long long)(1023 - 5 * (L + 2)) << 52);
-        for (int c = 0; c < nch; c++, j++) {
-          const int buf = j % OACC;
-          bool have = mbar_wait(accf_bar(buf), (uint32_t)((j / OACC) & 1));
-          have = __all_sync(0xffffffffu, have) != 0;
-          if (!have) {
-            if (lane == 0) set_status(p.status, FPP_ERR_TIMEOUT, 214, t);
-            *abort_flag = 1;
-            stop = true;
-            break;
+        for (int i = 0; i < OCOLS; i++) acc[i] = 0;
+        for (int c = 0; c < nch && !stop; c++, unit++, unit_rest += G.L1 > G.L0) {
+          for (int l = 0; l < OLEV; l++) {
+            if (l > G.L1 - G.L0) break;  // a group of one level
+            bool have = mbar_wait(accf_bar(l), (uint32_t)((l == 0 ? unit : unit_rest) & 1));
+            have = __all_sync(0xffffffffu, have) != 0;
+            if (!have) {
+              if (lane == 0) set_status(p.status, FPP_ERR_TIMEOUT, 214, t);
+              *abort_flag = 1;
+            }
+            if (__shfl_sync(0xffffffffu, *abort_flag, 0)) {
+              stop = true;
+              break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t tm = tmem + (uint32_t)(acc_col(l) + colh * OCOLS) + lane_base;
+            const int w = 1 << (kOzakiBits * (G.L1 - G.L0 - l));  // weight of the level
+#pragma unroll
+            for (int i0 = 0; i0 < OCOLS; i0 += 16) {
+              float v[16];
+              tmem_ld16(tm + i0, v);
+#pragma unroll
+              for (int i = 0; i < 16; i++)
+                acc[i0 + i] += (long long)__float2int_rn(v[i]) * w;
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acce_bar(l));
           }
-          if (__shfl_sync(0xffffffffu, *abort_flag, 0)) {
-            stop = true;
-            break;
-          }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t tm = tmem + (uint32_t)(buf * OBN + half * 64) + lane_base;
-          float v[32];
-          tmem_ld32(tm, v);
-#pragma unroll
-          for (int i = 0; i < 32; i++) acc[i] = fma((double)v[i], sL, acc[i]);
-          tmem_ld32(tm + 32, v);
-#pragma unroll
-          for (int i = 0; i < 32; i++) acc[32 + i] = fma((double)v[i], sL, acc[32 + i]);
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) mbar_arrive(acce_bar(buf));
         }
-      }
-      if (stop || r >= p.M) continue;
-      const double pr = p.pa[r];
-      double *crow = p.C + (size_t)r * p.ldc + n0;
+        if (stop) break;
+        if (r < g.M) {
+          // The sum of the groups so far returns to the thread that stored it:
+          // the lowest group as a 64-bit integer, then FP64, in units of the lowest
+          // group's weight.
+          const bool last = gr + 1 == ngr;
+          const int er = last ? g.ea[r] : 0;
+          const int shift = 2 - kOzakiBits * (2 + p.n_levels - 1);
 #pragma unroll
-      for (int i = 0; i < 64; i++)
-        if (n0 + i < p.N) crow[i] = acc[i] * pr * p.pb[n0 + i];
+          for (int i = 0; i < OCOLS; i += 4) {
+            asm volatile("" ::: "memory");  // one block of loads in flight per four columns
+            const int nc = min(g.N - (n0 + i), 4);
+            if (nc <= 0) break;
+            double *dst = crow + i;
+            if (gr == 0) {
+              const long long o[4] = {acc[i], acc[i + 1], acc[i + 2], acc[i + 3]};
+              store4(dst, reinterpret_cast<const double(&)[4]>(o), nc, vec);
+              continue;
+            }
+            double before[4], o[4];
+            load4(dst, before, nc, vec);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              // after combine in units of the lowest group's weight
+              double v;
+              if (gr == 1)
+                v = long_k ? combine_long(acc[i + k], __double_as_longlong(before[k]))
+                           : combine(acc[i + k], __double_as_longlong(before[k]));
+              else
+                v = fma(long_k ? __ll2double_rn(acc[i + k]) : exact_double(acc[i + k]),
+                        72057594037927936.0, before[k]);
+              if (last) {
+                const int ec = k < nc ? g.eb[n0 + i + k] : 0;
+                v = (er == kOzakiNanRow || ec == kOzakiNanRow)
+                        ? __longlong_as_double(0x7ff8000000000000ll)
+                        : scale_pow2(v, er + ec + shift);
+              }
+              o[k] = v;
+            }
+            store4(dst, o, nc, vec);
+          }
+        }
+        __syncwarp();
+      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -267,40 +554,97 @@ k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
 }
 
 // Digit planes of the rows of X (rows x K, leading dimension ldx): a warp per
-// row; rows >= rows and columns >= K of the padded planes are written as zeros.
+// row, four entries per lane; rows >= rows and columns >= K of the padded planes
+// are zeros.  All in integer arithmetic (FP64 issues 2 per clock and SM, this
+// kernel moves an entry per clock): the row maximum by comparing the bit
+// patterns of |x|, the digits from the significand shifted to the row's scale
+// (rounded to nearest), each digit pair turned to fp16 by one packed subtract.
 __global__ void __launch_bounds__(256)
 k_ozaki_split(int rows, int K, long long ldx, const double *__restrict__ X, int rows_pad,
-              int k_pad, __half *__restrict__ planes, double *__restrict__ p2) {
+              int k_pad, __half *__restrict__ planes, int *__restrict__ exps) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= rows_pad) return;
   const int r = warp;
   const size_t plane = (size_t)rows_pad * k_pad;
   __half *dst = planes + (size_t)r * k_pad;
+  const int nq = k_pad >> 2;
   if (r >= rows) {
-    for (int k = lane; k < k_pad; k += 32)
-      for (int s = 0; s < kOzakiDigits; s++) dst[s * plane + k] = __float2half_rn(0.0f);
+    for (int s = 0; s < kOzakiDigits; s++)
+      for (int q = lane; q < nq; q += 32)
+        reinterpret_cast<uint2 *>(dst + s * plane)[q] = make_uint2(0u, 0u);
     return;
   }
   const double *x = X + (size_t)r * ldx;
-  double mx = 0.0;
-  for (int k = lane; k < K; k += 32) mx = fmax(mx, fabs(x[k]));
+  const bool al = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+  auto load4 = [&](int k, unsigned long long (&b)[4]) {
+    if (al && k + 4 <= K) {
+      const ulonglong2 u = reinterpret_cast<const ulonglong2 *>(x + k)[0];
+      const ulonglong2 v = reinterpret_cast<const ulonglong2 *>(x + k)[1];
+      b[0] = u.x, b[1] = u.y, b[2] = v.x, b[3] = v.y;
+    } else {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  // the row's power of two: max |x| < 2^e (e = 0 for an all-zero row)
-  int e = 0;
-  if (mx > 0.0) frexp(mx, &e);
-  if (lane == 0) p2[r] = ldexp(1.0, e);
-  const double inv = ldexp(1.0, -e);
-  // 55-bit fixed point of |x| 2^-e (exact scaling; truncation below 2^-55)
-  const double two55 = 36028797018963968.0;
-  for (int k = lane; k < k_pad; k += 32) {
-    const double v = k < K ? x[k] : 0.0;
-    const unsigned long long X55 = __double2ull_rz(fabs(v) * inv * two55);
-    const bool neg = v < 0.0;
+      for (int i = 0; i < 4; i++)
+        b[i] = k + i < K ? (unsigned long long)__double_as_longlong(x[k + i]) : 0ull;
+    }
+  };
+  constexpr unsigned long long kAbs = 0x7fffffffffffffffull;
+  unsigned long long mx = 0ull;
+  for (int k = 4 * lane; k < K; k += 128) {
+    unsigned long long b[4];
+    load4(k, b);
 #pragma unroll
-    for (int s = 0; s < kOzakiDigits; s++) {
-      const int d = (int)((X55 >> (kOzakiBits * (kOzakiDigits - 1 - s))) & 31ull);
-      dst[s * plane + k] = __int2half_rn(neg ? -d : d);
+    for (int i = 0; i < 4; i++) mx = max(mx, b[i] & kAbs);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  // max |x| < 2^e: the biased exponent of the largest entry (a subnormal row
+  // keeps the scale of the smallest normal number); Inf and NaN mark the row
+  const bool bad = mx >= 0x7ff0000000000000ull;
+  const int bex = max((int)(mx >> 52), 1);
+  const int e = mx == 0ull ? 0 : bex - 1022;
+  if (lane == 0) exps[r] = bad ? kOzakiNanRow : e;
+  for (int q = lane; q < nq; q += 32) {
+    const int k = 4 * q;
+    unsigned long long b[4];
+    load4(k, b);
+    // signed 55-bit fixed point of x 2^-(e + 1), LSB 2^-56
+    long long f[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const unsigned long long a = b[i] & kAbs;
+      const int ex = (int)(a >> 52);
+      unsigned long long m = a & 0xfffffffffffffull;
+      if (ex > 0) m |= 0x10000000000000ull;
+      m <<= 2;                                    // the largest entry's place
+      const int sh = bex - max(ex, 1);            // >= 0
+      if (sh > 0) m = sh < 56 ? (m + (1ull << (sh - 1))) >> sh : 0ull;
+      f[i] = (b[i] >> 63) ? -(long long)m : (long long)m;
+      if (bad) f[i] = 0;
+    }
+#pragma unroll
+    for (int s = kOzakiDigits - 1; s >= 0; s--) {
+      unsigned d[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        // balanced digit in [-64, 63] (the top one is what remains, <= 64)
+        int v;
+        if (s > 0) {
+          v = (int)((f[i] + 64) & 127) - 64;
+          f[i] = (f[i] - v) >> kOzakiBits;
+        } else {
+          v = (int)f[i];
+        }
+        d[i] = (unsigned)(v + 512);
+      }
+      // 0x6400 | n is the fp16 number 1024 + n, n < 1024
+      const unsigned p01 = 0x64006400u | d[0] | (d[1] << 16);
+      const unsigned p23 = 0x64006400u | d[2] | (d[3] << 16);
+      const __half2 off = __float2half2_rn(1536.0f);
+      const __half2 h01 = __hsub2(*reinterpret_cast<const __half2 *>(&p01), off);
+      const __half2 h23 = __hsub2(*reinterpret_cast<const __half2 *>(&p23), off);
+      reinterpret_cast<uint2 *>(dst + s * plane)[q] =
+          make_uint2(*reinterpret_cast<const unsigned *>(&h01),
+                     *reinterpret_cast<const unsigned *>(&h23));
     }
   }
 }
@@ -336,43 +680,55 @@ OzakiShape ozaki_shape(int rows, int K) {
 }
 
 int launch_ozaki_split(int rows, int K, const double *X, long long ldx, __half *planes,
-                       double *p2, cudaStream_t stream) {
+                       int *exps, cudaStream_t stream) {
   if (rows <= 0) return 0;
   const OzakiShape sh = ozaki_shape(rows, K);
   const int threads = 256;
   const long long warps = sh.rows_pad;
   const int blocks = (int)((warps * 32 + threads - 1) / threads);
   k_ozaki_split<<<blocks, threads, 0, stream>>>(rows, K, ldx, X, sh.rows_pad, sh.k_pad,
-                                                 planes, p2);
+                                                 planes, exps);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-int launch_ozaki_gemm(int M, int N, int K, const __half *a_planes, const double *pa,
-                      const __half *b_planes, const double *pb, double *C, long long ldc,
-                      DeviceStatus *status, cudaStream_t stream, bool b_lower) {
-  if (M <= 0 || N <= 0) return 0;
-  if (K <= 0) return -2;
-  const OzakiShape sa = ozaki_shape(M, K), sb = ozaki_shape(N, K);
-  if (((uintptr_t)a_planes | (uintptr_t)b_planes) % 16 != 0 || ldc < N) return -2;
+int launch_ozaki_gemm(const OzakiProblem *probs, int n_probs, DeviceStatus *status,
+                      cudaStream_t stream, int n_levels) {
+  if (n_probs > kOzakiMaxGroups || (n_levels != 8 && n_levels != 9)) return -2;
   OzakiParams p;
   std::memset(&p, 0, sizeof(p));
-  // one map over all digit planes of an operand: rows s * rows_pad + row
-  if (make_map(&p.a, a_planes, sa.k_pad, sa.rows_pad * kOzakiDigits, sa.k_pad, OBM) ||
-      make_map(&p.b, b_planes, sb.k_pad, sb.rows_pad * kOzakiDigits, sb.k_pad, OBN))
-    return -3;
-  p.M = M;
-  p.N = N;
-  p.Mp = sa.rows_pad;
-  p.Np = sb.rows_pad;
-  p.kblocks = sa.k_pad / OBK;
-  p.n_chunks = (p.kblocks + kChunkBlocks - 1) / kChunkBlocks;
-  p.b_lower = b_lower ? 1 : 0;
-  p.tiles_n = (N + OBN - 1) / OBN;
-  p.n_tiles = (sa.rows_pad / OBM) * p.tiles_n;
-  p.pa = pa;
-  p.pb = pb;
-  p.C = C;
-  p.ldc = ldc;
+  int tiles = 0;
+  for (int k = 0; k < n_probs; k++) {
+    const OzakiProblem &q = probs[k];
+    if (q.M <= 0 || q.N <= 0) continue;
+    if (q.a.K <= 0 || q.a.K != q.b.K || q.a_row0 < 0 || q.a_row0 + q.M > q.a.rows ||
+        q.N > q.b.rows || q.ldc < q.N)
+      return -2;
+    const OzakiShape sa = ozaki_shape(q.a.rows, q.a.K), sb = ozaki_shape(q.b.rows, q.b.K);
+    if (((uintptr_t)q.a.planes | (uintptr_t)q.b.planes) % 16 != 0) return -2;
+    const int i = p.n_groups++;
+    // one map over all digit planes of an operand: rows s * rows_pad + row
+    if (make_map(&p.a[i], q.a.planes, sa.k_pad, sa.rows_pad * kOzakiDigits, sa.k_pad, OBM) ||
+        make_map(&p.b[i], q.b.planes, sb.k_pad, sb.rows_pad * kOzakiDigits, sb.k_pad, OBN))
+      return -3;
+    OzakiGroup &g = p.g[i];
+    g.M = q.M;
+    g.N = q.N;
+    g.Mp = sa.rows_pad;
+    g.Np = sb.rows_pad;
+    g.a_row0 = q.a_row0;
+    g.kblocks = sa.k_pad / OBK;
+    g.tiles_n = (q.N + OBN - 1) / OBN;
+    g.tile0 = tiles;
+    g.b_lower = q.b_lower ? 1 : 0;
+    g.ea = q.a.exps + q.a_row0;
+    g.eb = q.b.exps;
+    g.C = q.C;
+    g.ldc = q.ldc;
+    tiles += (q.M + OBM - 1) / OBM * g.tiles_n;
+  }
+  if (tiles == 0) return 0;
+  p.n_tiles = tiles;
+  p.n_levels = n_levels;
   p.status = status;
   int dev = 0, ctas = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || ozaki_launch_shape(dev, &ctas) != 0) return -1;
@@ -381,7 +737,7 @@ int launch_ozaki_gemm(int M, int N, int K, const __half *a_planes, const double 
   cfg.blockDim = dim3(OTHREADS, 1, 1);
   cfg.dynamicSmemBytes = OSMEM_BYTES;
   cfg.stream = stream;
-  cfg.gridDim = dim3(p.n_tiles < ctas ? p.n_tiles : ctas, 1, 1);
+  cfg.gridDim = dim3(tiles < ctas ? tiles : ctas, 1, 1);
   if (cudaLaunchKernelEx(&cfg, k_ozaki_gemm, p) != cudaSuccess) return -1;
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

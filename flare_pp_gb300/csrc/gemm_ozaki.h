@@ -10,9 +10,9 @@
 
 namespace fpp {
 
-constexpr int kOzakiDigits = 11;    // signed digits per operand entry
-constexpr int kOzakiBits = 5;       // bits per digit (|digit| <= 31)
-constexpr int kOzakiChunkK = 1536;  // K columns per exact FP32 level sum
+constexpr int kOzakiDigits = 8;  // balanced digits per operand entry
+constexpr int kOzakiBits = 7;    // bits per digit (|digit| <= 64)
+constexpr int kOzakiMaxGroups = 8;
 
 // Padded shape of one operand's digit planes: rows to a multiple of 128,
 // K to a multiple of 64; plane_bytes covers all kOzakiDigits planes.
@@ -23,18 +23,35 @@ struct OzakiShape {
 OzakiShape ozaki_shape(int rows, int K);
 
 // Digit planes (kOzakiDigits x rows_pad x k_pad fp16, zero padded) and the
-// power of two 2^e of each row (max |row| < 2^e) of X (rows x K, row stride
-// ldx, device memory).  The entries must be finite.
+// exponent e of each row (max |row| < 2^e; kOzakiNanRow if the row holds a
+// non-finite entry) of X (rows x K, row stride ldx, device memory).
+constexpr int kOzakiNanRow = -(1 << 30);
 int launch_ozaki_split(int rows, int K, const double *X, long long ldx, __half *planes,
-                       double *p2, cudaStream_t stream);
+                       int *exps, cudaStream_t stream);
 
-// C (M x N, row stride ldc) = A B^T from the digit planes and powers of two
-// of A (M x K) and B (N x K).  C need not be initialised.  b_lower: B is
-// lower triangular (B[n][k] = 0 for k > n; an L^-1, or an R^-1 transposed),
-// and the K blocks above each column tile's last row are skipped.  0 on
-// success.
-int launch_ozaki_gemm(int M, int N, int K, const __half *a_planes, const double *pa,
-                      const __half *b_planes, const double *pb, double *C, long long ldc,
-                      DeviceStatus *status, cudaStream_t stream, bool b_lower = false);
+// An operand split by launch_ozaki_split.
+struct OzakiMat {
+  const __half *planes;
+  const int *exps;
+  int rows, K;
+};
+
+// One product of a grouped launch: C (M x N, row stride ldc) = A B^T with rows
+// a_row0 .. a_row0 + M of operand a and rows 0 .. N of operand b.  C need not
+// be initialised.  b_lower: B is lower triangular (B[n][k] = 0 for k > n; an
+// L^-1, or an R^-1 transposed), and the K blocks above each column tile's last
+// row are skipped.  Rows or columns with a non-finite operand come out NaN.
+struct OzakiProblem {
+  OzakiMat a, b;
+  int a_row0, M, N;
+  double *C;
+  long long ldc;
+  bool b_lower;
+};
+// Up to kOzakiMaxGroups products in one persistent launch (their tiles share
+// the SMs).  n_levels: 8, or 9 where the dropped digit pairs must stay below the
+// operands' rounding (43 pairs instead of 36).  0 on success.
+int launch_ozaki_gemm(const OzakiProblem *probs, int n_probs, DeviceStatus *status,
+                      cudaStream_t stream, int n_levels = 8);
 
 }  // namespace fpp

@@ -42,10 +42,19 @@ struct DevBuf {
   template <typename T> T *as() const { return static_cast<T *>(ptr); }
 };
 
-// Workspace of the FP64-accurate tensor-core GEMM (digit planes and row
-// powers of two of both operands, status word), kept between calls.
+// Digit planes and row exponents of one operand of the FP64-accurate
+// tensor-core GEMM (gemm_ozaki.h).  ready: a constant operand of a model whose
+// planes are up to date (reset where the matrix changes).
+struct OzakiOperand {
+  DevBuf planes, exps;
+  int rows = 0, K = 0;
+  bool ready = false;
+};
+
+// Workspace of that GEMM (both operands, status word), kept between calls.
 struct OzakiWork {
-  DevBuf a, b, pa, pb, status;
+  OzakiOperand a, b;
+  DevBuf status;
 };
 
 // Cell quantities of Structure (structure.cpp:15-35), computed on the host
@@ -130,6 +139,7 @@ struct StructureState {
   DevBuf phat_hi, phat_lo;            // split fp16 operands (species-sorted)
   DevBuf order, order_inv;            // species-sorted atom order
   DevBuf V, V64;                      // beta p products
+  OzakiOperand oz_p;                  // digit planes of phat64
   DevBuf w64;                         // dE/dp (FP64 path)
   DevBuf u;                           // dE/dc per atom (adjoint)
   DevBuf pair_f;                      // double3/float per pair force
