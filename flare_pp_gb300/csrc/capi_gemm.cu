@@ -37,8 +37,9 @@ OzakiMat ozaki_mat(const OzakiOperand &op) {
   return OzakiMat{op.planes.as<__half>(), op.exps.as<int>(), op.rows, op.K};
 }
 
-int ozaki_run(const OzakiProblem *probs, int n, DeviceStatus *status, cudaStream_t st) {
-  const int rc = launch_ozaki_gemm(probs, n, status, st);
+int ozaki_run(const OzakiProblem *probs, int n, DeviceStatus *status, cudaStream_t st,
+              int n_levels) {
+  const int rc = launch_ozaki_gemm(probs, n, status, st, n_levels);
   if (rc != 0) return fail(FPP_ERR_CUDA, "tensor-core FP64 GEMM launch failed (" +
                                              std::to_string(rc) + ")");
   return FPP_OK;

@@ -531,11 +531,16 @@ static int upload_beta(fpp_model *m, int s, const std::vector<double> &B) {
   auto &sp = m->sp[s];
   std::vector<double> pad((size_t)nd * ldb, 0.0);
   double amax = 0;
+  bool finite = true;
   for (int i = 0; i < nd; i++)
     for (int j = 0; j < nd; j++) {
-      pad[(size_t)i * ldb + j] = B[(size_t)i * nd + j];
-      amax = std::max(amax, std::fabs(B[(size_t)i * nd + j]));
+      const double v = B[(size_t)i * nd + j];
+      pad[(size_t)i * ldb + j] = v;
+      amax = std::max(amax, std::fabs(v));
+      finite = finite && std::isfinite(v);
     }
+  sp.beta_finite = finite;
+  sp.oz_beta.ready = false;
   double scale = 1.0;
   if (amax > 0) scale = std::ldexp(1.0, (int)std::floor(std::log2(16384.0 / amax)));
   std::vector<__half> hi(pad.size()), lo(pad.size());
@@ -779,6 +784,43 @@ static int center_from_structure(fpp_model *m, fpp_structure *s, cudaStream_t st
   return set_center(m, pbar);
 }
 
+// V = phat beta (FP64), every species' rows against its own beta, in one launch
+// of the FP64-accurate tensor-core GEMM with nine digit levels, whose error is
+// below a DGEMM's.  cuBLAS's DGEMM runs at the FP64 rate, 1.1 TFLOP/s; an E/F/S
+// call on 4394 atoms, n_d = 544, spent 2478 us in two of them and spends 262 us
+// here, one of 2000 atoms, n_d = 1050, took 5180 us and takes 1216, and the
+// smallest (32-128 atoms, n_d = 30-1500) are no slower (0.39 -> 0.39 to 1.03 ->
+// 0.69 ms), so no size keeps the DGEMM.  Non-finite coefficients (a potential
+// file may hold any number) keep the DGEMM: their Inf and NaN spread as in FP64
+// arithmetic.
+static int contract64(fpp_model *m, fpp_structure *s, const double *phat, int ldp,
+                      cudaStream_t st) {
+  StructureState &S = s->st;
+  const int nd = m->n_d;
+  OzakiProblem q[kOzakiMaxGroups];
+  int nq = 0;
+  for (int sp = 0; sp < m->n_species; sp++) {
+    if (s->n_rows[sp] == 0) continue;
+    auto &M = m->sp[sp];
+    double *V = S.V64.as<double>() + (size_t)s->row_off[sp] * ldp;
+    if (!M.beta_finite) {
+      cublasHandle_t h;
+      FPP_TRY(get_cublas(m, st, &h));
+      const double one = 1.0, zero = 0.0;
+      FPP_CUBLAS(cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, nd, s->n_rows[sp], nd, &one,
+                             M.beta64.as<double>(), m->ldb,
+                             phat + (size_t)s->row_off[sp] * ldp, ldp, &zero, V, ldp));
+      continue;
+    }
+    // beta is symmetric: row n of B is column n
+    FPP_TRY(ozaki_const(M.oz_beta, nd, nd, M.beta64.as<double>(), m->ldb, st));
+    if (nq == 0) FPP_TRY(ozaki_split(S.oz_p, s->total_rows, nd, phat, ldp, st));
+    q[nq++] = OzakiProblem{ozaki_mat(S.oz_p), ozaki_mat(M.oz_beta), s->row_off[sp],
+                           s->n_rows[sp], nd, V, ldp, false};
+  }
+  return ozaki_run(q, nq, S.status.as<DeviceStatus>(), st, 9);
+}
+
 // Forward, contraction and adjoint of the mapped form; leaves atom_e, pair_f
 // and (with gather) forces / reduce_out in the structure workspace.
 int mapped_core(fpp_model *m, fpp_structure *s, int precision, cudaStream_t st,
@@ -811,16 +853,7 @@ int mapped_core(fpp_model *m, fpp_structure *s, int precision, cudaStream_t st,
     S.mark(3, st);
     double *phat = S.phat64.as<double>();
     if (m->beta_power == 2) {
-      cublasHandle_t h;
-      FPP_TRY(get_cublas(m, st, &h));
-      const double one = 1.0, zero = 0.0;
-      for (int sp = 0; sp < m->n_species; sp++) {
-        if (s->n_rows[sp] == 0) continue;
-        FPP_CUBLAS(cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, nd, s->n_rows[sp], nd, &one,
-                               m->sp[sp].beta64.as<double>(), m->ldb,
-                               phat + (size_t)s->row_off[sp] * ldp, ldp, &zero,
-                               S.V64.as<double>() + (size_t)s->row_off[sp] * ldp, ldp));
-      }
+      FPP_TRY(contract64(m, s, phat, ldp, st));
       g.V64 = S.V64.as<double>();
     }
     S.mark(4, st);

@@ -54,6 +54,9 @@ struct fpp_model {
     fpp::DevBuf beta_hi, beta_lo;       // half[n_d_pad * ldb] split operands
     double beta_scale = 1;              // beta ~ (hi + lo/2048) / beta_scale
     std::vector<double> B_host;         // dense beta (n_d x n_d), power 2
+    bool beta_finite = true;            // every entry of it
+    // digit planes of the constant GEMM operands, split on first use
+    fpp::OzakiOperand oz_beta;
   };
   std::vector<Species> sp;
   int beta_power = 0;                   // 0: no mapped coefficients yet
@@ -134,7 +137,8 @@ int ozaki_split(OzakiOperand &op, int rows, int K, const double *X, long long ld
 int ozaki_const(OzakiOperand &op, int rows, int K, const double *X, long long ldx,
                 cudaStream_t st);
 OzakiMat ozaki_mat(const OzakiOperand &op);
-int ozaki_run(const OzakiProblem *probs, int n, DeviceStatus *status, cudaStream_t st);
+int ozaki_run(const OzakiProblem *probs, int n, DeviceStatus *status, cudaStream_t st,
+              int n_levels = 8);
 // the workspace's status word, allocated and cleared on first use
 int ozaki_status(OzakiWork &w, cudaStream_t st, DeviceStatus **out);
 }  // namespace fpp
