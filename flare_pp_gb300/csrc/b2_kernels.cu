@@ -19,6 +19,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "basis.cuh"
 #include "b2_kernels.h"
@@ -41,6 +42,10 @@ void fill_fp32_cutoffs(B2Args &a) {
     const double ci = rc > a.r1 ? 1.0 / (rc - a.r1) : 0.0;
     a.cinv_hi[k] = (float)ci;
     a.cinv_lo[k] = (float)(ci - (double)a.cinv_hi[k]);
+    // ci + lo = 1 / (rc - r1) to about 2^-106: lo from the residual 1 - ci d
+    const double d = rc - a.r1;
+    a.cinv64_hi[k] = ci;
+    a.cinv64_lo[k] = ci != 0.0 ? std::fma(-ci, d, 1.0) * ci : 0.0;
   }
 }
 
@@ -79,6 +84,9 @@ int upload_harmonic_tables(cudaStream_t stream) {
       double dl = 1;  // D_lm of the division-free FP32 recurrence
       for (int k = m + 2; k <= l; k++) dl *= k - m;
       const double vf = v / dl;
+      double df = 1;  // (2m - 1)!!
+      for (int k = 1; k < 2 * m; k += 2) df *= k;
+      t.norm_q[l * (kMaxL + 1) + m] = v * (df / dl);
       t.norm_hi[l * (kMaxL + 1) + m] = (float)vf;
       t.norm_lo[l * (kMaxL + 1) + m] = (float)(vf - (double)(float)vf);
     }
@@ -184,6 +192,25 @@ int with_shape(const B2Args &a, F &&f) {
     }
   }
   return f(GenericShape{});
+}
+
+// The same for the single-bond and pair kernels, whose FP64 instantiations know
+// lmax (0..4; FP64 instructions are what bounds them, and only lmax changes their
+// number: channels past N are skipped by predicates).
+template <typename T, typename F>
+int with_lmax(const B2Args &a, F &&f) {
+  if constexpr (sizeof(T) == 8) {
+    switch (a.lmax) {
+      case 0: return f(Shape<0, 0, 0>{});
+      case 1: return f(Shape<0, 1, 0>{});
+      case 2: return f(Shape<0, 2, 0>{});
+      case 3: return f(Shape<0, 3, 0>{});
+      case 4: return f(Shape<0, 4, 0>{});
+      default: return f(GenericShape{});
+    }
+  } else {
+    return with_shape<T>(a, f);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -303,11 +330,15 @@ k_b2_forward(B2Args a, const int *__restrict__ offset,
         }
         if (keep) {
           sj = sp;
-          // FP32: hi/lo reciprocal of (rc - r1); FP64: the division
-          radial_basis<T>(r, r1t, rct, N, a.cutoff_kind, g_s + (size_t)b * GP,
-                          nullptr, 1, sizeof(T) == 4 ? T(a.cinv_hi[kc]) : T(0),
-                          sizeof(T) == 4 ? T(a.cinv_lo[kc]) : T(0));
-          real_harmonics<T>(x, y, z, LMAX, y_s + b, nullptr, WS);
+          radial_basis<T>(r, r1t, rct, N, a.cutoff_kind, g_s + (size_t)b * GP, nullptr, 1,
+                          sizeof(T) == 4 ? T(a.cinv_hi[kc]) : T(a.cinv64_hi[kc]),
+                          sizeof(T) == 4 ? T(a.cinv_lo[kc]) : T(a.cinv64_lo[kc]));
+          if constexpr (sizeof(T) == 8 && SH::kL1 > 0) {
+            const T ir = T(1) / r;
+            harmonics64<SH::kL1 - 1>(x * ir, y * ir, z * ir, y_s + b, WS);
+          } else {
+            real_harmonics<T>(x, y, z, LMAX, y_s + b, nullptr, WS);
+          }
         }
       }
       for (int sp = 0; sp < NS; sp++) {
@@ -1287,8 +1318,8 @@ k_pair_force(B2Args a, int strict, long long n_pairs, const int *__restrict__ nb
   if (keep) {
     T gr[kMaxN], dg[kMaxN];
     radial_basis_reg<T>(r, r1t, rct, N, a.cutoff_kind, gr, dg,
-                        sizeof(T) == 4 ? T(a.cinv_hi[kc]) : T(0),
-                        sizeof(T) == 4 ? T(a.cinv_lo[kc]) : T(0));
+                        sizeof(T) == 4 ? T(a.cinv_hi[kc]) : T(a.cinv64_hi[kc]),
+                        sizeof(T) == 4 ? T(a.cinv_lo[kc]) : T(a.cinv64_lo[kc]));
     const T *ur = u + (size_t)i * sb + (size_t)sj * N * H;
     T fr = T(0);
     if constexpr (sizeof(T) == 4) {
@@ -1313,6 +1344,26 @@ k_pair_force(B2Args a, int strict, long long n_pairs, const int *__restrict__ nb
       f[1] = f01.y;
       f[2] = f2r.x;
       fr = f2r.y;
+    } else if constexpr (SH::kL1 > 0) {
+      const T ir = T(1) / r;
+      const T ux = x * ir, uy = y * ir, uz = z * ir;
+      harmonics64_adjoint<SH::kL1 - 1>(
+          ux, uy, uz,
+          [&](int lm) {
+            double ag = 0.0, bd = 0.0;
+#pragma unroll
+            for (int n = 0; n < kMaxN; n++)
+              if (n < N) {
+                const double uv = ur[n * H + lm];
+                ag = fma(uv, gr[n], ag);
+                bd = fma(uv, dg[n], bd);
+              }
+            return make_double2(ag, bd);
+          },
+          f, fr);
+      f[0] = fma(f[0], ir, fr * ux);
+      f[1] = fma(f[1], ir, fr * uy);
+      f[2] = fma(f[2], ir, fr * uz);
     } else {
       harmonics_visit<T>(x, y, z, LMAX, [&](int lm, T Yv, T Yx, T Yy, T Yz) {
         T ag = T(0), bd = T(0);
@@ -1329,10 +1380,12 @@ k_pair_force(B2Args a, int strict, long long n_pairs, const int *__restrict__ nb
         f[2] += ag * Yz;
       });
     }
-    const T ir = T(1) / r;
-    f[0] += fr * x * ir;
-    f[1] += fr * y * ir;
-    f[2] += fr * z * ir;
+    if constexpr (sizeof(T) == 4 || SH::kL1 == 0) {
+      const T ir = T(1) / r;
+      f[0] += fr * x * ir;
+      f[1] += fr * y * ir;
+      f[2] += fr * z * ir;
+    }
   }
   if (sizeof(T) == 4) {
     reinterpret_cast<float4 *>(pair_f)[p] =
@@ -1793,105 +1846,59 @@ int launch_kuf_adjoint(const KufArgs &k, int ks, int threads, int n_items, int i
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-// F_i = sum over pairs of i (f_ij - f_ji); each block also reduces its atoms'
-// energies and virials (sum f_ij (x) r_ij) into one partial row (fixed tree
-// order, so the result is deterministic).  128 threads per block.
-template <typename T>
-__global__ void __launch_bounds__(128)
-k_gather(int noa, const int *__restrict__ offset, const int *__restrict__ rev,
-         const float4 *__restrict__ rel32, const dvec4 *__restrict__ rel,
-         const T *__restrict__ pair_f, const double *__restrict__ atom_e,
-         double *__restrict__ forces, double *__restrict__ partial) {
-  __shared__ double sm[10][128];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double acc[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  if (sizeof(T) == 4 && i < noa) {
-    // FP32 pair forces: per-atom sums kept as float-float (exact to ~2^-48)
-    // and the virial compensated, so no FP64 instruction runs per pair
-    float Fh[3] = {0, 0, 0}, Fl[3] = {0, 0, 0};
-    float Vs[9], Vc[9];
-#pragma unroll
-    for (int k = 0; k < 9; k++) Vs[k] = Vc[k] = 0.0f;
-    for (int p = offset[i]; p < offset[i + 1]; p++) {
-      const int q = rev[p];
-      const float4 fp = reinterpret_cast<const float4 *>(pair_f)[p];
-      const float4 fq = q >= 0 ? reinterpret_cast<const float4 *>(pair_f)[q]
-                               : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float fv[3] = {fp.x, fp.y, fp.z}, gv[3] = {fq.x, fq.y, fq.z};
-#pragma unroll
-      for (int a = 0; a < 3; a++) {
-        float s, e;
-        two_sum(Fh[a], fv[a], s, e);
-        Fl[a] += e;
-        two_sum(s, -gv[a], Fh[a], e);
-        Fl[a] += e;
-      }
-      const float4 r = rel32[p];
-      const float rr[3] = {r.x, r.y, r.z};
-#pragma unroll
-      for (int a = 0; a < 3; a++)
-#pragma unroll
-        for (int b = 0; b < 3; b++) {
-          const int k = a * 3 + b;
-          const float x = fv[a] * rr[b];
-          const float t = Vs[k] + x;
-          Vc[k] += fabsf(Vs[k]) >= fabsf(x) ? (Vs[k] - t) + x : (x - t) + Vs[k];
-          Vs[k] = t;
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < 3; a++) forces[3 * i + a] = double(Fh[a]) + double(Fl[a]);
-#pragma unroll
-    for (int k = 0; k < 9; k++) acc[1 + k] = double(Vs[k]) + double(Vc[k]);
-    acc[0] = atom_e[i];
-  } else if (i < noa) {
+// The FP64 gather: eight lanes per atom (a thread per atom left most of the chip
+// idle, waiting on the dependent loads rev[p] -> f[rev[p]]: 66 us at 2000 atoms).
+// F_i = sum over pairs of i (f_ij - f_ji); warps walk atoms with a grid stride and
+// each block writes one partial row of its atoms' energies and virials
+// (sum f_ij (x) r_ij); every sum runs in a fixed order.
+constexpr int kGather64Lanes = 8;
+__global__ void __launch_bounds__(32 * kGatherWarps)
+k_gather64(int noa, const int *__restrict__ offset, const int *__restrict__ rev,
+           const dvec4 *__restrict__ rel, const dvec4 *__restrict__ pair_f,
+           const double *__restrict__ atom_e, double *__restrict__ forces,
+           double *__restrict__ partial) {
+  __shared__ double sm[kGatherWarps][10];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int kGroups = 32 / kGather64Lanes;
+  const int g = lane / kGather64Lanes, gl = lane % kGather64Lanes;
+  double tot[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // energy, virial of this lane's pairs
+  const int stride = gridDim.x * kGatherWarps * kGroups;
+  for (int i0 = (blockIdx.x * kGatherWarps + warp) * kGroups; i0 < noa; i0 += stride) {
+    const int i = i0 + g;
+    const bool live = i < noa;
     double F[3] = {0, 0, 0};
-    for (int p = offset[i]; p < offset[i + 1]; p++) {
-      const int q = rev[p];
-      const double f0 = double(pair_f[(size_t)p * 4 + 0]);
-      const double f1 = double(pair_f[(size_t)p * 4 + 1]);
-      const double f2 = double(pair_f[(size_t)p * 4 + 2]);
-      F[0] += f0;
-      F[1] += f1;
-      F[2] += f2;
-      if (q >= 0) {  // always present for a periodic list; -1 is reported upstream
-        F[0] -= double(pair_f[(size_t)q * 4 + 0]);
-        F[1] -= double(pair_f[(size_t)q * 4 + 1]);
-        F[2] -= double(pair_f[(size_t)q * 4 + 2]);
-      }
-      double rr[3];
-      if (sizeof(T) == 8) {
-        const dvec4 r = rel[p];
-        rr[0] = r.y;
-        rr[1] = r.z;
-        rr[2] = r.w;
-      } else {
-        const float4 r = rel32[p];
-        rr[0] = r.x;
-        rr[1] = r.y;
-        rr[2] = r.z;
-      }
-      const double ff[3] = {f0, f1, f2};
+    const int beg = live ? offset[i] : 0, end = live ? offset[i + 1] : 0;
+    for (int p = beg + gl; p < end; p += kGather64Lanes) {
+      const int q = rev[p];  // -1 (reported upstream): no reverse pair
+      const dvec4 fp = pair_f[p], r = rel[p];
+      const dvec4 fq = q >= 0 ? pair_f[q] : dvec4{0, 0, 0, 0};
+      F[0] += fp.x - fq.x;
+      F[1] += fp.y - fq.y;
+      F[2] += fp.z - fq.z;
+      const double ff[3] = {fp.x, fp.y, fp.z}, rr[3] = {r.y, r.z, r.w};
 #pragma unroll
       for (int a = 0; a < 3; a++)
 #pragma unroll
-        for (int b = 0; b < 3; b++) acc[1 + a * 3 + b] += ff[a] * rr[b];
+        for (int b = 0; b < 3; b++) tot[1 + a * 3 + b] = fma(ff[a], rr[b], tot[1 + a * 3 + b]);
     }
-    forces[3 * i + 0] = F[0];
-    forces[3 * i + 1] = F[1];
-    forces[3 * i + 2] = F[2];
-    acc[0] = atom_e[i];
+#pragma unroll
+    for (int o = kGather64Lanes / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int a = 0; a < 3; a++) F[a] += __shfl_xor_sync(0xffffffffu, F[a], o);
+    if (live && gl < 3) forces[3 * i + gl] = gl == 0 ? F[0] : (gl == 1 ? F[1] : F[2]);
+    if (live && gl == 0) tot[0] += atom_e[i];
   }
 #pragma unroll
-  for (int k = 0; k < 10; k++) sm[k][threadIdx.x] = acc[k];
+  for (int k = 0; k < 10; k++) tot[k] = warp_sum(tot[k]);
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < 10; k++) sm[warp][k] = tot[k];
   __syncthreads();
-  for (int st = 64; st > 0; st >>= 1) {
-    if ((int)threadIdx.x < st)
-#pragma unroll
-      for (int k = 0; k < 10; k++) sm[k][threadIdx.x] += sm[k][threadIdx.x + st];
-    __syncthreads();
+  if (threadIdx.x < 10) {
+    double v = 0.0;
+    for (int w = 0; w < kGatherWarps; w++) v += sm[w][threadIdx.x];
+    partial[(size_t)blockIdx.x * 10 + threadIdx.x] = v;
   }
-  if (threadIdx.x < 10) partial[(size_t)blockIdx.x * 10 + threadIdx.x] = sm[threadIdx.x][0];
 }
 
 // Sum of the per-block partial rows: out[0] = E, out[1..9] = sum f (x) r.
@@ -1955,7 +1962,7 @@ int launch_b2_forward(B2Args a, const Neigh &nb, const int *species,
   const int wpb = warps_per_block(per);
   if (wpb == 0) return -1;
   size_t smem = per * wpb;
-  return with_shape<T>(a, [&](auto sh) {
+  return with_lmax<T>(a, [&](auto sh) {
     auto kern = k_b2_forward<T, decltype(sh)>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess)
@@ -2030,7 +2037,7 @@ int launch_b2_adjoint(B2Args a, const AdjArgs &g, const Neigh &nb,
   }
   if (cudaGetLastError() != cudaSuccess) return -1;
   if (n_pairs > 0) {
-    with_shape<T>(a, [&](auto sh) {
+    with_lmax<T>(a, [&](auto sh) {
       k_pair_force<T, decltype(sh)><<<(unsigned)((n_pairs + 127) / 128), 128, 0, stream>>>(
           a, g.strict, n_pairs, nbr_i, nb.rel, nb.rel32, nb.geom, nb.nbr_s, species, u_buf,
           pair_f);
@@ -2047,9 +2054,10 @@ int launch_b2_adjoint(B2Args a, const AdjArgs &g, const Neigh &nb,
         a.noa, nb.offset, nb.rev, nb.rel32, reinterpret_cast<const float4 *>(pair_f), atom_e,
         forces, atom_vir);
   } else {
-    nblk = ceil_div(a.noa, 128);
-    k_gather<T><<<nblk, 128, 0, stream>>>(a.noa, nb.offset, nb.rev, nb.rel32, nb.rel, pair_f,
-                                          atom_e, forces, atom_vir);
+    nblk = std::min(ceil_div(a.noa, kGatherWarps * (32 / kGather64Lanes)), 152 * 4);
+    k_gather64<<<nblk, 32 * kGatherWarps, 0, stream>>>(
+        a.noa, nb.offset, nb.rev, nb.rel, reinterpret_cast<const dvec4 *>(pair_f), atom_e,
+        forces, atom_vir);
   }
   if (cudaGetLastError() != cudaSuccess) return -1;
   k_reduce<<<10, 128, 0, stream>>>(nblk, atom_vir, reduce_out);

@@ -35,6 +35,8 @@ struct B2Args {
   // 1 / (rc - r1) per species pair as an FP32 hi/lo split (the Chebyshev
   // argument without a per-pair division or a rounded reciprocal)
   float cinv_hi[kMaxSpecies * kMaxSpecies], cinv_lo[kMaxSpecies * kMaxSpecies];
+  // the same as an FP64 hi/lo split (0: rc <= r1, the kernels divide)
+  double cinv64_hi[kMaxSpecies * kMaxSpecies], cinv64_lo[kMaxSpecies * kMaxSpecies];
   size_t smem_per_warp;      // filled by the launcher
   size_t smem_per_warp_adj;  // filled by the launcher
 };

@@ -17,6 +17,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace fpp {
@@ -30,6 +32,9 @@ struct HarmonicTables {
   double norm[(kMaxL + 1) * (kMaxL + 1)];
   float norm_hi[(kMaxL + 1) * (kMaxL + 1)];
   float norm_lo[(kMaxL + 1) * (kMaxL + 1)];
+  // norm * (2m-1)!! / D_lm: the factor of Q_l^m when the division-free
+  // recurrence starts from Q_m^m = 1 (FP64 kernels with lmax known)
+  double norm_q[(kMaxL + 1) * (kMaxL + 1)];
   double dfact[kMaxL + 1];
   float dfact_f[kMaxL + 1];  // exact in FP32 (at most 15!! = 2027025)
 };
@@ -52,9 +57,9 @@ static __device__ __noinline__ void cosine_cutoff(T r, T rc, T &fc, T &dfc) {
   dfc = -pi * sin_t(pi * r / rc) / (T(2) * rc);
 }
 
-// FP32: the argument is (r - r1) (cinv_hi + cinv_lo) with the reciprocal
-// 1 / (rc - r1) split hi/lo in FP64 (FP32 callers always pass it); FP64: the
-// correctly rounded division.
+// The argument is (r - r1) (cinv_hi + cinv_lo) with the reciprocal 1 / (rc - r1)
+// split hi/lo (FP32 callers always pass it); FP64 callers that pass none get
+// correctly rounded divisions.
 template <typename T>
 __device__ __forceinline__ void radial_basis(T r, T r1, T rc, int N, int cutoff_kind,
                                              T *out_g, T *out_dg, int stride,
@@ -78,6 +83,11 @@ __device__ __forceinline__ void radial_basis(T r, T r1, T rc, int N, int cutoff_
   // a branch around it was never taken.
   T c, x;
   if constexpr (sizeof(T) == 4) {
+    c = cinv_hi;
+    x = fma_t(r - r1, cinv_hi, (r - r1) * cinv_lo);
+  } else if (cinv_hi != T(0)) {
+    // a division is a dozen FP64 instructions; the split reciprocal rounds the
+    // argument as well
     c = cinv_hi;
     x = fma_t(r - r1, cinv_hi, (r - r1) * cinv_lo);
   } else {
@@ -126,6 +136,11 @@ __device__ __forceinline__ void radial_basis_reg(T r, T r1, T rc, int N, int cut
   const bool inside = !(r < r1 || r > rc);
   T c, x;
   if constexpr (sizeof(T) == 4) {  // split reciprocal, as in radial_basis
+    c = cinv_hi;
+    x = fma_t(r - r1, cinv_hi, (r - r1) * cinv_lo);
+  } else if (cinv_hi != T(0)) {
+    // a division is a dozen FP64 instructions; the split reciprocal rounds the
+    // argument as well
     c = cinv_hi;
     x = fma_t(r - r1, cinv_hi, (r - r1) * cinv_lo);
   } else {
@@ -380,6 +395,111 @@ __device__ __forceinline__ void harmonics_visit_f2(float x, float y, float z, in
       if (m > 0) emit(l * l + l - m, B, Bxy);
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 harmonics with lmax = L known.  FP64 issues two per clock and SM, so the
+// kernels that use them are bound by the count of FP64 instructions: no
+// divisions (the recurrence carries D_lm, divided out by norm_q), no integer
+// conversions (the loops unroll, the factors are constants), and the extension
+// off the sphere that is cheapest: Q_l^m as a polynomial in z alone, whose
+// gradient differs from the solid harmonic's by a radial part that the
+// projection removes.
+// ---------------------------------------------------------------------------
+
+// visit(l, m, N_lm Q_l^m(z), N_lm dQ_l^m/dz) for m <= l <= L, l fastest.
+template <int L, int M, bool kGrad, typename Visit>
+__device__ __forceinline__ void legendre64_column(double z, Visit visit) {
+  double q1 = 1.0, q2 = 0.0, d1 = 0.0, d2 = 0.0;
+#pragma unroll
+  for (int l = M; l <= L; l++) {
+    double q, d = 0.0;
+    if (l == M) {
+      q = 1.0;
+    } else if (l == M + 1) {
+      q = double(2 * M + 1) * z;
+      d = double(2 * M + 1);
+    } else {
+      const double a = double(2 * l - 1);
+      const double b = double((l + M - 1) * (l - 1 >= M + 2 ? l - 1 - M : 1));
+      const double az = a * z;
+      q = fma(az, q1, -b * q2);
+      if (kGrad) d = fma(az, d1, fma(a, q1, -b * d2));
+    }
+    q2 = q1;
+    q1 = q;
+    d2 = d1;
+    d1 = d;
+    const double n = c_harm.norm_q[l * (kMaxL + 1) + M];
+    visit(l, l == M ? n : n * q, l == M ? 0.0 : n * d);
+  }
+}
+
+template <int L, int M, typename F>
+__device__ __forceinline__ void for_each_order(double ux, double uy, double A, double B,
+                                               double Ap, double Bp, F &f) {
+  if constexpr (M <= L) {
+    // A, B = Re, Im (x + i y)^M;  Ap, Bp those of M - 1
+    f(std::integral_constant<int, M>{}, A, B, Ap, Bp);
+    for_each_order<L, M + 1>(ux, uy, fma(ux, A, -(uy * B)), fma(uy, A, ux * B), A, B, f);
+  }
+}
+
+// Y_lm of the unit vector (ux, uy, uz) at out[lm * stride].
+template <int L>
+__device__ __forceinline__ void harmonics64(double ux, double uy, double uz, double *out,
+                                            int stride) {
+  auto order = [&](auto mc, double A, double B, double, double) {
+    constexpr int m = decltype(mc)::value;
+    legendre64_column<L, m, false>(uz, [&](int l, double nq, double) {
+      out[(l * l + l + m) * stride] = nq * A;
+      if (m > 0) out[(l * l + l - m) * stride] = nq * B;
+    });
+  };
+  for_each_order<L, 0>(ux, uy, 1.0, 0.0, 0.0, 0.0, order);
+}
+
+// For weights (a, b) = weight(lm):  fr = sum b Y_lm(u)  and  g = sum a grad Y_lm
+// (r) times r, tangential to u.  Per lm three multiply-adds into the sums over l
+// of its order m; the trigonometric factors enter once per order.
+template <int L, typename Weight>
+__device__ __forceinline__ void harmonics64_adjoint(double ux, double uy, double uz,
+                                                    Weight weight, double (&g)[3],
+                                                    double &fr) {
+  double gx = 0.0, gy = 0.0, gz = 0.0, s = 0.0;
+  auto order = [&](auto mc, double A, double B, double Ap, double Bp) {
+    constexpr int m = decltype(mc)::value;
+    double PA = 0.0, PB = 0.0, QA = 0.0, QB = 0.0, RA = 0.0, RB = 0.0;
+    legendre64_column<L, m, true>(uz, [&](int l, double nq, double nd) {
+      const double2 w = weight(l * l + l + m);
+      PA = fma(nq, w.x, PA);
+      if (l > m) QA = fma(nd, w.x, QA);
+      RA = fma(nq, w.y, RA);
+      if (m > 0) {
+        const double2 v = weight(l * l + l - m);
+        PB = fma(nq, v.x, PB);
+        if (l > m) QB = fma(nd, v.x, QB);
+        RB = fma(nq, v.y, RB);
+      }
+    });
+    if constexpr (m == 0) {
+      gz += QA;
+      s += RA;
+    } else {
+      // d(A, B)/dx = m (Ap, Bp),  d(A, B)/dy = m (-Bp, Ap)
+      const double ma = double(m) * Ap, mb = double(m) * Bp;
+      gx = fma(PA, ma, fma(PB, mb, gx));
+      gy = fma(PB, ma, fma(-PA, mb, gy));
+      gz = fma(QA, A, fma(QB, B, gz));
+      s = fma(RA, A, fma(RB, B, s));
+    }
+  };
+  for_each_order<L, 0>(ux, uy, 1.0, 0.0, 0.0, 0.0, order);
+  const double ug = fma(ux, gx, fma(uy, gy, uz * gz));
+  g[0] = fma(-ug, ux, gx);
+  g[1] = fma(-ug, uy, gy);
+  g[2] = fma(-ug, uz, gz);
+  fr = s;
 }
 
 }  // namespace fpp

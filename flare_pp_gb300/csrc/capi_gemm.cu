@@ -14,11 +14,12 @@ namespace fpp {
 int ozaki_split(OzakiOperand &op, int rows, int K, const double *X, long long ldx,
                 cudaStream_t st) {
   const OzakiShape sh = ozaki_shape(rows, K);
-  FPP_TRY(op.planes.reserve(std::max<size_t>(sh.plane_bytes, 16)));
-  FPP_TRY(op.exps.reserve(sizeof(int) * std::max(rows, 1)));
+  // one allocation: the planes, then the row exponents
+  FPP_TRY(op.buf.reserve(sh.plane_bytes + sizeof(int) * (size_t)std::max(rows, 1)));
   op.rows = rows;
   op.K = K;
-  if (launch_ozaki_split(rows, K, X, ldx, op.planes.as<__half>(), op.exps.as<int>(), st) != 0)
+  op.exps_at = sh.plane_bytes;
+  if (launch_ozaki_split(rows, K, X, ldx, op.planes(), op.exps(), st) != 0)
     return fail(FPP_ERR_CUDA, "digit-plane split launch failed");
   return FPP_OK;
 }
@@ -34,7 +35,7 @@ int ozaki_const(OzakiOperand &op, int rows, int K, const double *X, long long ld
 }
 
 OzakiMat ozaki_mat(const OzakiOperand &op) {
-  return OzakiMat{op.planes.as<__half>(), op.exps.as<int>(), op.rows, op.K};
+  return OzakiMat{op.planes(), op.exps(), op.rows, op.K};
 }
 
 int ozaki_run(const OzakiProblem *probs, int n, DeviceStatus *status, cudaStream_t st,

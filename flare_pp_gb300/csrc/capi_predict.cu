@@ -124,8 +124,6 @@ int forward64(fpp_structure *s, const B2Args &a0, const int *pair_tab, bool want
   FPP_TRY(S.c64.reserve(sizeof(double) * std::max(1, S.noa) * sb));
   FPP_TRY(S.norm64.reserve(sizeof(double) * std::max(1, S.noa)));
   FPP_TRY(reserve_zero(S.p64, want_p ? sizeof(double) * std::max(1, S.noa) * a.n_d : 8, st));
-  FPP_TRY(reserve_zero(S.V64, sizeof(double) * (size_t)s->total_rows * ldp, st));
-  FPP_TRY(reserve_zero(S.w64, sizeof(double) * (size_t)s->total_rows * ldp, st));
   FPP_TRY(reserve_zero(S.phat64, sizeof(double) * (size_t)s->total_rows * ldp, st));
   if (launch_b2_forward<double>(a, neigh_of(S), S.species.as<int>(),
                                 s->row_of_atom.as<int>(), pair_tab, S.c64.as<double>(),
@@ -797,6 +795,7 @@ static int contract64(fpp_model *m, fpp_structure *s, const double *phat, int ld
                       cudaStream_t st) {
   StructureState &S = s->st;
   const int nd = m->n_d;
+  FPP_TRY(S.V64.reserve(sizeof(double) * (size_t)s->total_rows * ldp));
   OzakiProblem q[kOzakiMaxGroups];
   int nq = 0;
   for (int sp = 0; sp < m->n_species; sp++) {
@@ -1585,6 +1584,7 @@ int fpp_predict(fpp_model *m, fpp_structure *s, double *mean_efs, double *varian
   FPP_CUDA(cudaMemsetAsync(rown.ptr, 0, sizeof(double) * s->total_rows, st));
   FPP_CUDA(cudaMemsetAsync(E.ptr, 0, sizeof(double) * s->total_rows, st));
   FPP_CUDA(cudaMemsetAsync(zc.ptr, 0, sizeof(double) * s->total_rows, st));
+  FPP_TRY(S.w64.reserve(sizeof(double) * (size_t)s->total_rows * ldp));
   FPP_CUDA(cudaMemsetAsync(S.w64.ptr, 0, sizeof(double) * (size_t)s->total_rows * ldp, st));
   if (launch_gather_rows(noa, s->row_of_atom.as<int>(), S.norm64.as<double>(),
                          rown.as<double>(), st) != 0)

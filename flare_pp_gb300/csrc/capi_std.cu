@@ -216,7 +216,8 @@ int fpp_std_atom_compute(fpp_model *m, int32_t nlocal, int32_t nall, const doubl
   DevBuf q, rown, K, V, out;
   FPP_TRY(out.reserve(sizeof(double) * inum));
   if (use_map) {
-    // y = M_s phat for the rows of species s (into V64, sized by forward64)
+    // y = M_s phat for the rows of species s
+    FPP_TRY(S.V64.reserve(sizeof(double) * (size_t)s->total_rows * ldp));
     for (int sp = 0; sp < m->n_species; sp++) {
       if (s->n_rows[sp] == 0) continue;
       FPP_CUBLAS_STD(cublasDgemm(h, CUBLAS_OP_T, CUBLAS_OP_N, nd, s->n_rows[sp], nd, &one,

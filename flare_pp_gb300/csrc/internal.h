@@ -1,5 +1,6 @@
 // Internal host-side state behind the C ABI handles.
 #pragma once
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstddef>
@@ -46,9 +47,12 @@ struct DevBuf {
 // tensor-core GEMM (gemm_ozaki.h).  ready: a constant operand of a model whose
 // planes are up to date (reset where the matrix changes).
 struct OzakiOperand {
-  DevBuf planes, exps;
+  DevBuf buf;
+  size_t exps_at = 0;
   int rows = 0, K = 0;
   bool ready = false;
+  __half *planes() const { return buf.as<__half>(); }
+  int *exps() const { return reinterpret_cast<int *>(buf.as<char>() + exps_at); }
 };
 
 // Workspace of that GEMM (both operands, status word), kept between calls.
