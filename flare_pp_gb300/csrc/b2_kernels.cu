@@ -775,8 +775,8 @@ __device__ __forceinline__ double w_mixed2(const AdjArgs &g, int si, int nd, flo
 }
 
 // w = dE/dp of one atom into w_s[nd] (all lanes), returning the atom energy:
-// from the contraction V (mapped power 2), the beta vector (power 1), or
-// given per operand row (kernel form).
+// from the contraction V (mapped power 2), the beta vector (power 1), or the
+// kernel form's G rows.
 template <typename T, typename Store>
 __device__ __forceinline__ double adjoint_w(const B2Args &a, const AdjArgs &g, int si,
                                             int row, double nrm, float2 nrm32, Store store,
@@ -843,9 +843,12 @@ __device__ __forceinline__ double adjoint_w(const B2Args &a, const AdjArgs &g, i
       else
         store(d, T((float(g.beta1[(size_t)si * nd + d]) - ef * ph) * inv));
     }
-  } else {  // kWGiven: dE/dp supplied per operand row (kernel form)
-    for (int d = lane; d < nd; d += 32) store(d, T(g.w_given[(size_t)row * g.ldp + d]));
-    e = g.e_given ? g.e_given[row] : 0.0;
+  } else {  // kWKernel: dE/dp = (G - (sum_k C z) phat) / |p| (kernel form)
+    const double zc = g.zc_given[row], inv = nrm >= 1e-8 ? 1.0 / nrm : 0.0;
+    for (int d = lane; d < nd; d += 32)
+      store(d, T(fma(-zc, g.phat64[(size_t)row * g.ldp + d], g.V64[(size_t)row * g.ldv + d]) *
+                 inv));
+    e = g.e_given[row];
   }
   return e;
 }

@@ -47,7 +47,7 @@ inline __host__ __device__ int u_row_stride(const B2Args &a) {
   return a.n_species * a.N * a.H;
 }
 
-enum WMode { kWFromV2 = 0, kWFromV1 = 1, kWGiven = 2 };
+enum WMode { kWFromV2 = 0, kWFromV1 = 1, kWKernel = 2 };
 
 struct AdjArgs {
   int mode;              // WMode
@@ -67,8 +67,8 @@ struct AdjArgs {
   float c0_hi[kMaxSpecies], c0_lo[kMaxSpecies];  // the same as float-float
   // mapped power 1: beta vector per species [n_species][n_d]
   const double *beta1;
-  // given dE/dp and energies per operand row (row stride ldp)
-  const double *w_given;
+  // kernel form: V64 = G = C dhat and phat64 rows; per row E and sum_k C z
+  const double *zc_given;
   const double *e_given;
   DeviceStatus *status;  // staged adjoint: where a wait that ran out is recorded
 };

@@ -484,15 +484,18 @@ int fpp_model_set_sparse(fpp_model *m, int32_t species, int32_t n_sparse,
   FPP_TRY(sp.d_desc.reserve(sizeof(double) * n1 * nd));
   FPP_TRY(sp.d_dhat.reserve(sizeof(double) * n1 * nd));
   FPP_TRY(sp.d_norms.reserve(sizeof(double) * n1));
-  FPP_TRY(sp.d_alpha.reserve(sizeof(double) * n1));
+  FPP_TRY(sp.d_calpha.reserve(sizeof(double) * n1));
+  sp.oz_dhat.ready = sp.oz_dhatT.ready = sp.oz_Linv.ready = false;
+  m->oz_Linv.ready = m->oz_RinvT.ready = false;
   if (n_sparse) {
     FPP_CUDA(cudaMemcpy(sp.d_desc.ptr, descriptors, sizeof(double) * n_sparse * nd, cudaMemcpyHostToDevice));
     FPP_CUDA(cudaMemcpy(sp.d_dhat.ptr, dhat.data(), sizeof(double) * n_sparse * nd, cudaMemcpyHostToDevice));
     FPP_CUDA(cudaMemcpy(sp.d_norms.ptr, norms, sizeof(double) * n_sparse, cudaMemcpyHostToDevice));
     // empty sparse environments carry no weight (normalized_dot_product.cpp:157)
     std::vector<double> aeff(n_sparse);
-    for (int k = 0; k < n_sparse; k++) aeff[k] = norms[k] >= 1e-8 ? alpha[k] : 0.0;
-    FPP_CUDA(cudaMemcpy(sp.d_alpha.ptr, aeff.data(), sizeof(double) * n_sparse, cudaMemcpyHostToDevice));
+    const double f = m->sigma * m->sigma * m->power;
+    for (int k = 0; k < n_sparse; k++) aeff[k] = norms[k] >= 1e-8 ? f * alpha[k] : 0.0;
+    FPP_CUDA(cudaMemcpy(sp.d_calpha.ptr, aeff.data(), sizeof(double) * n_sparse, cudaMemcpyHostToDevice));
   }
   int off = 0;
   for (auto &x : m->sp) {
@@ -511,6 +514,7 @@ int fpp_model_set_R_inv(fpp_model *m, int32_t n, const double *R_inv) {
   FPP_TRY(m->R_inv.reserve(sizeof(double) * std::max(1, n) * std::max(1, n)));
   if (n) FPP_CUDA(cudaMemcpy(m->R_inv.ptr, R_inv, sizeof(double) * n * n, cudaMemcpyHostToDevice));
   m->has_R_inv = true;
+  m->oz_RinvT.ready = false;
   // upper triangular (the QR solve's): the variance products skip its zeros
   bool upper = true;
   for (int i = 1; i < n && upper; i++)
@@ -1394,118 +1398,130 @@ int fpp_predict_energy_uncertainty(fpp_model *m, fpp_structure *s, double *energ
   a.noa = noa;
   FPP_TRY(forward64(s, a, m->pair_tab.as<int>(), false, st));
   const int R = s->total_rows;
-  cublasHandle_t h;
-  FPP_TRY(get_cublas(m, st, &h));
-  const double one = 1.0, zero = 0.0;
-  DevBuf rown, K, kE, ones, al, y, Q, q;
-  FPP_TRY(rown.reserve(sizeof(double) * std::max(1, R)));
-  FPP_CUDA(cudaMemsetAsync(rown.ptr, 0, sizeof(double) * R, st));
-  if (launch_gather_rows(noa, s->row_of_atom.as<int>(), S.norm64.as<double>(),
-                         rown.as<double>(), st) != 0)
+  const double *phat = S.phat64.as<double>();
+  // per row: |p|, q = |L_inv k|^2; per sparse environment: k_E, y = R_inv^T k_E
+  FPP_TRY(m->kf_rows.reserve(sizeof(double) * 2 * std::max(1, R)));
+  double *rown = m->kf_rows.as<double>(), *q = rown + R;
+  FPP_CUDA(cudaMemsetAsync(rown, 0, sizeof(double) * 2 * R, st));
+  if (launch_gather_rows(noa, s->row_of_atom.as<int>(), S.norm64.as<double>(), rown, st) != 0)
     return fail(FPP_ERR_CUDA, "gather launch failed");
-  // per species block: K_s[c][k] = k(atom c, sparse k) (column-major S_s x
-  // n_rows_s, at the block's row offset times S_s); only the energy column of
-  // the kernel matrix is needed, so no force or stress columns are formed
+  // per species block: K_s[c][k] = k(atom c, sparse k), rows of ldk entries; only
+  // the energy column of the kernel matrix is needed, so no force or stress
+  // columns are formed
   std::vector<size_t> koff(m->n_species + 1, 0);
-  for (int sp = 0; sp < m->n_species; sp++)
-    koff[sp + 1] = koff[sp] + (size_t)m->sp[sp].n_sparse * std::max(s->n_rows[sp], 0);
-  FPP_TRY(K.reserve(sizeof(double) * std::max<size_t>(1, koff[m->n_species])));
-  FPP_TRY(kE.reserve(sizeof(double) * std::max(1, n)));
-  FPP_CUDA(cudaMemsetAsync(kE.ptr, 0, sizeof(double) * std::max(1, n), st));
-  int max_rows = 1;
-  for (int sp = 0; sp < m->n_species; sp++) max_rows = std::max(max_rows, s->n_rows[sp]);
-  FPP_TRY(ones.reserve(sizeof(double) * max_rows));
-  {
-    std::vector<double> o(max_rows, 1.0);
-    FPP_CUDA(cudaMemcpyAsync(ones.ptr, o.data(), sizeof(double) * max_rows,
-                             cudaMemcpyHostToDevice, st));
-    FPP_CUDA(cudaStreamSynchronize(st));
-  }
+  std::vector<int> ldk(m->n_species, 0);
+  size_t partial = 1;
   for (int sp = 0; sp < m->n_species; sp++) {
-    const int Ss = m->sp[sp].n_sparse, nsa = s->n_rows[sp];
+    ldk[sp] = round_up(std::max(m->sp[sp].n_sparse, 1), 4);  // 32-byte rows
+    koff[sp + 1] = koff[sp] + (size_t)ldk[sp] * s->n_rows[sp];
+    partial = std::max(partial, envs_colsum_partial(s->n_rows[sp], m->sp[sp].n_sparse));
+  }
+  FPP_TRY(m->kf_z.reserve(sizeof(double) * std::max<size_t>(1, koff[m->n_species])));
+  FPP_TRY(m->kf_cols.reserve(sizeof(double) * (2 * (size_t)std::max(1, n) + partial)));
+  double *K = m->kf_z.as<double>();
+  double *kE = m->kf_cols.as<double>(), *y = kE + n, *part = y + n;
+  FPP_CUDA(cudaMemsetAsync(kE, 0, sizeof(double) * n, st));
+  DeviceStatus *status;
+  FPP_TRY(ozaki_status(m->oz, st, &status));
+  // z[c][k] = phat_c . dhat_k on the tensor cores, FP64-accurate, all species in
+  // one launch
+  FPP_TRY(ozaki_split(S.oz_p, R, nd, phat, ldp, st));
+  OzakiProblem prob[kOzakiMaxGroups];
+  int np = 0;
+  for (int sp = 0; sp < m->n_species; sp++) {
+    auto &M = m->sp[sp];
+    const int Ss = M.n_sparse, nsa = s->n_rows[sp];
     if (Ss == 0 || nsa == 0) continue;
-    double *C = K.as<double>() + koff[sp];
-    const double *Ph = S.phat64.as<double>() + (size_t)s->row_off[sp] * ldp;
-    // z[c][k] = phat_c . dhat_k on the tensor cores, FP64-accurate
-    FPP_TRY(ozaki_dgemm_nt(nsa, Ss, nd, Ph, ldp, m->sp[sp].d_dhat.as<double>(), nd, C, Ss,
-                           m->oz, st));
-    if (launch_envs_block(nsa, Ss, C, Ss, rown.as<double>() + s->row_off[sp],
-                          m->sp[sp].d_norms.as<double>(), m->sigma * m->sigma, m->power, C,
-                          Ss, st) != 0)
+    FPP_TRY(ozaki_const(M.oz_dhat, Ss, nd, M.d_dhat.as<double>(), nd, st));
+    prob[np++] = OzakiProblem{ozaki_mat(S.oz_p), ozaki_mat(M.oz_dhat), s->row_off[sp], nsa, Ss,
+                              K + koff[sp], ldk[sp], false};
+  }
+  FPP_TRY(ozaki_run(prob, np, status, st));
+  for (int sp = 0; sp < m->n_species; sp++)
+    // k in place of z, and k_E = sum over the species' atoms of k(atom, sparse)
+    if (launch_envs_block_colsum(s->n_rows[sp], m->sp[sp].n_sparse, K + koff[sp], ldk[sp],
+                                 rown + s->row_off[sp], m->sp[sp].d_norms.as<double>(),
+                                 m->sigma * m->sigma, m->power, part,
+                                 kE + m->sp[sp].sparse_offset, st) != 0)
       return fail(FPP_ERR_CUDA, "kernel block launch failed");
-    // k_E = sum over the species' atoms of k(atom, sparse)
-    FPP_CUBLAS(cublasDgemv(h, CUBLAS_OP_N, Ss, nsa, &one, C, Ss, ones.as<double>(), 1, &zero,
-                           kE.as<double>() + m->sp[sp].sparse_offset, 1));
-  }
-  FPP_TRY(ozaki_check_status(m->oz, st));
-  double e_mean = 0, e_var = 0;
-  if (energy) {
-    std::vector<double> h_al(std::max(n, 1), 0.0);
-    for (auto &x : m->sp)
-      for (int k = 0; k < x.n_sparse; k++) h_al[x.sparse_offset + k] = x.alpha[k];
-    FPP_TRY(al.reserve(sizeof(double) * h_al.size()));
-    FPP_CUDA(cudaMemcpyAsync(al.ptr, h_al.data(), sizeof(double) * h_al.size(),
-                             cudaMemcpyHostToDevice, st));
-    FPP_CUBLAS(cublasSetPointerMode(h, CUBLAS_POINTER_MODE_HOST));
-    FPP_CUBLAS(cublasDdot(h, n, kE.as<double>(), 1, al.as<double>(), 1, &e_mean));
-  }
-  if (energy_variance) {
+  if (energy_variance && n > 0) {
     // variance_efs[0] = |R_inv^T k_E|^2 (R_inv row-major: column-major R_inv^T)
-    FPP_TRY(y.reserve(sizeof(double) * std::max(1, n)));
-    FPP_CUBLAS(cublasDgemv(h, CUBLAS_OP_N, n, n, &one, m->R_inv.as<double>(), n,
-                           kE.as<double>(), 1, &zero, y.as<double>(), 1));
-    FPP_CUBLAS(cublasDdot(h, n, y.as<double>(), 1, y.as<double>(), 1, &e_var));
+    cublasHandle_t h;
+    FPP_TRY(get_cublas(m, st, &h));
+    const double one = 1.0, zero = 0.0;
+    FPP_CUBLAS(cublasDgemv(h, CUBLAS_OP_N, n, n, &one, m->R_inv.as<double>(), n, kE, 1, &zero,
+                           y, 1));
   }
   if (local_variances) {
     // q_c = |L_inv k_c|^2, species block by species block when L_inv is
     // block diagonal, else against the whole L_inv
-    FPP_TRY(q.reserve(sizeof(double) * std::max(1, R)));
-    FPP_CUDA(cudaMemsetAsync(q.ptr, 0, sizeof(double) * std::max(1, R), st));
+    np = 0;
     if (m->L_inv_species_blocks) {
-      FPP_TRY(Q.reserve(sizeof(double) * std::max<size_t>(1, koff[m->n_species])));
+      FPP_TRY(m->kf_q.reserve(sizeof(double) * std::max<size_t>(1, koff[m->n_species])));
+      double *Q = m->kf_q.as<double>();
       for (int sp = 0; sp < m->n_species; sp++) {
-        const int Ss = m->sp[sp].n_sparse, nsa = s->n_rows[sp], off = m->sp[sp].sparse_offset;
+        auto &M = m->sp[sp];
+        const int Ss = M.n_sparse, nsa = s->n_rows[sp], off = M.sparse_offset;
         if (Ss == 0 || nsa == 0) continue;
-        const double *Lb = m->L_inv.as<double>() + (size_t)off * n + off;
-        // Q[c][i] = sum_k K[c][k] L_inv[i][k] on the tensor cores
-        FPP_TRY(ozaki_dgemm_nt(nsa, Ss, Ss, K.as<double>() + koff[sp], Ss, Lb, n,
-                               Q.as<double>() + koff[sp], Ss, m->oz, st, m->L_inv_lower));
-        if (launch_row_sq(nsa, Ss, Q.as<double>() + koff[sp], Ss,
-                          q.as<double>() + s->row_off[sp], st) != 0)
-          return fail(FPP_ERR_CUDA, "row-norm launch failed");
+        // Q[c][i] = sum_k K[c][k] L_inv[i][k]
+        FPP_TRY(ozaki_split(M.oz_c, nsa, Ss, K + koff[sp], ldk[sp], st));
+        FPP_TRY(ozaki_const(M.oz_Linv, Ss, Ss, m->L_inv.as<double>() + (size_t)off * n + off, n,
+                            st));
+        prob[np++] = OzakiProblem{ozaki_mat(M.oz_c), ozaki_mat(M.oz_Linv), 0, nsa, Ss,
+                                  Q + koff[sp], ldk[sp], m->L_inv_lower};
       }
+      FPP_TRY(ozaki_run(prob, np, status, st));
+      for (int sp = 0; sp < m->n_species; sp++)
+        if (m->sp[sp].n_sparse > 0 &&
+            launch_row_sq(s->n_rows[sp], m->sp[sp].n_sparse, Q + koff[sp], ldk[sp],
+                          q + s->row_off[sp], st) != 0)
+          return fail(FPP_ERR_CUDA, "row-norm launch failed");
     } else {
-      DevBuf Kf;
-      FPP_TRY(Kf.reserve(sizeof(double) * (size_t)std::max(1, R) * std::max(1, n)));
-      FPP_CUDA(cudaMemsetAsync(Kf.ptr, 0, sizeof(double) * (size_t)R * n, st));
+      const int ldq = round_up(std::max(n, 1), 4);
+      const size_t rows = (size_t)std::max(1, R) * ldq;
+      FPP_TRY(m->kf_q.reserve(sizeof(double) * 2 * rows));
+      double *Kf = m->kf_q.as<double>(), *Q = Kf + rows;
+      FPP_CUDA(cudaMemsetAsync(Kf, 0, sizeof(double) * (size_t)R * ldq, st));
       for (int sp = 0; sp < m->n_species; sp++) {
         const int Ss = m->sp[sp].n_sparse, nsa = s->n_rows[sp];
         if (Ss == 0 || nsa == 0) continue;
-        FPP_CUDA(cudaMemcpy2DAsync(Kf.as<double>() + (size_t)s->row_off[sp] * n +
-                                       m->sp[sp].sparse_offset,
-                                   sizeof(double) * n, K.as<double>() + koff[sp],
-                                   sizeof(double) * Ss, sizeof(double) * Ss, nsa,
-                                   cudaMemcpyDeviceToDevice, st));
+        FPP_CUDA(cudaMemcpy2DAsync(Kf + (size_t)s->row_off[sp] * ldq + m->sp[sp].sparse_offset,
+                                   sizeof(double) * ldq, K + koff[sp], sizeof(double) * ldk[sp],
+                                   sizeof(double) * Ss, nsa, cudaMemcpyDeviceToDevice, st));
       }
-      FPP_TRY(Q.reserve(sizeof(double) * (size_t)std::max(1, R) * std::max(1, n)));
-      FPP_TRY(ozaki_dgemm_nt(R, n, n, Kf.as<double>(), n, m->L_inv.as<double>(), n,
-                             Q.as<double>(), n, m->oz, st, m->L_inv_lower));
-      if (launch_row_sq(R, n, Q.as<double>(), n, q.as<double>(), st) != 0)
-        return fail(FPP_ERR_CUDA, "row-norm launch failed");
+      if (n > 0) {
+        FPP_TRY(ozaki_split(m->oz.a, R, n, Kf, ldq, st));
+        FPP_TRY(ozaki_const(m->oz_Linv, n, n, m->L_inv.as<double>(), n, st));
+        prob[0] = OzakiProblem{ozaki_mat(m->oz.a), ozaki_mat(m->oz_Linv), 0, R, n, Q, ldq,
+                               m->L_inv_lower};
+        FPP_TRY(ozaki_run(prob, 1, status, st));
+        if (launch_row_sq(R, n, Q, ldq, q, st) != 0)
+          return fail(FPP_ERR_CUDA, "row-norm launch failed");
+      }
     }
-    std::vector<double> hq(R), hn(R);
-    FPP_TRY(ozaki_check_status(m->oz, st));
-    FPP_CUDA(cudaMemcpy(hq.data(), q.ptr, sizeof(double) * R, cudaMemcpyDeviceToHost));
-    FPP_CUDA(cudaMemcpy(hn.data(), rown.ptr, sizeof(double) * R, cudaMemcpyDeviceToHost));
+  }
+  // one synchronization: row scalars, k_E and y to the host
+  std::vector<double> hrow(2 * (size_t)std::max(1, R)), hcol(2 * (size_t)std::max(1, n));
+  if (local_variances)
+    FPP_CUDA(cudaMemcpyAsync(hrow.data(), rown, sizeof(double) * 2 * R, cudaMemcpyDeviceToHost,
+                             st));
+  if (n > 0 && (energy || energy_variance))
+    FPP_CUDA(cudaMemcpyAsync(hcol.data(), kE, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost,
+                             st));
+  FPP_TRY(ozaki_check_status(m->oz, st));
+  double e_mean = 0, e_var = 0;
+  for (auto &x : m->sp)
+    for (int k = 0; k < x.n_sparse; k++) e_mean += hcol[x.sparse_offset + k] * x.alpha[k];
+  for (int k = 0; k < n; k++) e_var += hcol[n + k] * hcol[n + k];
+  if (local_variances) {
     const double sig2 = m->sigma * m->sigma;
     std::vector<int> cnt(m->n_species, 0);
     for (int i = 0; i < noa; i++) {
       const int sp = S.species_host[i];
       const int row = s->row_off[sp] + cnt[sp]++;
-      local_variances[i] = (hn[row] >= 1e-8 ? sig2 : 0.0) - hq[row];
+      local_variances[i] = (hrow[row] >= 1e-8 ? sig2 : 0.0) - hrow[R + row];
     }
   }
-  FPP_CUDA(cudaStreamSynchronize(st));
   if (energy) *energy = e_mean;
   if (energy_variance) *energy_variance = e_var;
   return FPP_OK;
@@ -1537,10 +1553,10 @@ int fpp_predict(fpp_model *m, fpp_structure *s, double *mean_efs, double *varian
   const int noa = S.noa, nd = m->n_d, ldp = round_up(nd, 64);
   const int n_out = 1 + 3 * noa + 6;
   const int nst = m->n_sparse_total;
-  cublasHandle_t h;
-  FPP_TRY(get_cublas(m, st, &h));
-  const double one = 1.0, zero = 0.0;
   if (variance_efs) {
+    cublasHandle_t h;
+    FPP_TRY(get_cublas(m, st, &h));
+    const double one = 1.0, zero = 0.0;
     if (!m->has_R_inv) return fail(FPP_ERR_INVALID, "R_inv not set (fpp_model_set_R_inv)");
     DevBuf K, alpha, mean, V, var;
     FPP_TRY(envs_struc_device(m, s, st, K));
@@ -1576,52 +1592,73 @@ int fpp_predict(fpp_model *m, fpp_structure *s, double *mean_efs, double *varian
   B2Args a = m->args;
   a.noa = noa;
   FPP_TRY(forward64(s, a, m->pair_tab.as<int>(), false, st));
-  double *phat = S.phat64.as<double>();
-  DevBuf rown, E, zc, Z, G, DT;
-  FPP_TRY(rown.reserve(sizeof(double) * std::max(1, s->total_rows)));
-  FPP_TRY(E.reserve(sizeof(double) * std::max(1, s->total_rows)));
-  FPP_TRY(zc.reserve(sizeof(double) * std::max(1, s->total_rows)));
-  FPP_CUDA(cudaMemsetAsync(rown.ptr, 0, sizeof(double) * s->total_rows, st));
-  FPP_CUDA(cudaMemsetAsync(E.ptr, 0, sizeof(double) * s->total_rows, st));
-  FPP_CUDA(cudaMemsetAsync(zc.ptr, 0, sizeof(double) * s->total_rows, st));
-  FPP_TRY(S.w64.reserve(sizeof(double) * (size_t)s->total_rows * ldp));
-  FPP_CUDA(cudaMemsetAsync(S.w64.ptr, 0, sizeof(double) * (size_t)s->total_rows * ldp, st));
-  if (launch_gather_rows(noa, s->row_of_atom.as<int>(), S.norm64.as<double>(),
-                         rown.as<double>(), st) != 0)
+  const double *phat = S.phat64.as<double>();
+  const int R = s->total_rows;
+  // per row: |p|, E, sum_k C z
+  FPP_TRY(m->kf_rows.reserve(sizeof(double) * 3 * std::max(1, R)));
+  double *rown = m->kf_rows.as<double>(), *E = rown + R, *zc = E + R;
+  FPP_CUDA(cudaMemsetAsync(rown, 0, sizeof(double) * 3 * R, st));
+  if (launch_gather_rows(noa, s->row_of_atom.as<int>(), S.norm64.as<double>(), rown, st) != 0)
     return fail(FPP_ERR_CUDA, "gather launch failed");
-  FPP_TRY(G.reserve(sizeof(double) * (size_t)s->total_rows * ldp));
+  FPP_TRY(S.V64.reserve(sizeof(double) * (size_t)R * ldp));  // G
+  double *G = S.V64.as<double>();
+  std::vector<size_t> zoff(m->n_species + 1, 0);
+  std::vector<int> ldz(m->n_species, 0);
   for (int sp = 0; sp < m->n_species; sp++) {
-    const int Ss = m->sp[sp].n_sparse, nsa = s->n_rows[sp];
-    if (Ss == 0 || nsa == 0) continue;
-    const size_t r0 = s->row_off[sp];
-    FPP_TRY(Z.reserve(sizeof(double) * (size_t)nsa * Ss));
-    const double *Dh = m->sp[sp].d_dhat.as<double>();
-    // Z[i][k] = phat_i . dhat_k (tensor cores, FP64-accurate)
-    FPP_TRY(ozaki_dgemm_nt(nsa, Ss, nd, phat + r0 * ldp, ldp, Dh, nd, Z.as<double>(), Ss,
-                           m->oz, st));
-    if (launch_kernel_c(nsa, Ss, Z.as<double>(), Ss, m->sp[sp].d_alpha.as<double>(),
-                        rown.as<double>() + r0, m->sigma * m->sigma, m->power,
-                        E.as<double>() + r0, zc.as<double>() + r0, st) != 0)
-      return fail(FPP_ERR_CUDA, "kernel-form launch failed");
-    // G[i][d] = sum_k C[i][k] dhat_k[d] = (C Dhat^T^T): B operand Dhat^T (nd x S)
-    FPP_TRY(DT.reserve(sizeof(double) * (size_t)nd * Ss));
-    if (launch_transpose(Ss, nd, Dh, nd, DT.as<double>(), Ss, st) != 0)
-      return fail(FPP_ERR_CUDA, "transpose launch failed");
-    FPP_TRY(ozaki_dgemm_nt(nsa, nd, Ss, Z.as<double>(), Ss, DT.as<double>(), Ss,
-                           G.as<double>() + r0 * ldp, ldp, m->oz, st));
-    if (launch_kernel_w(nsa, nd, G.as<double>() + r0 * ldp, ldp, phat + r0 * ldp, ldp,
-                        zc.as<double>() + r0, rown.as<double>() + r0,
-                        S.w64.as<double>() + r0 * ldp, ldp, st) != 0)
-      return fail(FPP_ERR_CUDA, "kernel-form launch failed");
-    FPP_CUDA(cudaStreamSynchronize(st));  // Z is reused by the next species
+    ldz[sp] = round_up(std::max(m->sp[sp].n_sparse, 1), 4);  // 32-byte rows
+    zoff[sp + 1] = zoff[sp] + (size_t)ldz[sp] * s->n_rows[sp];
   }
-  FPP_TRY(ozaki_check_status(m->oz, st));
+  FPP_TRY(m->kf_z.reserve(sizeof(double) * std::max<size_t>(1, zoff[m->n_species])));
+  double *Z = m->kf_z.as<double>();
+  DeviceStatus *status;
+  FPP_TRY(ozaki_status(m->oz, st, &status));
+  // Z[i][k] = phat_i . dhat_k and, after C has taken its place, G[i][d] =
+  // sum_k C[i][k] dhat_k[d]: on the tensor cores, FP64-accurate, each product of
+  // all species in one launch
+  FPP_TRY(ozaki_split(S.oz_p, R, nd, phat, ldp, st));
+  OzakiProblem prob[kOzakiMaxGroups];
+  int np = 0;
+  for (int sp = 0; sp < m->n_species; sp++) {
+    auto &M = m->sp[sp];
+    const int Ss = M.n_sparse, nsa = s->n_rows[sp];
+    if (nsa > 0 && Ss == 0)
+      FPP_CUDA(cudaMemsetAsync(G + (size_t)s->row_off[sp] * ldp, 0,
+                               sizeof(double) * (size_t)nsa * ldp, st));
+    if (Ss == 0 || nsa == 0) continue;
+    FPP_TRY(ozaki_const(M.oz_dhat, Ss, nd, M.d_dhat.as<double>(), nd, st));
+    prob[np++] = OzakiProblem{ozaki_mat(S.oz_p), ozaki_mat(M.oz_dhat), s->row_off[sp], nsa, Ss,
+                              Z + zoff[sp], ldz[sp], false};
+  }
+  FPP_TRY(ozaki_run(prob, np, status, st));
+  np = 0;
+  for (int sp = 0; sp < m->n_species; sp++) {
+    auto &M = m->sp[sp];
+    const int Ss = M.n_sparse, nsa = s->n_rows[sp], r0 = s->row_off[sp];
+    if (Ss == 0 || nsa == 0) continue;
+    if (launch_kernel_c(nsa, Ss, Z + zoff[sp], ldz[sp], M.d_calpha.as<double>(), rown + r0,
+                        m->power, E + r0, zc + r0, st) != 0)
+      return fail(FPP_ERR_CUDA, "kernel-form launch failed");
+    FPP_TRY(ozaki_split(M.oz_c, nsa, Ss, Z + zoff[sp], ldz[sp], st));
+    if (!(M.oz_dhatT.ready && M.oz_dhatT.rows == nd && M.oz_dhatT.K == Ss)) {
+      DevBuf DT;  // dhat transposed, for its digit planes only
+      FPP_TRY(DT.reserve(sizeof(double) * (size_t)nd * Ss));
+      if (launch_transpose(Ss, nd, M.d_dhat.as<double>(), nd, DT.as<double>(), Ss, st) != 0)
+        return fail(FPP_ERR_CUDA, "transpose launch failed");
+      FPP_TRY(ozaki_const(M.oz_dhatT, nd, Ss, DT.as<double>(), Ss, st));
+    }
+    prob[np++] = OzakiProblem{ozaki_mat(M.oz_c), ozaki_mat(M.oz_dhatT), 0, nsa, nd,
+                              G + (size_t)r0 * ldp, ldp, false};
+  }
+  FPP_TRY(ozaki_run(prob, np, status, st));
   AdjArgs g;
   std::memset(&g, 0, sizeof(g));
-  g.mode = kWGiven;
+  g.mode = kWKernel;
   g.ldp = ldp;
-  g.w_given = S.w64.as<double>();
-  g.e_given = E.as<double>();
+  g.ldv = ldp;
+  g.V64 = G;
+  g.phat64 = phat;
+  g.zc_given = zc;
+  g.e_given = E;
   FPP_TRY(adjoint_buffers(S, sizeof(double), u_row_stride(a)));
   FPP_CUDA(cudaMemsetAsync(S.status.ptr, 0, sizeof(DeviceStatus), st));
   if (launch_b2_adjoint<double>(a, g, neigh_of(S), S.species.as<int>(),
@@ -1632,13 +1669,9 @@ int fpp_predict(fpp_model *m, fpp_structure *s, double *mean_efs, double *varian
                                 S.reduce_out.as<double>(), true, S.u.as<double>(),
                                 S.n_pairs, S.nbr_i.as<int>(), st) != 0)
     return fail(FPP_ERR_CUDA, "adjoint (FP64) launch failed");
-  double e, stress[6];
-  std::vector<double> F(3 * (size_t)noa);
-  FPP_TRY(finish_outputs(s, st, &e, F.data(), stress, nullptr, 0));
-  mean_efs[0] = e;
-  for (size_t k = 0; k < F.size(); k++) mean_efs[1 + k] = F[k];
-  for (int k = 0; k < 6; k++) mean_efs[1 + 3 * noa + k] = stress[k];
-  return FPP_OK;
+  FPP_TRY(finish_outputs(s, st, mean_efs, mean_efs + 1, mean_efs + 1 + 3 * (size_t)noa, nullptr,
+                         0));
+  return ozaki_check_status(m->oz, st);
 }
 
 }  // extern "C"

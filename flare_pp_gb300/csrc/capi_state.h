@@ -49,14 +49,16 @@ struct fpp_model {
     std::vector<double> norms, alpha;
     fpp::DevBuf d_desc;                 // double[n_sparse * n_d] unnormalised
     fpp::DevBuf d_dhat;                 // double[n_sparse * n_d] normalised (0 if empty)
-    fpp::DevBuf d_norms, d_alpha;       // double[n_sparse]
+    fpp::DevBuf d_norms;                // double[n_sparse]
+    fpp::DevBuf d_calpha;               // double[n_sparse] sigma^2 power alpha (0 if empty)
     fpp::DevBuf beta64;                 // double[n_d * ldb] dense symmetric
     fpp::DevBuf beta_hi, beta_lo;       // half[n_d_pad * ldb] split operands
     double beta_scale = 1;              // beta ~ (hi + lo/2048) / beta_scale
     std::vector<double> B_host;         // dense beta (n_d x n_d), power 2
     bool beta_finite = true;            // every entry of it
     // digit planes of the constant GEMM operands, split on first use
-    fpp::OzakiOperand oz_beta;
+    fpp::OzakiOperand oz_beta, oz_dhat, oz_dhatT, oz_Linv;
+    fpp::OzakiOperand oz_c;             // workspace: C (or K) rows of the species' atoms
   };
   std::vector<Species> sp;
   int beta_power = 0;                   // 0: no mapped coefficients yet
@@ -87,6 +89,11 @@ struct fpp_model {
   long long kuf_items = 0;              // (structure, atom) work items of it
   int last_pair_batches = 0;            // atom batches of the last pair compute
   fpp::OzakiWork oz;                    // kernel-form GEMM workspace
+  fpp::OzakiOperand oz_Linv;            // digit planes of L_inv, of R_inv^T
+  fpp::OzakiOperand oz_RinvT;
+  // kernel-form workspaces (grown on demand, kept between calls): per-row
+  // scalars, z / C / K blocks, second products, column sums and partials
+  fpp::DevBuf kf_rows, kf_z, kf_q, kf_cols;
   fpp_structure *batch = nullptr;       // packed structure of a batched prediction
   fpp::DevBuf batch_aoff, batch_poff, batch_sums, batch_src;
   // envs_struc workspace (grown on demand, kept between calls)

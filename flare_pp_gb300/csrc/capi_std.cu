@@ -121,6 +121,8 @@ int fpp_model_set_L_inv(fpp_model *m, int32_t n, const double *L_inv) {
         break;
       }
   m->L_inv_lower = lower;
+  m->oz_Linv.ready = false;
+  for (auto &x : m->sp) x.oz_Linv.ready = false;
   return FPP_OK;
 }
 

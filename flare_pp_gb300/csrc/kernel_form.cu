@@ -1,10 +1,11 @@
 // NormalizedDotProduct kernel form in FP64 (normalized_dot_product.cpp:115-210).
 //
 // Mean prediction through the adjoint (no stored derivatives):
-//   z = phat D^T (cuBLAS),  E_i = sig2 sum_k a_k z^p,  C = sig2 a p z^(p-1),
-//   G = C D (cuBLAS),       dE/dp_i = (G_i - (sum_k C_ik z_ik) phat_i) / |p_i|.
+//   z = phat D^T,  E_i = sig2 sum_k a_k z^p,  C = sig2 a p z^(p-1),
+//   G = C D,       dE/dp_i = (G_i - (sum_k C_ik z_ik) phat_i) / |p_i|
+// (products by the FP64-accurate tensor-core GEMM; dE/dp in the adjoint kernel).
 // Full kernel matrix (variance, training columns) through stored derivatives,
-// as the reference does: fd = D dp^T (cuBLAS), then the energy, force and
+// as the reference does: fd = D dp^T, then the energy, force and
 // stress columns assembled per sparse environment.
 #include <cuda_runtime.h>
 
@@ -28,48 +29,27 @@ __device__ __forceinline__ double powi(double x, double p) {
   return pow(x, p);
 }
 
-// One warp per operand row: E, C in place of z, zc = sum_k C z.
+// One warp per operand row: C in place of z, zc = sum_k C z, E = zc / power.
 __global__ void k_kernel_c(int rows, int S, double *__restrict__ Z, int ldz,
-                           const double *__restrict__ alpha_eff,
-                           const double *__restrict__ rownorm, double sig2,
-                           double power, double *__restrict__ E,
-                           double *__restrict__ zc) {
+                           const double *__restrict__ calpha,
+                           const double *__restrict__ rownorm, double power,
+                           double *__restrict__ E, double *__restrict__ zc) {
   const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
   const bool empty = !(rownorm[row] >= 1e-8);
-  double e = 0.0, c = 0.0;
+  double c = 0.0;
   for (int k = lane; k < S; k += 32) {
     const double z = Z[(size_t)row * ldz + k];
-    const double a = alpha_eff[k];
-    double ck = 0.0;
-    if (!empty) {
-      e += sig2 * a * powi(z, power);
-      ck = sig2 * a * power * powi(z, power - 1.0);
-      c += ck * z;
-    }
+    const double ck = empty ? 0.0 : calpha[k] * powi(z, power - 1.0);
+    if (!empty) c = fma(ck, z, c);
     Z[(size_t)row * ldz + k] = ck;
   }
-  e = wsum(e);
   c = wsum(c);
   if (lane == 0) {
-    E[row] = e;
+    E[row] = c / power;
     zc[row] = c;
   }
-}
-
-__global__ void k_kernel_w(int rows, int nd, const double *__restrict__ G, int ldg,
-                           const double *__restrict__ phat, int ldp,
-                           const double *__restrict__ zc,
-                           const double *__restrict__ rownorm, double *__restrict__ w,
-                           int ldw) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)rows * nd) return;
-  const int row = (int)(t / nd), d = (int)(t - (long long)row * nd);
-  const double n = rownorm[row];
-  double v = 0.0;
-  if (n >= 1e-8) v = (G[(size_t)row * ldg + d] - zc[row] * phat[(size_t)row * ldp + d]) / n;
-  w[(size_t)row * ldw + d] = v;
 }
 
 __global__ void k_gather_rows(int noa, const int *__restrict__ row_of_atom,
@@ -194,6 +174,54 @@ int launch_envs_block(int S1, int S2, const double *Z, int ldz, const double *n1
   return LAUNCH_OK;
 }
 
+// The same in place with the column sums: a thread per column and chunk of rows,
+// then a thread per column over the chunks (a separate pass over the block and a
+// matrix-vector product with ones before: two more reads of it).
+constexpr int kColsumRows = 64;
+__global__ void __launch_bounds__(128)
+k_envs_block_colsum(int rows, int S, double *__restrict__ Z, int ldz,
+                    const double *__restrict__ rownorm, const double *__restrict__ snorm,
+                    double sig2, double power, double *__restrict__ partial) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= S) return;
+  const bool live = snorm[k] >= 1e-8;
+  const int r0 = blockIdx.y * kColsumRows, r1 = min(rows, r0 + kColsumRows);
+  double sum = 0.0;
+#pragma unroll 8
+  for (int r = r0; r < r1; r++) {
+    double *z = Z + (size_t)r * ldz + k;
+    const double v = live && rownorm[r] >= 1e-8 ? sig2 * powi(*z, power) : 0.0;
+    *z = v;
+    sum += v;
+  }
+  partial[(size_t)blockIdx.y * S + k] = sum;
+}
+__global__ void __launch_bounds__(128)
+k_colsum_finish(int chunks, int S, const double *__restrict__ partial, double *__restrict__ out) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= S) return;
+  double sum = 0.0;
+#pragma unroll 8
+  for (int c = 0; c < chunks; c++) sum += partial[(size_t)c * S + k];
+  out[k] += sum;
+}
+
+size_t envs_colsum_partial(int rows, int S) {
+  return (size_t)ceil_div(rows, kColsumRows) * S;
+}
+
+int launch_envs_block_colsum(int rows, int S, double *Z, int ldz, const double *rownorm,
+                             const double *snorm, double sig2, double power, double *partial,
+                             double *out, cudaStream_t st) {
+  if (rows <= 0 || S <= 0) return 0;
+  const int chunks = ceil_div(rows, kColsumRows), cols = ceil_div(S, 128);
+  if (chunks > 65535) return -1;
+  k_envs_block_colsum<<<dim3(cols, chunks), 128, 0, st>>>(rows, S, Z, ldz, rownorm, snorm, sig2,
+                                                          power, partial);
+  k_colsum_finish<<<cols, 128, 0, st>>>(chunks, S, partial, out);
+  return LAUNCH_OK;
+}
+
 // row sums of squares: out[j] = sum_k V[j, k]^2
 __global__ void k_row_sq(int rows, int cols, const double *__restrict__ V, int ldv,
                          double *__restrict__ out) {
@@ -210,22 +238,11 @@ __global__ void k_row_sq(int rows, int cols, const double *__restrict__ V, int l
 }
 
 
-int launch_kernel_c(int rows, int S, double *Z, int ldz, const double *alpha_eff,
-                    const double *rownorm, double sig2, double power, double *E,
-                    double *zc, cudaStream_t st) {
+int launch_kernel_c(int rows, int S, double *Z, int ldz, const double *calpha,
+                    const double *rownorm, double power, double *E, double *zc,
+                    cudaStream_t st) {
   if (rows == 0) return 0;
-  k_kernel_c<<<ceil_div(rows, 4), 128, 0, st>>>(rows, S, Z, ldz, alpha_eff, rownorm,
-                                                sig2, power, E, zc);
-  return LAUNCH_OK;
-}
-
-int launch_kernel_w(int rows, int nd, const double *G, int ldg, const double *phat,
-                    int ldp, const double *zc, const double *rownorm, double *w,
-                    int ldw, cudaStream_t st) {
-  long long n = (long long)rows * nd;
-  if (n == 0) return 0;
-  k_kernel_w<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(rows, nd, G, ldg, phat, ldp,
-                                                          zc, rownorm, w, ldw);
+  k_kernel_c<<<ceil_div(rows, 4), 128, 0, st>>>(rows, S, Z, ldz, calpha, rownorm, power, E, zc);
   return LAUNCH_OK;
 }
 

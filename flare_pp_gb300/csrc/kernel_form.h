@@ -5,12 +5,11 @@
 #include "common.cuh"
 
 namespace fpp {
-int launch_kernel_c(int rows, int S, double *Z, int ldz, const double *alpha_eff,
-                    const double *rownorm, double sig2, double power, double *E,
-                    double *zc, cudaStream_t st);
-int launch_kernel_w(int rows, int nd, const double *G, int ldg, const double *phat,
-                    int ldp, const double *zc, const double *rownorm, double *w,
-                    int ldw, cudaStream_t st);
+// C = calpha z^(power - 1) in place of z (calpha = sigma^2 power alpha), per row
+// zc = sum_k C z and E = zc / power (sigma^2 sum_k alpha z^power).
+int launch_kernel_c(int rows, int S, double *Z, int ldz, const double *calpha,
+                    const double *rownorm, double power, double *E, double *zc,
+                    cudaStream_t st);
 int launch_gather_rows(int noa, const int *row_of_atom, const double *v_atom,
                        double *v_row, cudaStream_t st);
 int launch_envs_energy(int S, int ns, const double *ndm, int ldn, const double *snorm,
@@ -28,6 +27,13 @@ int launch_envs_stress(int S, int nq, const double *fkv, int ldf, const int *q_p
 int launch_envs_block(int S1, int S2, const double *Z, int ldz, const double *n1,
                       const double *n2, double sig2, double power, double *K, int ldk,
                       cudaStream_t st);
+// The kernel between atoms (rows of Z) and sparse environments in place of z,
+// and its column sums over the rows, out[k] += sum_i (out: S, zeroed by the
+// caller; partial: scratch of envs_colsum_partial(rows, S) doubles; fixed order).
+size_t envs_colsum_partial(int rows, int S);
+int launch_envs_block_colsum(int rows, int S, double *Z, int ldz, const double *rownorm,
+                             const double *snorm, double sig2, double power, double *partial,
+                             double *out, cudaStream_t st);
 int launch_row_sq(int rows, int cols, const double *V, int ldv, double *out,
                   cudaStream_t st);
 // The descriptor pairs of one species: flags[p] = 1 when pair p's central
