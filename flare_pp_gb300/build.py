@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libflare_pp_gb300.so")
-SOURCES = ["neighbors.cu", "b2_kernels.cu", "gemm_tc.cu", "kernel_form.cu",
+SOURCES = ["neighbors.cu", "b2_kernels.cu", "b3_real.cu", "gemm_tc.cu", "kernel_form.cu",
            "capi_core.cu", "capi_predict.cu", "capi_pair.cu", "capi_solve.cu",
            "capi_noalloc.cu", "capi_struc.cu", "capi_std.cu",
            "capi_likelihood.cu", "gemm_ozaki.cu", "capi_gemm.cu", "capi_batch.cu"]

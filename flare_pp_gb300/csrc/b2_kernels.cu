@@ -22,8 +22,10 @@
 #include <cmath>
 
 #include "basis.cuh"
+#include "b2_device.cuh"
 #include "b2_kernels.h"
 #include "b3.cuh"
+#include "b3_real.h"
 #include "common.cuh"
 #include "tc_prims.cuh"
 
@@ -101,23 +103,6 @@ int upload_harmonic_tables(cudaStream_t stream) {
   return e == cudaSuccess ? 0 : -1;
 }
 
-// Running sum; compensated (Neumaier) when T is float.
-template <typename T> struct Acc {
-  T s = T(0), c = T(0);
-  __device__ __forceinline__ void add(T x) {
-    if (sizeof(T) == 4) {
-      T t = s + x;
-      if (fabs_t(s) >= fabs_t(x))
-        c += (s - t) + x;
-      else
-        c += (x - t) + s;
-      s = t;
-    } else {
-      s += x;
-    }
-  }
-};
-
 // x^2 + y^2 + z^2 of a pair vector, rounded as the host computes it.
 __device__ __forceinline__ double rsq_exact(const dvec4 &r) {
   return dadd(dadd(dmul(r.y, r.y), dmul(r.z, r.z)), dmul(r.w, r.w));
@@ -129,34 +114,6 @@ __device__ __forceinline__ double rsq_exact(const dvec4 &r) {
 static __device__ __noinline__ bool strict_keep(const dvec4 *__restrict__ rel, long long p,
                                                 double rc) {
   return rsq_exact(rel[p]) < dmul(rc, rc);
-}
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// Error-free sum a + b = s + e (Knuth's two-sum), FP32.
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
-  s = a + b;
-  const float bb = s - a;
-  e = (a - (s - bb)) + (b - bb);
-}
-
-// Warp sum of the float-float values (hi, lo), kept as float-float: FP32
-// arithmetic only (FP64 instructions are scarce on this GPU).
-__device__ __forceinline__ void ff_warp_sum(float &hi, float &lo) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float h2 = __shfl_xor_sync(0xffffffffu, hi, o);
-    const float l2 = __shfl_xor_sync(0xffffffffu, lo, o);
-    float s, e;
-    two_sum(hi, h2, s, e);
-    e += lo + l2;
-    hi = s + e;
-    lo = e - (hi - s);
-  }
 }
 
 // Descriptor shape known at compile time for the common settings (N, lmax,
@@ -239,13 +196,13 @@ __host__ __device__ inline FwdLayout<T> fwd_layout(const B2Args &a) {
   // c rows padded to a multiple of 4 entries (16-byte aligned rows)
   const int sbp = a.n_species * a.N * ((a.H + 3) & ~3);
   size_t st = sizeof(T) * ((size_t)L.W * L.GP + (size_t)a.H * (L.W + 1));
-  size_t pb = sizeof(T) * (size_t)a.n_d;
+  size_t pb = a.c_only ? 0 : sizeof(T) * (size_t)a.n_d;
   L.stage = ((st > pb ? st : pb) + 15) & ~(size_t)15;
   // FP32: running sums only (compensated within a window); FP64: running
   // sums and their compensation terms across windows
   L.csum = (sizeof(T) * (sizeof(T) == 8 ? 2 : 1) * (size_t)sbp + 15) & ~(size_t)15;
   L.lists = (sizeof(int) * ((size_t)a.n_species * L.W + 2 * L.W + a.n_species) + 15) & ~(size_t)15;
-  L.cz = a.kind == kB3
+  L.cz = a.kind == kB3 && !a.c_only
              ? (sizeof(T) * 2 * (size_t)a.n_species * a.N * (a.H + 1) + 15) & ~(size_t)15
              : 0;
   L.total = L.stage + L.csum + L.lists + L.cz;
@@ -449,6 +406,7 @@ k_b2_forward(B2Args a, const int *__restrict__ offset,
     }
     c_out[(size_t)atom * sb + k] = v;
   }
+  if (a.c_only) return;  // the coupling runs in b3_real.cu
   __syncwarp();
   // ---- 3. B2 contraction per radial pair q, all l (B3: per radial triple) ----
   const int L1 = LMAX + 1;
@@ -459,9 +417,7 @@ k_b2_forward(B2Args a, const int *__restrict__ offset,
     V2<T> *z = reinterpret_cast<V2<T> *>(base + Lay.stage + Lay.csum + Lay.lists);
     b3_to_complex2<T>(c_s, NS * N, H, z, lane, HP);
     __syncwarp();
-    // FP32 at lmax 3 (the B3 workload shape): the contraction unrolled
-    constexpr int kB3L = (sizeof(T) == 4 && SH::kL1 == 4) ? 3 : -1;
-    b3_contract<T, kB3L>(a.lmax, a.n_ls, a.n_tri, H, pair_tab, z, p_s, lane);
+    b3_contract<T>(a.lmax, a.n_ls, a.n_tri, H, pair_tab, z, p_s, lane);
     __syncwarp();
     for (int d = lane; d < nd; d += 32) nacc.add(p_s[d] * p_s[d]);
   }
@@ -626,16 +582,9 @@ k_b2_forward(B2Args a, const int *__restrict__ offset,
     inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
     invf = float(inv);
   } else {
-    // |p|^2 as float-float; sqrt and 1/sqrt by one correction step of the
-    // FP32 values (relative error ~1 ulp of FP32), no FP64 arithmetic
-    float hi = float(nacc.s), lo = float(nacc.c);
-    ff_warp_sum(hi, lo);
-    const float r0 = sqrtf(hi);
-    const float rc = r0 > 0.0f ? (fmaf(-r0, r0, hi) + lo) / (2.0f * r0) : 0.0f;
-    const float y0 = r0 > 0.0f ? 1.0f / r0 : 0.0f;
-    invf = fmaf(-y0 * y0, rc, y0);
-    nrm_hi = r0;
-    nrm_lo = rc;
+    const float2 n2 = norm_ff(Acc<float>{float(nacc.s), float(nacc.c)}, invf);
+    nrm_hi = n2.x;
+    nrm_lo = n2.y;
   }
   if (lane == 0) {
     if (sizeof(T) == 4)  // FP32 kernels: |p| as a float-float pair in the 8-byte slot
@@ -646,28 +595,9 @@ k_b2_forward(B2Args a, const int *__restrict__ offset,
   __syncwarp();
   const int row = row_of_atom[atom];
   if (sizeof(T) == 4 && phat_hi && !p_out && !phat64 && (nd & 3) == 0) {
-    // split operand only: four entries per lane, 16-byte reads, 8-byte writes
-    const float4 *P4 = reinterpret_cast<const float4 *>(p_s);
-    const float4 *B4 = reinterpret_cast<const float4 *>(pbar + (size_t)si * nd);
-    uint2 *H4 = reinterpret_cast<uint2 *>(phat_hi + (size_t)row * ldp);
-    uint2 *L4 = reinterpret_cast<uint2 *>(phat_lo + (size_t)row * ldp);
-    for (int q = lane; q < (nd >> 2); q += 32) {
-      const float4 v = P4[q], b = B4[q];
-      const float2 x01 = make_float2((v.x * invf - b.x) * 8192.0f, (v.y * invf - b.y) * 8192.0f);
-      const float2 x23 = make_float2((v.z * invf - b.z) * 8192.0f, (v.w * invf - b.w) * 8192.0f);
-      // paired conversions (round to nearest); the residual of each entry
-      // scaled by 2^11 is the lo plane
-      const __half2 h01 = __float22half2_rn(x01), h23 = __float22half2_rn(x23);
-      const float2 g01 = __half22float2(h01), g23 = __half22float2(h23);
-      const __half2 r01 = __float22half2_rn(
-          make_float2((x01.x - g01.x) * 2048.0f, (x01.y - g01.y) * 2048.0f));
-      const __half2 r23 = __float22half2_rn(
-          make_float2((x23.x - g23.x) * 2048.0f, (x23.y - g23.y) * 2048.0f));
-      H4[q] = make_uint2(*reinterpret_cast<const unsigned *>(&h01),
-                         *reinterpret_cast<const unsigned *>(&h23));
-      L4[q] = make_uint2(*reinterpret_cast<const unsigned *>(&r01),
-                         *reinterpret_cast<const unsigned *>(&r23));
-    }
+    // split operand only
+    write_split_row(reinterpret_cast<const float *>(p_s), nd, invf, pbar + (size_t)si * nd,
+                    phat_hi + (size_t)row * ldp, phat_lo + (size_t)row * ldp, lane);
     return;
   }
   for (int d = lane; d < nd; d += 32) {
@@ -683,95 +613,6 @@ k_b2_forward(B2Args a, const int *__restrict__ offset,
       phat_lo[(size_t)row * ldp + d] = __float2half_rn(rem);
     }
   }
-}
-
-// The mixed power-2 w = dE/dp and energy of one atom from its rows of V and of
-// the split operand (global or shared memory): four consecutive entries per
-// lane, 16-byte (8-byte for the fp16 planes) loads, |p| and E as float-float.
-// Every entry is stored by the lane that read it, so store may overwrite V4
-// in place.
-template <typename T, typename Store>
-__device__ __forceinline__ double w_mixed2(const AdjArgs &g, int si, int nd, float2 nrm32,
-                                           const float4 *V4, const uint2 *H4,
-                                           const uint2 *L4, Store store, int lane) {
-  double e;
-  const bool empty = nrm32.x * nrm32.x < g.empty_thresh_f;
-  const int nq = nd >> 2;
-  const float4 *G4 = reinterpret_cast<const float4 *>(g.gvec + (size_t)si * nd);
-  const float4 *B4 = reinterpret_cast<const float4 *>(g.pbar + (size_t)si * nd);
-  auto deltas = [&](uint2 h, uint2 l, float (&dl)[4]) {
-    const float2 h01 = __half22float2(*reinterpret_cast<const __half2 *>(&h.x));
-    const float2 h23 = __half22float2(*reinterpret_cast<const __half2 *>(&h.y));
-    const float2 l01 = __half22float2(*reinterpret_cast<const __half2 *>(&l.x));
-    const float2 l23 = __half22float2(*reinterpret_cast<const __half2 *>(&l.y));
-    dl[0] = (h01.x + l01.x * (1.0f / 2048.0f)) * (1.0f / 8192.0f);
-    dl[1] = (h01.y + l01.y * (1.0f / 2048.0f)) * (1.0f / 8192.0f);
-    dl[2] = (h23.x + l23.x * (1.0f / 2048.0f)) * (1.0f / 8192.0f);
-    dl[3] = (h23.y + l23.y * (1.0f / 2048.0f)) * (1.0f / 8192.0f);
-  };
-  // loads of kU iterations are issued before any of them is used (one atom's
-  // rows are a few KB: the loop is latency-bound without this)
-  constexpr int kU = 4;
-  Acc<float> acc;
-  for (int q0 = lane; q0 < nq; q0 += 32 * kU) {
-    uint2 h[kU], l[kU];
-    float4 v[kU], gg[kU];
-#pragma unroll
-    for (int u = 0; u < kU; u++) {
-      const int q = q0 + 32 * u;
-      if (q < nq) {
-        h[u] = H4[q];
-        l[u] = L4[q];
-        v[u] = V4[q];
-        gg[u] = G4[q];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kU; u++) {
-      if (q0 + 32 * u < nq) {
-        float dl[4];
-        deltas(h[u], l[u], dl);
-        acc.add((2.0f * gg[u].x + v[u].x) * dl[0]);
-        acc.add((2.0f * gg[u].y + v[u].y) * dl[1]);
-        acc.add((2.0f * gg[u].z + v[u].z) * dl[2]);
-        acc.add((2.0f * gg[u].w + v[u].w) * dl[3]);
-      }
-    }
-  }
-  float hi = acc.s, lo = acc.c;
-  ff_warp_sum(hi, lo);
-  const ff et = ff_add(ff_norm(hi, lo), ff{g.c0_hi[si], g.c0_lo[si]});
-  const float ef = empty ? 0.0f : et.hi + et.lo;
-  const float inv = empty ? 0.0f : 1.0f / nrm32.x;
-  e = empty ? 0.0 : double(et.hi) + double(et.lo);
-  for (int q0 = lane; q0 < nq; q0 += 32 * kU) {
-    uint2 h[kU], l[kU];
-    float4 v[kU], gg[kU], pb[kU];
-#pragma unroll
-    for (int u = 0; u < kU; u++) {
-      const int q = q0 + 32 * u;
-      if (q < nq) {
-        h[u] = H4[q];
-        l[u] = L4[q];
-        v[u] = V4[q];
-        gg[u] = G4[q];
-        pb[u] = B4[q];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kU; u++) {
-      const int q = q0 + 32 * u;
-      if (q < nq) {
-        float dl[4];
-        deltas(h[u], l[u], dl);
-        store(4 * q + 0, T(2.0f * ((gg[u].x + v[u].x) - ef * (pb[u].x + dl[0])) * inv));
-        store(4 * q + 1, T(2.0f * ((gg[u].y + v[u].y) - ef * (pb[u].y + dl[1])) * inv));
-        store(4 * q + 2, T(2.0f * ((gg[u].z + v[u].z) - ef * (pb[u].z + dl[2])) * inv));
-        store(4 * q + 3, T(2.0f * ((gg[u].w + v[u].w) - ef * (pb[u].w + dl[3])) * inv));
-      }
-    }
-  }
-  return e;
 }
 
 // w = dE/dp of one atom into w_s[nd] (all lanes), returning the atom energy:
@@ -804,11 +645,17 @@ __device__ __forceinline__ double adjoint_w(const B2Args &a, const AdjArgs &g, i
     }
   } else if (g.mode == kWFromV2 && (nd & 3) == 0) {
     // the mixed power-2 form, rows read from global memory
-    e = w_mixed2<T>(g, si, nd, nrm32,
-                    reinterpret_cast<const float4 *>(g.V32 + (size_t)row * g.ldv),
-                    reinterpret_cast<const uint2 *>(g.phat_hi + (size_t)row * g.ldp),
-                    reinterpret_cast<const uint2 *>(g.phat_lo + (size_t)row * g.ldp), store,
-                    lane);
+    e = w_mixed2(g, si, nd, nrm32,
+                 reinterpret_cast<const float4 *>(g.V32 + (size_t)row * g.ldv),
+                 reinterpret_cast<const uint2 *>(g.phat_hi + (size_t)row * g.ldp),
+                 reinterpret_cast<const uint2 *>(g.phat_lo + (size_t)row * g.ldp),
+                 [&](int q, float4 w) {
+                   store(4 * q + 0, T(w.x));
+                   store(4 * q + 1, T(w.y));
+                   store(4 * q + 2, T(w.z));
+                   store(4 * q + 3, T(w.w));
+                 },
+                 lane);
   } else if (g.mode == kWFromV2 || g.mode == kWFromV1) {
     // mixed form on the centred operand delta = phat - pbar (float):
     //   power 2: E = c0 + sum_d (2 g_d + V_d) delta_d,  V = beta delta,
@@ -1047,10 +894,10 @@ k_b2_wu_staged(B2Args a, AdjArgs g, const int *__restrict__ species,
     mbar_wait(bar, 0);
     return;
   }
-  const double e = w_mixed2<float>(
+  const double e = w_mixed2(
       g, si, nd, nrm32, reinterpret_cast<const float4 *>(v_s),
       reinterpret_cast<const uint2 *>(base + Ly.hi), reinterpret_cast<const uint2 *>(base + Ly.lo),
-      [&](int d, float v) { v_s[d] = v; }, lane);
+      [&](int q, float4 w) { reinterpret_cast<float4 *>(v_s)[q] = w; }, lane);
   if (lane == 0) atom_e[atom] = e;
   __syncwarp();
   b2_u_columns<float, SH>(a, v_s, reinterpret_cast<const float *>(base + Ly.c),
@@ -1067,28 +914,16 @@ k_b2_wu_staged(B2Args a, AdjArgs g, const int *__restrict__ species,
 // (the inverse of b3_to_complex's linear map), written to global memory.
 // ---------------------------------------------------------------------------
 template <typename T>
-__host__ __device__ inline size_t b3_adjoint_smem_per_warp(const B2Args &a, bool fixed = false) {
+__host__ __device__ inline size_t b3_adjoint_smem_per_warp(const B2Args &a) {
   const size_t nr = (size_t)a.n_species * a.N;
-  // fixed: the private rows of positions 2 and 3 (position 1 is in
-  // registers); otherwise all three
-  const size_t priv = (fixed ? 4 : 6) * (size_t)a.H * 32;
-  size_t b;
-  if (fixed) {
-    // the private rows share memory with the w rows of the first round
-    const size_t rows_a = (size_t)(a.n_tri < 32 ? a.n_tri : 32) * a.n_ls;
-    const size_t rows_b = (size_t)(a.n_tri > 32 ? a.n_tri - 32 : 0) * a.n_ls;
-    b = sizeof(T) * ((priv > rows_a ? priv : rows_a) + ((rows_b + 3) & ~(size_t)3) +
-                     2 * nr * (a.H + 1) + 2 * nr * a.H);
-  } else {
-    // w (padded to 4 entries), complex c, summed u, and per-lane private rows
-    // of the lane's triple (complex entries interleaved)
-    b = sizeof(T) * ((size_t)((a.n_d + 3) & ~3) + 2 * nr * (a.H + 1) + 2 * nr * a.H + priv);
-  }
+  // w (padded to 4 entries), complex c, summed u, and per-lane private rows of the
+  // lane's triple (complex entries interleaved)
+  const size_t b = sizeof(T) * ((size_t)((a.n_d + 3) & ~3) + 2 * nr * (a.H + 1) +
+                                2 * nr * a.H + 6 * (size_t)a.H * 32);
   return (b + 15) & ~(size_t)15;
 }
 
-// LM >= 0: the adjoint's terms unrolled for lmax = LM (a.lmax must equal it)
-template <typename T, int LM = -1>
+template <typename T>
 __global__ void __launch_bounds__(128)
 k_b3_wu(B2Args a, AdjArgs g, const int *__restrict__ species,
         const int *__restrict__ row_of_atom, const int *__restrict__ tri,
@@ -1101,23 +936,10 @@ k_b3_wu(B2Args a, AdjArgs g, const int *__restrict__ species,
   const int H = a.H, H1 = a.H + 1, nd = a.n_d;
   const int nr = a.n_species * a.N, sb = nr * H;
   unsigned char *base = smem_raw + a.smem_per_warp_adj * warp;
-  T *w_s = reinterpret_cast<T *>(base);  // [nd] (fixed: rows of triples < 32)
-  T *w_b = nullptr;                      // fixed: rows of triples >= 32
-  V2<T> *z, *u2, *up;                    // [nr][H+1] complex c, [sb] summed u,
-                                         // [3 H][32] private rows
-  const int rows_a = a.n_tri < 32 ? a.n_tri : 32;
-  if constexpr (LM >= 0) {
-    const size_t priv = 4 * (size_t)H * 32, wa = (size_t)rows_a * a.n_ls;
-    const size_t wbn = (size_t)(a.n_tri - rows_a) * a.n_ls;
-    w_b = w_s + (priv > wa ? priv : wa);
-    z = reinterpret_cast<V2<T> *>(w_b + ((wbn + 3) & ~(size_t)3));
-    u2 = z + (size_t)nr * H1;
-    up = reinterpret_cast<V2<T> *>(w_s);
-  } else {
-    z = reinterpret_cast<V2<T> *>(w_s + ((nd + 3) & ~3));
-    u2 = z + (size_t)nr * H1;
-    up = u2 + sb;
-  }
+  T *w_s = reinterpret_cast<T *>(base);                             // [nd]
+  V2<T> *z = reinterpret_cast<V2<T> *>(w_s + ((nd + 3) & ~3));      // [nr][H+1] complex c
+  V2<T> *u2 = z + (size_t)nr * H1;                                  // [sb] summed u
+  V2<T> *up = u2 + sb;                                              // [3 H][32] private rows
   if (atom >= a.noa) return;
   const int si = species[atom];
   const int row = row_of_atom[atom];
@@ -1128,26 +950,15 @@ k_b3_wu(B2Args a, AdjArgs g, const int *__restrict__ species,
   // real c staged through u2 (free until the accumulation below)
   T *cst = reinterpret_cast<T *>(u2);
   for (int k = lane; k < sb; k += 32) cst[k] = c_in[(size_t)atom * sb + k];
-  const int split = rows_a * a.n_ls;
-  const double e = adjoint_w<T>(
-      a, g, si, row, nrm, nrm32,
-      [&](int d, T v) {
-        if (LM >= 0 && d >= split)
-          w_b[d - split] = v;
-        else
-          w_s[d] = v;
-      },
-      lane);
+  const double e =
+      adjoint_w<T>(a, g, si, row, nrm, nrm32, [&](int d, T v) { w_s[d] = v; }, lane);
   if (lane == 0) atom_e[atom] = e;
   __syncwarp();
   b3_to_complex2<T>(cst, nr, H, z, lane);
   __syncwarp();
   for (int k = lane; k < sb; k += 32) u2[k] = V2<T>{T(0), T(0)};
   __syncwarp();
-  if constexpr (LM >= 0)
-    b3_contract_adjoint_fixed<T, LM>(a.n_tri, H, nr, tri, z, w_s, w_b, up, u2, lane);
-  else
-    b3_contract_adjoint<T>(a.lmax, a.n_ls, a.n_tri, H, nr, tri, z, w_s, up, u2, lane);
+  b3_contract_adjoint<T>(a.lmax, a.n_ls, a.n_tri, H, nr, tri, z, w_s, up, u2, lane);
   // dE/dc_real: for m > 0 with u+ = u[l, m], u- = u[l, -m], s = (-1)^m:
   //   dE/dR = (s Re u+ + Re u-) / sqrt 2,  dE/dS = (Im u- - s Im u+) / sqrt 2
   const T is2 = T(0.70710678118654752440);
@@ -1977,6 +1788,41 @@ int launch_b2_forward(B2Args a, const Neigh &nb, const int *species,
   });
 }
 
+// The adjoint's pair part: pair forces from u, then (gather) forces, energy and
+// virial sums.
+template <typename T>
+static int launch_pair_stage(const B2Args &a, const AdjArgs &g, const Neigh &nb,
+                             const int *species, double *atom_e, T *pair_f, double *forces,
+                             double *atom_vir, double *reduce_out, bool gather, T *u_buf,
+                             long long n_pairs, const int *nbr_i, cudaStream_t stream) {
+  if (n_pairs > 0) {
+    with_lmax<T>(a, [&](auto sh) {
+      k_pair_force<T, decltype(sh)><<<(unsigned)((n_pairs + 127) / 128), 128, 0, stream>>>(
+          a, g.strict, n_pairs, nbr_i, nb.rel, nb.rel32, nb.geom, nb.nbr_s, species, u_buf,
+          pair_f);
+      return 0;
+    });
+    if (cudaGetLastError() != cudaSuccess) return -1;
+  }
+  if (!gather) return 0;
+  int nblk;
+  if constexpr (sizeof(T) == 4) {
+    // a few resident blocks per SM, each walking many atoms
+    nblk = std::min(ceil_div(a.noa, kGatherWarps * (32 / kGatherLanes)), 152 * 8);
+    k_gather_warp<<<nblk, 32 * kGatherWarps, 0, stream>>>(
+        a.noa, nb.offset, nb.rev, nb.rel32, reinterpret_cast<const float4 *>(pair_f), atom_e,
+        forces, atom_vir);
+  } else {
+    nblk = std::min(ceil_div(a.noa, kGatherWarps * (32 / kGather64Lanes)), 152 * 4);
+    k_gather64<<<nblk, 32 * kGatherWarps, 0, stream>>>(
+        a.noa, nb.offset, nb.rev, nb.rel, reinterpret_cast<const dvec4 *>(pair_f), atom_e,
+        forces, atom_vir);
+  }
+  if (cudaGetLastError() != cudaSuccess) return -1;
+  k_reduce<<<10, 128, 0, stream>>>(nblk, atom_vir, reduce_out);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
 template <typename T>
 int launch_b2_adjoint(B2Args a, const AdjArgs &g, const Neigh &nb,
                       const int *species, const int *row_of_atom,
@@ -1985,17 +1831,21 @@ int launch_b2_adjoint(B2Args a, const AdjArgs &g, const Neigh &nb,
                       double *reduce_out, bool gather, T *u_buf, long long n_pairs,
                       const int *nbr_i, cudaStream_t stream) {
   if (a.noa == 0) return 0;
-  // FP32 at lmax 3 (the B3 workload shape): the unrolled adjoint
-  const bool b3_fixed = a.kind == kB3 && sizeof(T) == 4 && a.lmax == 3;
-  a.smem_per_warp_adj = a.kind == kB3 ? b3_adjoint_smem_per_warp<T>(a, b3_fixed)
-                                      : adjoint_smem_per_warp(a, sizeof(T));
+  if (sizeof(T) == 4 && g.b3_nd > 0) {
+    if (launch_b3_adjoint(a, g.b3_nd, g, species, row_of_atom,
+                          reinterpret_cast<const float *>(c_in), norm_in, atom_e,
+                          reinterpret_cast<float *>(u_buf), stream) != 0)
+      return -1;
+    return launch_pair_stage<T>(a, g, nb, species, atom_e, pair_f, forces, atom_vir, reduce_out,
+                                gather, u_buf, n_pairs, nbr_i, stream);
+  }
+  a.smem_per_warp_adj =
+      a.kind == kB3 ? b3_adjoint_smem_per_warp<T>(a) : adjoint_smem_per_warp(a, sizeof(T));
   const int wpb = warps_per_block(a.smem_per_warp_adj);
   if (wpb == 0) return -1;
   size_t smem = a.smem_per_warp_adj * wpb;
   if (a.kind == kB3) {
-    auto kern3 = k_b3_wu<T, -1>;
-    if constexpr (sizeof(T) == 4)
-      if (b3_fixed) kern3 = k_b3_wu<T, 3>;
+    auto kern3 = k_b3_wu<T>;
     if (cudaFuncSetAttribute(kern3, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem) != cudaSuccess)
       return -1;
@@ -2039,32 +1889,8 @@ int launch_b2_adjoint(B2Args a, const AdjArgs &g, const Neigh &nb,
     if (rc != 0) return -1;
   }
   if (cudaGetLastError() != cudaSuccess) return -1;
-  if (n_pairs > 0) {
-    with_lmax<T>(a, [&](auto sh) {
-      k_pair_force<T, decltype(sh)><<<(unsigned)((n_pairs + 127) / 128), 128, 0, stream>>>(
-          a, g.strict, n_pairs, nbr_i, nb.rel, nb.rel32, nb.geom, nb.nbr_s, species, u_buf,
-          pair_f);
-      return 0;
-    });
-    if (cudaGetLastError() != cudaSuccess) return -1;
-  }
-  if (!gather) return 0;
-  int nblk;
-  if constexpr (sizeof(T) == 4) {
-    // a few resident blocks per SM, each walking many atoms
-    nblk = std::min(ceil_div(a.noa, kGatherWarps * (32 / kGatherLanes)), 152 * 8);
-    k_gather_warp<<<nblk, 32 * kGatherWarps, 0, stream>>>(
-        a.noa, nb.offset, nb.rev, nb.rel32, reinterpret_cast<const float4 *>(pair_f), atom_e,
-        forces, atom_vir);
-  } else {
-    nblk = std::min(ceil_div(a.noa, kGatherWarps * (32 / kGather64Lanes)), 152 * 4);
-    k_gather64<<<nblk, 32 * kGatherWarps, 0, stream>>>(
-        a.noa, nb.offset, nb.rev, nb.rel, reinterpret_cast<const dvec4 *>(pair_f), atom_e,
-        forces, atom_vir);
-  }
-  if (cudaGetLastError() != cudaSuccess) return -1;
-  k_reduce<<<10, 128, 0, stream>>>(nblk, atom_vir, reduce_out);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+  return launch_pair_stage<T>(a, g, nb, species, atom_e, pair_f, forces, atom_vir, reduce_out,
+                              gather, u_buf, n_pairs, nbr_i, stream);
 }
 
 template int launch_b2_forward<float>(B2Args, const Neigh &, const int *, const int *,

@@ -23,6 +23,7 @@ struct B2Args {
   int n_species, N, lmax, H, n_d;
   int cutoff_kind;  // CutoffKind
   int window;       // neighbors staged per pass in the forward kernel
+  int c_only;       // forward: the single-bond coefficients only (b3_real.h follows)
   int strict;       // pair filter rsq < rc^2 (pair style) instead of r <= rc (B2)
   double r1;
   double cutoffs[kMaxSpecies * kMaxSpecies];
@@ -70,6 +71,7 @@ struct AdjArgs {
   // kernel form: V64 = G = C dhat and phat64 rows; per row E and sum_k C z
   const double *zc_given;
   const double *e_given;
+  int b3_nd;             // > 0: mixed B3 operand of the real form, its columns (b3_real.h)
   DeviceStatus *status;  // staged adjoint: where a wait that ran out is recorded
 };
 

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "b2_kernels.h"
+#include "b3_real.h"
 #include "capi_state.h"
 #include "common.cuh"
 #include "gemm_tc.h"
@@ -232,12 +233,14 @@ int kuf_tiles(fpp_model *m, const KufArgs &ka, int n_items, cudaStream_t st, int
 
 // Mixed forward: c32, norms (atom order; FP32 hi/lo pairs in pn64's 8-byte
 // slots), split fp16 phat rows.
-static int forward32(fpp_structure *s, const B2Args &a0, const int *pair_tab,
-                     const float *pbar, cudaStream_t st) {
+// nd: the operand's columns; real_b3: B3 through b3_real.h.
+static int forward32(fpp_structure *s, const B2Args &a0, const int *pair_tab, int nd,
+                     bool real_b3, const float *pbar, cudaStream_t st) {
   StructureState &S = s->st;
   B2Args a = a0;
   a.noa = S.noa;
-  const int ldp = round_up(a.n_d, 64);
+  a.c_only = real_b3 ? 1 : 0;
+  const int ldp = round_up(nd, 64);
   const int sb = a.n_species * a.N * a.H;
   FPP_TRY(ensure_layout(s, a.n_species, st));
   FPP_TRY(S.c32.reserve(sizeof(float) * std::max(1, S.noa) * sb));
@@ -250,6 +253,11 @@ static int forward32(fpp_structure *s, const B2Args &a0, const int *pair_tab,
                                S.phat_hi.as<__half>(), S.phat_lo.as<__half>(), ldp,
                                pbar, st) != 0)
     return fail(FPP_ERR_CUDA, "B2 forward (FP32) launch failed");
+  if (real_b3 &&
+      launch_b3_couple(a, nd, S.species.as<int>(), s->row_of_atom.as<int>(), S.c32.as<float>(),
+                       S.pn64.as<double>(), S.phat_hi.as<__half>(), S.phat_lo.as<__half>(), ldp,
+                       pbar, st) != 0)
+    return fail(FPP_ERR_CUDA, "B3 coupling (FP32) launch failed");
   return FPP_OK;
 }
 
@@ -448,6 +456,8 @@ int fpp_model_create(const fpp_b2 *b2, double sigma, double power, fpp_model **o
   m->n_species = b2->args.n_species;
   m->n_d = b2->args.n_d;
   m->ldb = round_up(m->n_d, 64);
+  if (m->args.kind == kB3 && b3_real_fits(m->args.lmax, m->args.n_species * m->args.N))
+    m->mixed_cols = b3_real_columns(m->args.lmax, m->args.n_tri);
   m->sp.resize(m->n_species);
   *out = m;
   return FPP_OK;
@@ -532,32 +542,43 @@ static int upload_beta(fpp_model *m, int s, const std::vector<double> &B) {
   const int nd = m->n_d, ldb = m->ldb;
   auto &sp = m->sp[s];
   std::vector<double> pad((size_t)nd * ldb, 0.0);
-  double amax = 0;
   bool finite = true;
   for (int i = 0; i < nd; i++)
     for (int j = 0; j < nd; j++) {
       const double v = B[(size_t)i * nd + j];
       pad[(size_t)i * ldb + j] = v;
-      amax = std::max(amax, std::fabs(v));
       finite = finite && std::isfinite(v);
+    }
+  // the mixed operand: all columns, or the listed ones (-1: padding)
+  const std::vector<int> &cols = m->mixed_cols;
+  const int mnd = cols.empty() ? nd : (int)cols.size(), mld = round_up(mnd, 64);
+  std::vector<double> mix((size_t)mnd * mld, 0.0);
+  double amax = 0;
+  for (int i = 0; i < mnd; i++)
+    for (int j = 0; j < mnd; j++) {
+      const int a = cols.empty() ? i : cols[i], b = cols.empty() ? j : cols[j];
+      if (a < 0 || b < 0) continue;
+      const double v = B[(size_t)a * nd + b];
+      mix[(size_t)i * mld + j] = v;
+      amax = std::max(amax, std::fabs(v));
     }
   sp.beta_finite = finite;
   sp.oz_beta.ready = false;
   double scale = 1.0;
   if (amax > 0) scale = std::ldexp(1.0, (int)std::floor(std::log2(16384.0 / amax)));
-  std::vector<__half> hi(pad.size()), lo(pad.size());
-  for (size_t k = 0; k < pad.size(); k++) {
-    const float x = (float)(pad[k] * scale);
+  std::vector<__half> hi(mix.size()), lo(mix.size());
+  for (size_t k = 0; k < mix.size(); k++) {
+    const float x = (float)(mix[k] * scale);
     const __half h = __float2half_rn(x);
-    const float rem = (float)((pad[k] * scale - (double)__half2float(h)) * 2048.0);
+    const float rem = (float)((mix[k] * scale - (double)__half2float(h)) * 2048.0);
     hi[k] = h;
     lo[k] = __float2half_rn(rem);
   }
   sp.beta_scale = scale;
   sp.B_host = B;
   FPP_TRY(sp.beta64.reserve(sizeof(double) * pad.size()));
-  FPP_TRY(sp.beta_hi.reserve(sizeof(__half) * pad.size()));
-  FPP_TRY(sp.beta_lo.reserve(sizeof(__half) * pad.size()));
+  FPP_TRY(sp.beta_hi.reserve(sizeof(__half) * hi.size()));
+  FPP_TRY(sp.beta_lo.reserve(sizeof(__half) * lo.size()));
   FPP_CUDA(cudaMemcpy(sp.beta64.ptr, pad.data(), sizeof(double) * pad.size(), cudaMemcpyHostToDevice));
   FPP_CUDA(cudaMemcpy(sp.beta_hi.ptr, hi.data(), sizeof(__half) * hi.size(), cudaMemcpyHostToDevice));
   FPP_CUDA(cudaMemcpy(sp.beta_lo.ptr, lo.data(), sizeof(__half) * lo.size(), cudaMemcpyHostToDevice));
@@ -668,22 +689,29 @@ namespace fpp {
 // Centre of the mixed operand for every species: pbar (rounded to FP32, the
 // values the kernels use), g = beta pbar and c0 = pbar^T beta pbar in FP64.
 static int set_center(fpp_model *m, const std::vector<std::vector<double>> &pbar) {
-  const int nd = m->n_d, ns = m->n_species;
-  std::vector<float> pb((size_t)ns * nd, 0.f), gv((size_t)ns * nd, 0.f);
+  const int nd = m->n_d, ns = m->n_species, mnd = mixed_nd(m);
+  // operand column j holds descriptor col(j); the others' centre is 0
+  const bool all = m->beta_power != 2 || m->mixed_cols.empty();
+  auto col = [&](int j) { return all ? j : m->mixed_cols[j]; };
+  std::vector<float> pb((size_t)ns * mnd, 0.f), gv((size_t)ns * mnd, 0.f);
   m->c0.assign(ns, 0.0);
   for (int s = 0; s < ns; s++) {
     std::vector<double> p(nd, 0.0);
-    for (int d = 0; d < nd; d++) {
-      pb[(size_t)s * nd + d] = (float)pbar[s][d];
-      p[d] = (double)pb[(size_t)s * nd + d];
+    for (int j = 0; j < mnd; j++) {
+      const int d = col(j);
+      if (d < 0) continue;
+      pb[(size_t)s * mnd + j] = (float)pbar[s][d];
+      p[d] = (double)pb[(size_t)s * mnd + j];
     }
     if (m->beta_power == 2 && !m->sp[s].B_host.empty()) {
       const double *B = m->sp[s].B_host.data();
       double c0 = 0;
-      for (int a = 0; a < nd; a++) {
+      for (int j = 0; j < mnd; j++) {
+        const int a = col(j);
+        if (a < 0) continue;
         double acc = 0;
         for (int b = 0; b < nd; b++) acc += B[(size_t)a * nd + b] * p[b];
-        gv[(size_t)s * nd + a] = (float)acc;
+        gv[(size_t)s * mnd + j] = (float)acc;
         c0 += p[a] * acc;
       }
       m->c0[s] = c0;
@@ -751,7 +779,9 @@ static int center_from_structure(fpp_model *m, fpp_structure *s, cudaStream_t st
   FPP_TRY(forward64(s, a, m->pair_tab.as<int>(), false, st));
   if ((int)m->centred.size() != m->n_species) m->centred.assign(m->n_species, 0);
   std::vector<std::vector<double>> pbar(m->n_species, std::vector<double>(nd, 0.0));
-  std::vector<float> old((size_t)m->n_species * nd, 0.f);
+  const int mnd = mixed_nd(m);
+  const bool all = m->beta_power != 2 || m->mixed_cols.empty();
+  std::vector<float> old((size_t)m->n_species * mnd, 0.f);
   if (m->pbar32.ptr)
     FPP_CUDA(cudaMemcpy(old.data(), m->pbar32.ptr, sizeof(float) * old.size(),
                         cudaMemcpyDeviceToHost));
@@ -760,7 +790,9 @@ static int center_from_structure(fpp_model *m, fpp_structure *s, cudaStream_t st
   FPP_TRY(partial.reserve(sizeof(double) * (size_t)kChunks * nd));
   std::vector<double> host((size_t)kChunks * nd);
   for (int sp = 0; sp < m->n_species; sp++) {
-    for (int d = 0; d < nd; d++) pbar[sp][d] = old[(size_t)sp * nd + d];
+    for (int j = 0; j < mnd; j++)
+      if (all || m->mixed_cols[j] >= 0)
+        pbar[sp][all ? j : m->mixed_cols[j]] = old[(size_t)sp * mnd + j];
     if (s->n_rows[sp] == 0 || (m->centred[sp] && !every_species)) continue;
     const int chunk = ceil_div(s->n_rows[sp], kChunks);
     const int nchunks = ceil_div(s->n_rows[sp], chunk);
@@ -878,31 +910,35 @@ int mapped_core(fpp_model *m, fpp_structure *s, int precision, cudaStream_t st,
     for (int sp = 0; sp < m->n_species; sp++)
       if (s->n_rows[sp] > 0 && !m->centred[sp]) recentre = true;
     if (recentre) FPP_TRY(center_from_structure(m, s, st));
-    FPP_TRY(forward32(s, a, m->pair_tab.as<int>(), m->pbar32.as<float>(), st));
+    const int mnd = mixed_nd(m), mldp = round_up(mnd, 64);
+    const bool real_b3 = m->beta_power == 2 && !m->mixed_cols.empty();
+    g.ldp = g.ldv = mldp;
+    g.b3_nd = real_b3 ? mnd : 0;
+    FPP_TRY(forward32(s, a, m->pair_tab.as<int>(), mnd, real_b3, m->pbar32.as<float>(), st));
     S.mark(3, st);
     if (m->beta_power == 2) {
-      FPP_TRY(reserve_zero(S.V, sizeof(float) * (size_t)s->total_rows * ldp, st));
+      FPP_TRY(reserve_zero(S.V, sizeof(float) * (size_t)s->total_rows * mldp, st));
       GroupedGemmArgs ga;
       std::memset(&ga, 0, sizeof(ga));
       ga.a_hi = S.phat_hi.as<__half>();
       ga.a_lo = S.phat_lo.as<__half>();
       ga.a_rows = s->total_rows;
-      ga.lda = ldp;
+      ga.lda = mldp;
       for (int sp = 0; sp < m->n_species; sp++) {
         if (s->n_rows[sp] == 0) continue;
         GemmGroup &q = ga.group[ga.n_groups++];
         q.b_hi = m->sp[sp].beta_hi.as<__half>();
         q.b_lo = m->sp[sp].beta_lo.as<__half>();
-        q.b_rows = nd;
-        q.ldb = m->ldb;
+        q.b_rows = mnd;
+        q.ldb = mldp;
         q.row0 = s->row_off[sp];
         q.M = s->n_rows[sp];
         q.out_scale = (float)(1.0 / (8192.0 * m->sp[sp].beta_scale));
       }
-      ga.N = nd;
-      ga.K = nd;
+      ga.N = mnd;
+      ga.K = mnd;
       ga.V = S.V.as<float>();
-      ga.ldv = ldp;
+      ga.ldv = mldp;
       ga.status = S.status.as<DeviceStatus>();
       const int rc = launch_split_gemm_grouped(ga, st);
       if (rc != 0)

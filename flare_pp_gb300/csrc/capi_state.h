@@ -42,6 +42,9 @@ struct fpp_model {
   double sigma = 1, power = 2;
   int n_species = 1, n_d = 0;
   int ldb = 0;                          // padded row length of beta operands
+  // columns of the mixed power-2 operand where they are not all n_d descriptors
+  // (B3 in real arithmetic, b3_real.h); empty: all of them
+  std::vector<int> mixed_cols;
   struct Species {
     int n_sparse = 0;
     int sparse_offset = 0;              // into the stacked alpha / R_inv
@@ -103,6 +106,10 @@ struct fpp_model {
 };
 
 namespace fpp {
+// columns of the mixed form's operand (power 2 may leave columns out)
+inline int mixed_nd(const fpp_model *m) {
+  return m->beta_power == 2 && !m->mixed_cols.empty() ? (int)m->mixed_cols.size() : m->n_d;
+}
 // constant-memory tables of the descriptor kernels (harmonic normalisations,
 // B3 couplings), uploaded once per device before the first kernel that reads
 // them
