@@ -70,7 +70,7 @@ __device__ __forceinline__ bool keep_pair32(const B2Args &a, int k, float rf,
 }
 int b3_n_ls_host(int lmax) { return b3_n_ls(lmax); }
 
-int upload_harmonic_tables(cudaStream_t stream) {
+HarmonicTables harmonic_tables() {
   HarmonicTables t;
   const double pi = 3.14159265358979323846;
   for (int l = 0; l <= kMaxL; l++)
@@ -98,6 +98,11 @@ int upload_harmonic_tables(cudaStream_t stream) {
     t.dfact[m] = d;
     t.dfact_f[m] = (float)d;
   }
+  return t;
+}
+
+int upload_harmonic_tables(cudaStream_t stream) {
+  const HarmonicTables t = harmonic_tables();
   cudaError_t e = cudaMemcpyToSymbolAsync(c_harm, &t, sizeof(t), 0,
                                           cudaMemcpyHostToDevice, stream);
   return e == cudaSuccess ? 0 : -1;

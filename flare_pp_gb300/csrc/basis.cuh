@@ -38,7 +38,10 @@ struct HarmonicTables {
   double dfact[kMaxL + 1];
   float dfact_f[kMaxL + 1];  // exact in FP32 (at most 15!! = 2027025)
 };
-static __constant__ HarmonicTables c_harm;  // uploaded by upload_harmonic_tables()
+// each translation unit's copy, uploaded from harmonic_tables() (upload_harmonic_tables,
+// upload_kuf_tables)
+static __constant__ HarmonicTables c_harm;
+HarmonicTables harmonic_tables();
 
 // N_lm * v (FP32: N_lm / D_lm * v), with the constant kept to ~48 bits in FP32
 __device__ __forceinline__ double norm_scale(int k, double v) { return c_harm.norm[k] * v; }
@@ -454,6 +457,31 @@ __device__ __forceinline__ void harmonics64(double ux, double uy, double uz, dou
     legendre64_column<L, m, false>(uz, [&](int l, double nq, double) {
       out[(l * l + l + m) * stride] = nq * A;
       if (m > 0) out[(l * l + l - m) * stride] = nq * B;
+    });
+  };
+  for_each_order<L, 0>(ux, uy, 1.0, 0.0, 0.0, 0.0, order);
+}
+
+// The same with the gradients dY_lm / dr_c at grad[(3 lm + c) * stride], ir = 1 / r.
+template <int L>
+__device__ __forceinline__ void harmonics64_grad(double ux, double uy, double uz, double ir,
+                                                 double *out, double *grad, int stride) {
+  auto order = [&](auto mc, double A, double B, double Ap, double Bp) {
+    constexpr int m = decltype(mc)::value;
+    // d(A, B)/dx = m (Ap, Bp),  d(A, B)/dy = m (-Bp, Ap)
+    const double ma = double(m) * Ap * ir, mb = double(m) * Bp * ir;
+    const double Ai = A * ir, Bi = B * ir;
+    auto emit = [&](int lm, double Yv, double gx, double gy, double gz) {
+      const double ug = m == 0 ? uz * gz : fma(ux, gx, fma(uy, gy, uz * gz));
+      out[lm * stride] = Yv;
+      grad[(3 * lm + 0) * stride] = fma(-ug, ux, gx);
+      grad[(3 * lm + 1) * stride] = fma(-ug, uy, gy);
+      grad[(3 * lm + 2) * stride] = fma(-ug, uz, gz);
+    };
+    legendre64_column<L, m, true>(uz, [&](int l, double nq, double nd) {
+      emit(l * l + l + m, m == 0 ? nq : nq * A, m == 0 ? 0.0 : nq * ma, m == 0 ? 0.0 : -nq * mb,
+           nd * Ai);
+      if (m > 0) emit(l * l + l - m, nq * B, nq * mb, nq * ma, nd * Bi);
     });
   };
   for_each_order<L, 0>(ux, uy, 1.0, 0.0, 0.0, 0.0, order);

@@ -9,6 +9,7 @@
 
 #include "b2_kernels.h"
 #include "capi_state.h"
+#include "kuf_gemm.h"
 #include "common.cuh"
 #include "internal.h"
 
@@ -51,7 +52,7 @@ int DevBuf::reserve(size_t n) {
 
 int ensure_tables(cudaStream_t stream) {
   // the harmonic normalisation and B3 coupling tables live in constant memory
-  // of this module; upload them once per device (under a lock: host threads
+  // of their translation units; upload them once per device (under a lock: host threads
   // may make their first call on a device at the same time)
   constexpr int kMaxDev = 64;
   static std::mutex mu;
@@ -61,7 +62,7 @@ int ensure_tables(cudaStream_t stream) {
   if (dev < 0 || dev >= kMaxDev) return fail(FPP_ERR_UNSUPPORTED, "device index beyond 63");
   std::lock_guard<std::mutex> lock(mu);
   if (uploaded[dev]) return FPP_OK;
-  if (upload_harmonic_tables(stream) != 0)
+  if (upload_harmonic_tables(stream) != 0 || upload_kuf_tables(stream) != 0)
     return fail(FPP_ERR_CUDA, "upload of harmonic tables failed");
   if (upload_descriptor_tables(stream) != 0)
     return fail(FPP_ERR_CUDA, "upload of B3 coupling tables failed");

@@ -18,6 +18,7 @@
 
 #include "b2_kernels.h"
 #include "b3_real.h"
+#include "capi_kuf.h"
 #include "capi_state.h"
 #include "common.cuh"
 #include "gemm_tc.h"
@@ -496,7 +497,7 @@ int fpp_model_set_sparse(fpp_model *m, int32_t species, int32_t n_sparse,
   FPP_TRY(sp.d_norms.reserve(sizeof(double) * n1));
   FPP_TRY(sp.d_calpha.reserve(sizeof(double) * n1));
   sp.oz_dhat.ready = sp.oz_dhatT.ready = sp.oz_Linv.ready = false;
-  m->oz_Linv.ready = m->oz_RinvT.ready = false;
+  m->oz_Linv.ready = m->oz_RinvT.ready = m->oz_kuf.ready = false;
   if (n_sparse) {
     FPP_CUDA(cudaMemcpy(sp.d_desc.ptr, descriptors, sizeof(double) * n_sparse * nd, cudaMemcpyHostToDevice));
     FPP_CUDA(cudaMemcpy(sp.d_dhat.ptr, dhat.data(), sizeof(double) * n_sparse * nd, cudaMemcpyHostToDevice));
@@ -1001,10 +1002,23 @@ static int envs_struc_device(fpp_model *m, fpp_structure *s, cudaStream_t st, De
   FPP_TRY(upload_pair_tab(m->pair_tab, m->pair_tab_host, st));
   B2Args a = m->args;
   a.noa = noa;
-  FPP_TRY(forward64(s, a, m->pair_tab.as<int>(), true, st));
-  double *phat = S.phat64.as<double>();
   FPP_TRY(K.reserve(sizeof(double) * (size_t)std::max(1, m->n_sparse_total) * n_out));
   FPP_CUDA(cudaMemsetAsync(K.ptr, 0, sizeof(double) * (size_t)m->n_sparse_total * n_out, st));
+  // B2: one GEMM over all descriptor pairs.  B3, and B2 shapes whose derivative rows do
+  // not fit in shared memory (several species at the largest N and lmax): stored
+  // derivatives, species by species
+  const bool gemm = kuf_gemm_fits(m);
+  FPP_TRY(forward64(s, a, m->pair_tab.as<int>(), !gemm, st));
+  double *phat = S.phat64.as<double>();
+  if (gemm && m->n_sparse_total > 0) {
+    KufItem it;
+    std::memset(&it, 0, sizeof(it));
+    it.s = s;
+    it.col_f0 = 1;
+    it.q.col_s = 1 + 3ll * noa;
+    FPP_TRY(kuf_gemm(m, m->kuf_work, {it}, K.as<double>(), n_out, st));
+    return ozaki_check_status(m->oz, st);
+  }
   // row-ordered atom norms
   DevBuf &rown = m->es_rown;
   FPP_TRY(rown.reserve(sizeof(double) * std::max(1, s->total_rows)));
@@ -1209,14 +1223,19 @@ int fpp_kuf_batched(fpp_model *m, fpp_structure *const *structures, int32_t n_st
   }
   FPP_TRY(upload_pair_tab(m->pair_tab, m->pair_tab_host, st));
   // FP64 descriptors of every structure, queued without synchronization
-  // (each structure keeps its own workspace), and the work list
+  // (each structure keeps its own workspace), and the work lists
   DevBuf dK, dfcol, dstruc, ditems;
   FPP_TRY(dK.reserve(sizeof(double) * (size_t)nst * n_labels));
   FPP_CUDA(cudaMemsetAsync(dK.ptr, 0, sizeof(double) * (size_t)nst * n_labels, st));
   FPP_TRY(dfcol.reserve(sizeof(int) * fcol.size()));
   FPP_CUDA(cudaMemcpyAsync(dfcol.ptr, fcol.data(), sizeof(int) * fcol.size(),
                            cudaMemcpyHostToDevice, st));
-  std::vector<int2> items;
+  int max_sparse = 0;
+  for (auto &x : m->sp) max_sparse = std::max(max_sparse, x.n_sparse);
+  const bool gemm = kuf_gemm_fits(m) && max_sparse >= kKufGemmSparse;
+  std::vector<KufItem> batch;  // by one GEMM
+  std::vector<int2> items;     // (structure, atom) by the adjoint
+  long long n_atoms = 0;
   for (int k = 0; k < n_structures; k++) {
     fpp_structure *s = structures[k];
     FPP_TRY(model_check(m, s));
@@ -1237,42 +1256,15 @@ int fpp_kuf_batched(fpp_model *m, fpp_structure *const *structures, int32_t n_st
     q.rel = S.nbr_rel.as<dvec4>();
     q.force_col = dfcol.as<int>() + fcol_off[k];
     q.vol_inv = 1.0 / S.ci.volume;
-    for (int i = 0; i < S.noa; i++) items.push_back(make_int2(k, i));
+    n_atoms += S.noa;
+    if (gemm && kuf_gemm_bytes(m, S.n_pairs) <= kKufGemmStructure) {
+      KufItem it{s, q, -1};
+      if (!(label_mask[k] & 2)) it.q.force_col = nullptr;
+      batch.push_back(it);
+    } else {
+      for (int i = 0; i < S.noa; i++) items.push_back(make_int2(k, i));
+    }
   }
-  if (items.empty()) {
-    FPP_CUDA(cudaMemcpy(kuf, dK.ptr, sizeof(double) * (size_t)nst * n_labels,
-                        cudaMemcpyDeviceToHost));
-    return FPP_OK;
-  }
-  FPP_TRY(dstruc.reserve(sizeof(KufStruc) * hs.size()));
-  FPP_CUDA(cudaMemcpyAsync(dstruc.ptr, hs.data(), sizeof(KufStruc) * hs.size(),
-                           cudaMemcpyHostToDevice, st));
-  FPP_TRY(ditems.reserve(sizeof(int2) * items.size()));
-  FPP_CUDA(cudaMemcpyAsync(ditems.ptr, items.data(), sizeof(int2) * items.size(),
-                           cudaMemcpyHostToDevice, st));
-  KufArgs ka;
-  std::memset(&ka, 0, sizeof(ka));
-  ka.a = m->args;
-  ka.strucs = dstruc.as<KufStruc>();
-  ka.items = ditems.as<int2>();
-  ka.n_items = (int)items.size();
-  for (int s = 0; s < m->n_species; s++) {
-    ka.sp[s].dhat = m->sp[s].d_dhat.as<double>();
-    ka.sp[s].norms = m->sp[s].d_norms.as<double>();
-    ka.sp[s].n_sparse = m->sp[s].n_sparse;
-    ka.sp[s].row0 = m->sp[s].sparse_offset;
-  }
-  ka.pair_tab = m->pair_tab.as<int>();
-  ka.sig2 = m->sigma * m->sigma;
-  ka.power = m->power;
-  ka.ldp = round_up(m->n_d, 64);
-  ka.kuf = dK.as<double>();
-  ka.n_labels = n_labels;
-  // tile shape: the cached choice for this device and descriptor, else the
-  // autotuner's (timed on a prefix of the work list, then Kuf is cleared)
-  int ks = 0, threads = 0;
-  FPP_TRY(kuf_tiles(m, ka, (int)items.size(), st, &ks, &threads));
-  FPP_CUDA(cudaMemsetAsync(dK.ptr, 0, sizeof(double) * (size_t)nst * n_labels, st));
   struct Events {  // released on every return path
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     ~Events() {
@@ -1282,13 +1274,48 @@ int fpp_kuf_batched(fpp_model *m, fpp_structure *const *structures, int32_t n_st
   } ev;
   FPP_CUDA(cudaEventCreate(&ev.e0));
   FPP_CUDA(cudaEventCreate(&ev.e1));
+  int ks = 32, threads = 32 * kKufAtoms;  // the gather's tile
+  KufArgs ka;
+  if (!items.empty()) {
+    FPP_TRY(dstruc.reserve(sizeof(KufStruc) * hs.size()));
+    FPP_CUDA(cudaMemcpyAsync(dstruc.ptr, hs.data(), sizeof(KufStruc) * hs.size(),
+                             cudaMemcpyHostToDevice, st));
+    FPP_TRY(ditems.reserve(sizeof(int2) * items.size()));
+    FPP_CUDA(cudaMemcpyAsync(ditems.ptr, items.data(), sizeof(int2) * items.size(),
+                             cudaMemcpyHostToDevice, st));
+    std::memset(&ka, 0, sizeof(ka));
+    ka.a = m->args;
+    ka.strucs = dstruc.as<KufStruc>();
+    ka.items = ditems.as<int2>();
+    ka.n_items = (int)items.size();
+    for (int s = 0; s < m->n_species; s++) {
+      ka.sp[s].dhat = m->sp[s].d_dhat.as<double>();
+      ka.sp[s].norms = m->sp[s].d_norms.as<double>();
+      ka.sp[s].n_sparse = m->sp[s].n_sparse;
+      ka.sp[s].row0 = m->sp[s].sparse_offset;
+    }
+    ka.pair_tab = m->pair_tab.as<int>();
+    ka.sig2 = m->sigma * m->sigma;
+    ka.power = m->power;
+    ka.ldp = round_up(m->n_d, 64);
+    ka.kuf = dK.as<double>();
+    ka.n_labels = n_labels;
+    // tile shape: the cached choice for this device and descriptor, else the
+    // autotuner's (timed on a prefix of the work list, then Kuf is cleared)
+    FPP_TRY(kuf_tiles(m, ka, (int)items.size(), st, &ks, &threads));
+    FPP_CUDA(cudaMemsetAsync(dK.ptr, 0, sizeof(double) * (size_t)nst * n_labels, st));
+  }
+  KufWork work;
   FPP_CUDA(cudaEventRecord(ev.e0, st));
-  if (launch_kuf_adjoint(ka, ks, threads, (int)items.size(), 0, st) != 0)
+  if (!batch.empty()) FPP_TRY(kuf_gemm(m, work, batch, dK.as<double>(), n_labels, st));
+  if (!items.empty() &&
+      launch_kuf_adjoint(ka, ks, threads, (int)items.size(), 0, st) != 0)
     return fail(FPP_ERR_CUDA, "Kuf (adjoint) launch failed");
   FPP_CUDA(cudaEventRecord(ev.e1, st));
   m->kuf_ks = ks;
   m->kuf_threads = threads;
-  m->kuf_items = (long long)items.size();
+  m->kuf_items = n_atoms;
+  if (!batch.empty()) FPP_TRY(ozaki_check_status(m->oz, st));
   FPP_CUDA(cudaMemcpyAsync(kuf, dK.ptr, sizeof(double) * (size_t)nst * n_labels,
                            cudaMemcpyDeviceToHost, st));
   FPP_CUDA(cudaStreamSynchronize(st));

@@ -27,6 +27,15 @@ struct fpp_lammps_ws {
   fpp::DevBuf d_x, d_type, d_ilist, d_nbrs, d_f, d_vir, d_e;
 };
 
+namespace fpp {
+// Workspace of the kernel columns by one GEMM (capi_kuf.h).
+struct KufWork {
+  DevBuf tables, pairs;        // structures and blocks; pairs by class
+  DevBuf z_planes, z;          // atoms: digit planes, z / a / sums of t
+  DevBuf planes, f, partial;   // derivative rows: digit planes, products; block sums
+};
+}  // namespace fpp
+
 struct fpp_b2 {
   fpp::B2Args args{};
   double rcut = 0;
@@ -94,12 +103,15 @@ struct fpp_model {
   fpp::OzakiWork oz;                    // kernel-form GEMM workspace
   fpp::OzakiOperand oz_Linv;            // digit planes of L_inv, of R_inv^T
   fpp::OzakiOperand oz_RinvT;
+  fpp::OzakiOperand oz_kuf;             // digit planes of dhat by pair class (capi_kuf.cu)
+  fpp::DevBuf kuf_tab;                  // its column tables
+  fpp::KufWork kuf_work;                // envs_struc workspace, kept between calls
   // kernel-form workspaces (grown on demand, kept between calls): per-row
   // scalars, z / C / K blocks, second products, column sums and partials
   fpp::DevBuf kf_rows, kf_z, kf_q, kf_cols;
   fpp_structure *batch = nullptr;       // packed structure of a batched prediction
   fpp::DevBuf batch_aoff, batch_poff, batch_sums, batch_src;
-  // envs_struc workspace (grown on demand, kept between calls)
+  // envs_struc workspace of the stored-derivative form (grown on demand, kept between calls)
   fpp::DevBuf es_rown, es_ndm, es_flags, es_pos, es_scan, es_plist, es_qatom, es_dmap,
       es_dp, es_sfd, es_fd;
   void *cublas = nullptr;               // cublasHandle_t

@@ -26,8 +26,9 @@ OzakiShape ozaki_shape(int rows, int K);
 // exponent e of each row (max |row| < 2^e; kOzakiNanRow if the row holds a
 // non-finite entry) of X (rows x K, row stride ldx, device memory).
 constexpr int kOzakiNanRow = -(1 << 30);
+// row_ptr (device): where each row starts, instead of X and ldx.
 int launch_ozaki_split(int rows, int K, const double *X, long long ldx, __half *planes,
-                       int *exps, cudaStream_t stream);
+                       int *exps, cudaStream_t stream, const double *const *row_ptr = nullptr);
 
 // An operand split by launch_ozaki_split.
 struct OzakiMat {
@@ -37,7 +38,7 @@ struct OzakiMat {
 };
 
 // One product of a grouped launch: C (M x N, row stride ldc) = A B^T with rows
-// a_row0 .. a_row0 + M of operand a and rows 0 .. N of operand b.  C need not
+// a_row0 .. a_row0 + M of operand a and rows b_row0 .. b_row0 + N of operand b.  C need not
 // be initialised.  b_lower: B is lower triangular (B[n][k] = 0 for k > n; an
 // L^-1, or an R^-1 transposed), and the K blocks above each column tile's last
 // row are skipped.  Rows or columns with a non-finite operand come out NaN.
@@ -47,6 +48,7 @@ struct OzakiProblem {
   double *C;
   long long ldc;
   bool b_lower;
+  int b_row0 = 0;
 };
 // Up to kOzakiMaxGroups products in one persistent launch (their tiles share
 // the SMs).  n_levels: 8, or 9 where the dropped digit pairs must stay below the

@@ -106,6 +106,16 @@ __host__ __device__ constexpr uint32_t idesc_f16() {
          ((uint32_t)(128 >> 4) << 24);
 }
 
+// The same with the columns N known at run time (a multiple of 16, at most 256).
+__device__ __forceinline__ void mma_f16_n(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t n,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(a), "l"(b), "r"(idesc_f16<0>() | ((n >> 3) << 17)), "r"(accumulate));
+}
+
 template <int NN>
 __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t a, uint64_t b,
                                         uint32_t accumulate) {

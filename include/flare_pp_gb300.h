@@ -275,14 +275,16 @@ int fpp_predict_energy_uncertainty(fpp_model *m, fpp_structure *s, double *energ
  * of each structure's labels, [E] [F of the listed atoms] [S], stacked in
  * structure order into kuf (host, n_sparse_total x n_labels, row-major),
  * FP64 on the GPU.  The columns are the envs_struc values of
- * normalized_dot_product.cpp:115-210, formed by the adjoint route (no
- * stored descriptor derivatives): one persistent launch over the (structure,
- * atom) work list of the whole batch, no synchronization per structure; the
- * kernel's tile shape (sparse environments per pass, threads per block) is
+ * normalized_dot_product.cpp:115-210: all pairs' derivative rows times the sparse
+ * environments as one FP64-accurate GEMM per chunk of structures, then a gather per
+ * atom (one synchronization for the batch; sums in a fixed order).  With fewer than ten
+ * sparse environments of every species, and for a structure whose rows would take more
+ * than 16 GB, the adjoint route instead: one persistent launch over the (structure,
+ * atom) work list, its tile shape (sparse environments per pass, threads per block)
  * autotuned once per device and descriptor shape and cached in the file
- * $FPP_TUNE_CACHE (else $HOME/.cache/flare_pp_gb300/tiles.txt).  Additions
- * into other atoms' columns are FP64 atomics, so results vary between runs
- * at the level of FP64 rounding.  B2 models only.
+ * $FPP_TUNE_CACHE (else $HOME/.cache/flare_pp_gb300/tiles.txt), its additions into
+ * other atoms' columns FP64 atomics (results vary between runs at the level of FP64
+ * rounding).  B3 models: stored derivatives, structure by structure.
  * label_mask[k]: bit 0 energy, bit 1 forces, bit 2 stress of structure k;
  * atom_offsets (n_structures + 1) and atoms list the force atoms of each
  * structure (the reference's atom_indices; NULL: every atom).  n_labels must
@@ -293,7 +295,7 @@ int fpp_kuf_batched(fpp_model *m, fpp_structure *const *structures,
                     double *kuf, int64_t n_labels, void *stream);
 /* The tile shape the last fpp_kuf_batched call on m used (sparse
  * environments per pass, threads per block), and (each may be NULL) the
- * CUDA-event time of its Kuf kernel in ms and its (structure, atom) work
+ * CUDA-event time of its Kuf kernels in ms and its (structure, atom) work
  * items.  No counterpart in the reference (an instrumentation call). */
 int fpp_model_kuf_tiles(const fpp_model *m, int32_t *ks, int32_t *threads,
                         float *kernel_ms, int64_t *n_items);
