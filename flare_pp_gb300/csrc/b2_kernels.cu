@@ -214,6 +214,120 @@ __host__ __device__ inline FwdLayout<T> fwd_layout(const B2Args &a) {
   return L;
 }
 
+// The FP64 single-bond sums of one atom (stages 1 and 2 of the forward).  FP64 issues
+// two per clock and SM, so what counts is how many FP64 instructions the warp issues:
+//  - pairs inside their cutoff are queued first, so that a window always holds 32 of them
+//    (a LAMMPS list with its skin filled three windows where two do);
+//  - a species' N H sums are dealt to the lanes one after the other (N ceil(H / 32)
+//    rounds per neighbor with a lane per (l, m) column: half the lanes idle at lmax 3);
+//  - the first chunk of 16 of a species is its sum, later ones are Kahan-folded.
+// The sums themselves run as before: neighbors in order, chunks of 16.
+// 4,394 atoms with a skin, N = 8, lmax = 3: 446 us before, 233 so; 8,192 atoms, N = 12,
+// lmax = 4: 899 and 623.
+template <typename SH>
+__device__ __forceinline__ void forward64_sums(const B2Args &a, int si, int beg, int end,
+                                               const dvec4 *__restrict__ rel,
+                                               const int *__restrict__ nbr_s, double *g_s,
+                                               double *y_s, double *c_s, double *cc_s,
+                                               int *list, int lane) {
+  constexpr int kSums = SH::kL1 == 5 ? 10 : 8;  // sums per lane and pass
+  const int N = SH::N(a), LMAX = SH::lmax(a), H = (LMAX + 1) * (LMAX + 1), NS = SH::NS(a);
+  const int W = a.window, GP = (N + 3) & ~3, WS = W + 1, HP = (H + 3) & ~3;
+  int *cnt_s = list + NS * W, *queue = cnt_s + NS;  // [NS], [2 W]
+  unsigned long long seen = 0ull;                   // species with a sum
+  int qn = 0, next = beg;
+  for (;;) {
+    while (qn < W && next < end) {
+      const int p = next + lane;
+      bool keep = false;
+      if (p < end) {
+        const dvec4 rd = rel[p];
+        const double rcut = a.cutoffs[si * NS + nbr_s[p]];
+        keep = a.strict ? (rsq_exact(rd) < dmul(rcut, rcut)) : (rd.x <= rcut);
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, keep);
+      if (keep) queue[qn + __popc(m & ((1u << lane) - 1u))] = p;
+      qn += __popc(m);
+      next += 32;
+    }
+    __syncwarp();
+    if (qn == 0) break;
+    const int cnt = min(qn, W);
+    // bases of the window's neighbors, a lane each, and their lists by species
+    int sj = -1;
+    if (lane < cnt) {
+      const int p = queue[lane];
+      sj = nbr_s[p];
+      const int kc = si * NS + sj;
+      const dvec4 rd = rel[p];
+      radial_basis<double>(rd.x, a.r1, a.cutoffs[kc], N, a.cutoff_kind,
+                           g_s + (size_t)lane * GP, nullptr, 1, a.cinv64_hi[kc],
+                           a.cinv64_lo[kc]);
+      if constexpr (SH::kL1 > 0) {
+        const double ir = 1.0 / rd.x;
+        harmonics64<SH::kL1 - 1>(rd.y * ir, rd.z * ir, rd.w * ir, y_s + lane, WS);
+      } else {
+        real_harmonics<double>(rd.y, rd.z, rd.w, LMAX, y_s + lane, nullptr, WS);
+      }
+    }
+    for (int sp = 0; sp < NS; sp++) {
+      const unsigned m = __ballot_sync(0xffffffffu, sj == sp);
+      if (sj == sp) list[sp * W + __popc(m & ((1u << lane) - 1u))] = lane;
+      if (lane == 0) cnt_s[sp] = __popc(m);
+    }
+    // the queue's rest to its front
+    const int rest = qn - cnt, moved = lane < rest ? queue[W + lane] : 0;
+    __syncwarp();
+    if (lane < rest) queue[lane] = moved;
+    qn = rest;
+    for (int sp = 0; sp < NS; sp++) {
+      const int ns_ = cnt_s[sp];
+      if (ns_ == 0) continue;
+      const int *ls = list + sp * W;
+      const bool first = !((seen >> sp) & 1ull);
+      seen |= 1ull << sp;
+      for (int o0 = 0; o0 < N * H; o0 += 32 * kSums) {
+        int yo[kSums], go[kSums], co[kSums];  // this lane's sums: (n, lm) of o0 + 32 j + lane
+#pragma unroll
+        for (int j = 0; j < kSums; j++) {
+          const int o = min(o0 + 32 * j + lane, N * H - 1), n = o / H, lm = o - n * H;
+          yo[j] = lm * WS;
+          go[j] = n;
+          co[j] = (sp * N + n) * HP + lm;
+        }
+        for (int k0 = 0; k0 < ns_; k0 += 16) {
+          double chunk[kSums];
+#pragma unroll
+          for (int j = 0; j < kSums; j++) chunk[j] = 0.0;
+          const int k1 = min(ns_, k0 + 16);
+          for (int k = k0; k < k1; k++) {
+            const int b = ls[k];
+            const double *yb = y_s + b, *gb = g_s + b * GP;
+#pragma unroll
+            for (int j = 0; j < kSums; j++)
+              if (o0 + 32 * j < N * H) chunk[j] = fma(gb[go[j]], yb[yo[j]], chunk[j]);
+          }
+#pragma unroll
+          for (int j = 0; j < kSums; j++)
+            if (o0 + 32 * j + lane < N * H) {
+              if (first && k0 == 0) {
+                c_s[co[j]] = chunk[j];
+                cc_s[co[j]] = 0.0;
+              } else {  // Kahan fold of the chunk
+                const double sum = c_s[co[j]];
+                const double yk = chunk[j] - cc_s[co[j]];
+                const double t = sum + yk;
+                cc_s[co[j]] = (t - sum) - yk;
+                c_s[co[j]] = t;
+              }
+            }
+        }
+      }
+    }
+    __syncwarp();
+  }
+}
+
 // FP32: registers capped for six blocks of four warps per SM (the shared
 // memory allows six); FP64: no cap (it would spill)
 template <typename T, typename SH>
@@ -243,7 +357,7 @@ k_b2_forward(B2Args a, const int *__restrict__ offset,
   T *c_s = reinterpret_cast<T *>(base + Lay.stage);   // [NS N][HP] running sums
   T *cc_s = c_s + sbp;  // FP64 only: [NS N][HP] compensation
   int *list = reinterpret_cast<int *>(base + Lay.stage + Lay.csum);  // [NS][W]
-  int *cnt_s = list + NS * W;                         // [NS]
+  int *cnt_s = list + NS * W;                         // [NS] (FP64: and [2 W] queued pairs)
   if (atom >= a.noa) return;
 
   for (int k = lane; k < sbp; k += 32) {
@@ -253,153 +367,122 @@ k_b2_forward(B2Args a, const int *__restrict__ offset,
   const int si = species[atom];
   const int beg = offset[atom], end = offset[atom + 1];
   __syncwarp();
-  for (int w0 = beg; w0 < end; w0 += W) {
-    const int cnt = min(W, end - w0);
-    // ---- 1. stage bases and species lists ----
-    if (lane < NS) cnt_s[lane] = 0;
-    __syncwarp();
-    for (int b0 = 0; b0 < cnt; b0 += 32) {
-      const int b = b0 + lane;
-      int sj = -1;
-      if (b < cnt) {
-        const int p = w0 + b;
-        const int sp = nbr_s[p];
-        const int kc = si * NS + sp;
-        T r, x, y, z, r1t, rct;
-        bool keep;
-        if (sizeof(T) == 8) {
-          const dvec4 rd = rel[p];
-          const double rcut = a.cutoffs[kc];
-          keep = a.strict ? (rsq_exact(rd) < dmul(rcut, rcut)) : (rd.x <= rcut);
-          r = T(rd.x);
-          x = T(rd.y);
-          y = T(rd.z);
-          z = T(rd.w);
-          r1t = T(a.r1);
-          rct = T(rcut);
-        } else {
+  if constexpr (sizeof(T) == 8) {
+    forward64_sums<SH>(a, si, beg, end, rel, nbr_s, g_s, y_s, c_s, cc_s, list, lane);
+  } else {
+    for (int w0 = beg; w0 < end; w0 += W) {
+      const int cnt = min(W, end - w0);
+      // ---- 1. stage bases and species lists ----
+      if (lane < NS) cnt_s[lane] = 0;
+      __syncwarp();
+      for (int b0 = 0; b0 < cnt; b0 += 32) {
+        const int b = b0 + lane;
+        int sj = -1;
+        if (b < cnt) {
+          const int p = w0 + b;
+          const int sp = nbr_s[p];
+          const int kc = si * NS + sp;
           const float4 rf = rel32[p];
-          x = T(rf.x);
-          y = T(rf.y);
-          z = T(rf.z);
-          r = T(rf.w);
-          if (a.strict)
-            keep = strict_keep(rel, p, a.cutoffs[kc]);
-          else
-            keep = keep_pair32(a, kc, rf.w, rel, geom, atom, p);
-          r1t = T(a.r1f);
-          rct = T(a.cutoffs32[kc]);
-        }
-        if (keep) {
-          sj = sp;
-          radial_basis<T>(r, r1t, rct, N, a.cutoff_kind, g_s + (size_t)b * GP, nullptr, 1,
-                          sizeof(T) == 4 ? T(a.cinv_hi[kc]) : T(a.cinv64_hi[kc]),
-                          sizeof(T) == 4 ? T(a.cinv_lo[kc]) : T(a.cinv64_lo[kc]));
-          if constexpr (sizeof(T) == 8 && SH::kL1 > 0) {
-            const T ir = T(1) / r;
-            harmonics64<SH::kL1 - 1>(x * ir, y * ir, z * ir, y_s + b, WS);
-          } else {
-            real_harmonics<T>(x, y, z, LMAX, y_s + b, nullptr, WS);
+          const bool keep = a.strict ? strict_keep(rel, p, a.cutoffs[kc])
+                                     : keep_pair32(a, kc, rf.w, rel, geom, atom, p);
+          if (keep) {
+            sj = sp;
+            radial_basis<T>(rf.w, a.r1f, a.cutoffs32[kc], N, a.cutoff_kind, g_s + (size_t)b * GP,
+                            nullptr, 1, a.cinv_hi[kc], a.cinv_lo[kc]);
+            real_harmonics<T>(rf.x, rf.y, rf.z, LMAX, y_s + b, nullptr, WS);
           }
         }
+        for (int sp = 0; sp < NS; sp++) {
+          const unsigned m = __ballot_sync(0xffffffffu, sj == sp);
+          if (sj == sp) list[sp * W + cnt_s[sp] + __popc(m & ((1u << lane) - 1u))] = b;
+          __syncwarp();
+          if (lane == 0) cnt_s[sp] += __popc(m);
+          __syncwarp();
+        }
       }
+      __syncwarp();
+      // ---- 2. accumulate: lane owns column lm ----
       for (int sp = 0; sp < NS; sp++) {
-        const unsigned m = __ballot_sync(0xffffffffu, sj == sp);
-        if (sj == sp) list[sp * W + cnt_s[sp] + __popc(m & ((1u << lane) - 1u))] = b;
-        __syncwarp();
-        if (lane == 0) cnt_s[sp] += __popc(m);
-        __syncwarp();
-      }
-    }
-    __syncwarp();
-    // ---- 2. accumulate: lane owns column lm ----
-    for (int sp = 0; sp < NS; sp++) {
-      const int ns_ = cnt_s[sp];
-      if (ns_ == 0) continue;
-      const int *ls = list + sp * W;
-      for (int lm0 = 0; lm0 < H; lm0 += 32) {
-        const int lm = lm0 + lane;
-        const bool act = lm < H;
-        const int lmc = act ? lm : 0;
-        T sum[kMaxN], comp[kMaxN];
-#pragma unroll
-        for (int n = 0; n < kMaxN; n++)
-          if (n < N) {
-            sum[n] = c_s[(sp * N + n) * HP + lmc];
-            // FP32: compensated within the window and folded at its end
-            comp[n] = sizeof(T) == 8 ? cc_s[(sp * N + n) * HP + lmc] : T(0);
-          }
-        for (int k0 = 0; k0 < ns_; k0 += 16) {
-          T chunk[kMaxN];
-#pragma unroll
-          for (int n = 0; n < kMaxN; n++) chunk[n] = T(0);
-          const int k1 = min(ns_, k0 + 16);
-          if constexpr (SH::kN > 0 && sizeof(T) == 4) {
-            // radial row of the neighbor in 16-byte loads (GP = N rounded up
-            // to 4), channels accumulated in pairs with paired multiply-adds
-            // (pad channels past N are computed and discarded)
-            constexpr int G4 = (SH::kN + 3) / 4;
-            float2 c2[2 * G4];
-#pragma unroll
-            for (int j = 0; j < 2 * G4; j++) c2[j] = make_float2(0.f, 0.f);
-            auto accum = [&](int b) {
-              const float yv = y_s[lmc * WS + b];
-              const float2 y2 = make_float2(yv, yv);
-              const float4 *gb4 = reinterpret_cast<const float4 *>(g_s + (size_t)b * (4 * G4));
-#pragma unroll
-              for (int j = 0; j < G4; j++) {
-                const float4 gv = gb4[j];
-                c2[2 * j] = ffma2(make_float2(gv.x, gv.y), y2, c2[2 * j]);
-                c2[2 * j + 1] = ffma2(make_float2(gv.z, gv.w), y2, c2[2 * j + 1]);
-              }
-            };
-            // two neighbors per iteration (same summation order)
-            int k = k0;
-            for (; k + 1 < k1; k += 2) {
-              const int b0 = ls[k], b1 = ls[k + 1];
-              accum(b0);
-              accum(b1);
-            }
-            if (k < k1) accum(ls[k]);
-#pragma unroll
-            for (int j = 0; j < 2 * G4; j++) {
-              if (2 * j < SH::kN) chunk[2 * j] = c2[j].x;
-              if (2 * j + 1 < SH::kN) chunk[2 * j + 1] = c2[j].y;
-            }
-          } else {
-            for (int k = k0; k < k1; k++) {
-              const int b = ls[k];
-              const T yv = y_s[lmc * WS + b];
-              const T *gb = g_s + (size_t)b * GP;
-#pragma unroll
-              for (int n = 0; n < kMaxN; n++)
-                if (n < N) chunk[n] += gb[n] * yv;
-            }
-          }
-#pragma unroll
-          for (int n = 0; n < kMaxN; n++)
-            if (n < N) {  // Kahan fold of the chunk
-              const T yk = chunk[n] - comp[n];
-              const T t = sum[n] + yk;
-              comp[n] = (t - sum[n]) - yk;
-              sum[n] = t;
-            }
-        }
-        if (act) {
+        const int ns_ = cnt_s[sp];
+        if (ns_ == 0) continue;
+        const int *ls = list + sp * W;
+        for (int lm0 = 0; lm0 < H; lm0 += 32) {
+          const int lm = lm0 + lane;
+          const bool act = lm < H;
+          const int lmc = act ? lm : 0;
+          T sum[kMaxN], comp[kMaxN];
 #pragma unroll
           for (int n = 0; n < kMaxN; n++)
             if (n < N) {
-              if (sizeof(T) == 8) {
-                c_s[(sp * N + n) * HP + lm] = sum[n];
-                cc_s[(sp * N + n) * HP + lm] = comp[n];
-              } else {
-                c_s[(sp * N + n) * HP + lm] = sum[n] - comp[n];
+              // compensated within the window and folded at its end
+              sum[n] = c_s[(sp * N + n) * HP + lmc];
+              comp[n] = T(0);
+            }
+          for (int k0 = 0; k0 < ns_; k0 += 16) {
+            T chunk[kMaxN];
+#pragma unroll
+            for (int n = 0; n < kMaxN; n++) chunk[n] = T(0);
+            const int k1 = min(ns_, k0 + 16);
+            if constexpr (SH::kN > 0) {
+              // radial row of the neighbor in 16-byte loads (GP = N rounded up
+              // to 4), channels accumulated in pairs with paired multiply-adds
+              // (pad channels past N are computed and discarded)
+              constexpr int G4 = (SH::kN + 3) / 4;
+              float2 c2[2 * G4];
+#pragma unroll
+              for (int j = 0; j < 2 * G4; j++) c2[j] = make_float2(0.f, 0.f);
+              auto accum = [&](int b) {
+                const float yv = y_s[lmc * WS + b];
+                const float2 y2 = make_float2(yv, yv);
+                const float4 *gb4 = reinterpret_cast<const float4 *>(g_s + (size_t)b * (4 * G4));
+#pragma unroll
+                for (int j = 0; j < G4; j++) {
+                  const float4 gv = gb4[j];
+                  c2[2 * j] = ffma2(make_float2(gv.x, gv.y), y2, c2[2 * j]);
+                  c2[2 * j + 1] = ffma2(make_float2(gv.z, gv.w), y2, c2[2 * j + 1]);
+                }
+              };
+              // two neighbors per iteration (same summation order)
+              int k = k0;
+              for (; k + 1 < k1; k += 2) {
+                const int b0 = ls[k], b1 = ls[k + 1];
+                accum(b0);
+                accum(b1);
+              }
+              if (k < k1) accum(ls[k]);
+#pragma unroll
+              for (int j = 0; j < 2 * G4; j++) {
+                if (2 * j < SH::kN) chunk[2 * j] = c2[j].x;
+                if (2 * j + 1 < SH::kN) chunk[2 * j + 1] = c2[j].y;
+              }
+            } else {
+              for (int k = k0; k < k1; k++) {
+                const int b = ls[k];
+                const T yv = y_s[lmc * WS + b];
+                const T *gb = g_s + (size_t)b * GP;
+#pragma unroll
+                for (int n = 0; n < kMaxN; n++)
+                  if (n < N) chunk[n] += gb[n] * yv;
               }
             }
+#pragma unroll
+            for (int n = 0; n < kMaxN; n++)
+              if (n < N) {  // Kahan fold of the chunk
+                const T yk = chunk[n] - comp[n];
+                const T t = sum[n] + yk;
+                comp[n] = (t - sum[n]) - yk;
+                sum[n] = t;
+              }
+          }
+          if (act) {
+#pragma unroll
+            for (int n = 0; n < kMaxN; n++)
+              if (n < N) c_s[(sp * N + n) * HP + lm] = sum[n] - comp[n];
+          }
         }
       }
+      __syncwarp();
     }
-    __syncwarp();
   }
   // (FP64: fold the compensation) publish c (unpadded rows in global memory)
   for (int k = lane; k < sb; k += 32) {
