@@ -1302,7 +1302,24 @@ k_pair_force(B2Args a, int strict, long long n_pairs, const int *__restrict__ nb
 
 // Stored derivatives of b2.cpp:181-242 for a list of structure pairs (FP64):
 // rows 3*idx + comp of dp = d p_i / d r_ij and force_dots = dp . p_i.
-// One warp per pair.
+// A block takes 16 pairs of the list: one warp evaluates their bases, a lane per pair
+// (an FP64 instruction costs the same for one lane as for 32; the bases by lane 0 of each
+// pair's own warp were four fifths of this kernel), then each warp forms the rows of its
+// pairs from alpha[l, n] = sum_m c[n, lm] Y[lm] and beta_c[l, n] = sum_m c[n, lm]
+// dY[lm]/dr_c:  dp_c[(n1, n2), l] = g'_{n2} rhat_c alpha[l, n1] + g_{n2} beta_c[l, n1]
+// and n1 <-> n2, each where that channel is of the neighbor's species.  108 atoms, N = 8,
+// lmax = 3, 5,800 pairs: 267 us by products of c and dc, 48 so.
+constexpr int kDpPairs = 16, kDpStride = kDpPairs + 1;
+
+__host__ __device__ inline int dp_sums_stride(const B2Args &a) {
+  return (a.n_species * a.N) | 1;  // odd: the degrees of a column group in different banks
+}
+__host__ __device__ inline size_t dp_smem(const B2Args &a, int warps) {
+  return sizeof(double) * ((size_t)(2 * a.N + 4 * a.H) * kDpStride + 3 * kDpPairs +
+                           (size_t)warps * 6 * dp_sums_stride(a) * (a.lmax + 1));
+}
+
+template <typename SH>
 __global__ void __launch_bounds__(128)
 k_b2_dp(B2Args a, int npl, const int *__restrict__ plist,
         const int *__restrict__ nbr_i, const int *__restrict__ nbr_s,
@@ -1313,54 +1330,76 @@ k_b2_dp(B2Args a, int npl, const int *__restrict__ plist,
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nwarps = blockDim.x >> 5;
-  const int idx = blockIdx.x * nwarps + warp;
-  const int N = a.N, H = a.H, NS = a.n_species, nd = a.n_d;
-  const int sb = NS * N * H;
-  double *base = reinterpret_cast<double *>(smem_raw) + (size_t)warp * (sb + 3 * N * H + 2 * N + 4 * H);
-  double *c_s = base;                 // [sb]
-  double *dc = c_s + sb;              // [3][N][H]
-  double *gb = dc + 3 * N * H;        // [N] g, [N] dg
-  double *yb = gb + 2 * N;            // [H] Y, [3H] dY
-  if (idx >= npl) return;
-  const int p = plist[idx];
-  const int i = nbr_i[p], sj = nbr_s[p];
-  const int si = species[i];
-  const dvec4 rd = rel[p];
-  const double rcut = a.cutoffs[si * NS + sj];
-  for (int k = lane; k < sb; k += 32) c_s[k] = c_in[(size_t)i * sb + k];
-  if (lane == 0) {
-    radial_basis<double>(rd.x, a.r1, rcut, N, a.cutoff_kind, gb, gb + N, 1);
-    real_harmonics<double>(rd.y, rd.z, rd.w, a.lmax, yb, yb + H, 1);
+  const int N = a.N, H = a.H, NS = a.n_species, nd = a.n_d, L1 = a.lmax + 1, nr = NS * N;
+  const int nrs = dp_sums_stride(a), nl = nrs * L1;
+  double *bas = reinterpret_cast<double *>(smem_raw);            // g, dg, Y, dY by pair
+  double *unit = bas + (size_t)(2 * N + 4 * H) * kDpStride;      // [3][kDpPairs]
+  double *ab = unit + 3 * kDpPairs + (size_t)warp * 6 * nl;      // rhat alpha, beta
+  const int t0 = blockIdx.x * kDpPairs, np = min(kDpPairs, npl - t0);
+  if (warp == 0 && lane < np) {
+    const int p = plist[t0 + lane], kc = species[nbr_i[p]] * NS + nbr_s[p];
+    const dvec4 rd = rel[p];
+    radial_basis<double>(rd.x, a.r1, a.cutoffs[kc], N, a.cutoff_kind, bas + lane,
+                         bas + N * kDpStride + lane, kDpStride, a.cinv64_hi[kc],
+                         a.cinv64_lo[kc]);
+    double *Y = bas + 2 * N * kDpStride + lane, *dY = Y + H * kDpStride;
+    const double ir = 1.0 / rd.x, ux = rd.y * ir, uy = rd.z * ir, uz = rd.w * ir;
+    if constexpr (SH::kL1 > 0)
+      harmonics64_grad<SH::kL1 - 1>(ux, uy, uz, ir, Y, dY, kDpStride);
+    else
+      real_harmonics<double>(rd.y, rd.z, rd.w, a.lmax, Y, dY, kDpStride);
+    unit[lane] = ux;
+    unit[kDpPairs + lane] = uy;
+    unit[2 * kDpPairs + lane] = uz;
   }
-  __syncwarp();
-  const double u[3] = {rd.y / rd.x, rd.z / rd.x, rd.w / rd.x};
-  for (int k = lane; k < 3 * N * H; k += 32) {
-    const int comp = k / (N * H), rem = k - comp * N * H, n = rem / H, lm = rem - n * H;
-    dc[k] = gb[N + n] * u[comp] * yb[lm] + gb[n] * yb[H + 3 * lm + comp];
-  }
-  __syncwarp();
-  const int L1 = a.lmax + 1;
-  double fdot[3] = {0, 0, 0};
-  for (int d = lane; d < nd; d += 32) {
-    const int q = d / L1, l = d - q * L1;
-    const int pr = pair_tab[q];
-    const int n1 = pr & 0xffff, n2 = pr >> 16;
-    const bool in1 = (n1 / N) == sj, in2 = (n2 / N) == sj;
-    const double pv = p_in[(size_t)i * nd + d];
-    for (int comp = 0; comp < 3; comp++) {
-      double v = 0.0;
-      for (int m = 0; m < 2 * l + 1; m++) {
-        const int lm = l * l + m;
-        if (in2) v += c_s[n1 * H + lm] * dc[comp * N * H + (n2 % N) * H + lm];
-        if (in1) v += dc[comp * N * H + (n1 % N) * H + lm] * c_s[n2 * H + lm];
+  __syncthreads();
+  for (int pi = warp; pi < np; pi += nwarps) {
+    const int idx = t0 + pi, p = plist[idx], i = nbr_i[p], s0 = nbr_s[p] * N;
+    const double *c = c_in + (size_t)i * nr * H;
+    const double *g = bas + pi, *dg = bas + N * kDpStride + pi;
+    const double *Y = bas + 2 * N * kDpStride + pi, *dY = Y + H * kDpStride;
+    for (int q = lane; q < nr * L1; q += 32) {
+      const int l = q / nr, n = q - l * nr;
+      double al = 0.0, be[3] = {0.0, 0.0, 0.0};
+      for (int lm = l * l; lm < (l + 1) * (l + 1); lm++) {
+        const double cv = c[n * H + lm];
+        al = fma(cv, Y[lm * kDpStride], al);
+#pragma unroll
+        for (int x = 0; x < 3; x++) be[x] = fma(cv, dY[(3 * lm + x) * kDpStride], be[x]);
       }
-      dp[(size_t)(3 * idx + comp) * ldd + d] = v;
-      fdot[comp] += v * pv;
+#pragma unroll
+      for (int x = 0; x < 3; x++) {
+        ab[x * nl + l * nrs + n] = al * unit[x * kDpPairs + pi];
+        ab[(3 + x) * nl + l * nrs + n] = be[x];
+      }
     }
-  }
-  for (int comp = 0; comp < 3; comp++) {
-    double v = warp_sum(fdot[comp]);
-    if (lane == 0) force_dots[3 * idx + comp] = v;
+    __syncwarp();
+    double fdot[3] = {0, 0, 0};
+    for (int d = lane; d < nd; d += 32) {
+      const int q = d / L1, l = d - q * L1;
+      const int pr = pair_tab[q];
+      const int n1 = pr & 0xffff, n2 = pr >> 16, m1 = n1 - s0, m2 = n2 - s0;
+      const bool in1 = (unsigned)m1 < (unsigned)N, in2 = (unsigned)m2 < (unsigned)N;
+      // the factors of a channel that is not the neighbor's are zero
+      const double g1 = in1 ? g[m1 * kDpStride] : 0.0, d1 = in1 ? dg[m1 * kDpStride] : 0.0;
+      const double g2 = in2 ? g[m2 * kDpStride] : 0.0, d2 = in2 ? dg[m2 * kDpStride] : 0.0;
+      const double *A1 = ab + l * nrs + n1, *A2 = ab + l * nrs + n2;
+      const double pv = p_in[(size_t)i * nd + d];
+#pragma unroll
+      for (int x = 0; x < 3; x++) {
+        double v = d2 * A1[x * nl];
+        v = fma(g2, A1[(3 + x) * nl], v);
+        v = fma(d1, A2[x * nl], v);
+        v = fma(g1, A2[(3 + x) * nl], v);
+        dp[(size_t)(3 * idx + x) * ldd + d] = v;
+        fdot[x] = fma(v, pv, fdot[x]);
+      }
+    }
+    for (int x = 0; x < 3; x++) {
+      const double v = warp_sum(fdot[x]);
+      if (lane == 0) force_dots[3 * idx + x] = v;
+    }
+    __syncwarp();
   }
 }
 
@@ -1383,19 +1422,19 @@ int launch_b2_dp(const B2Args &a, int npl, const int *plist, const int *nbr_i,
                                                          force_dots);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
   }
-  const int sb = a.n_species * a.N * a.H;
-  size_t per = sizeof(double) * (sb + 3 * a.N * a.H + 2 * a.N + 4 * a.H);
   int wpb = 4;
-  while (wpb > 1 && per * wpb > 200 * 1024) wpb >>= 1;
-  size_t smem = per * wpb;
+  while (wpb > 1 && dp_smem(a, wpb) > 200 * 1024) wpb >>= 1;
+  const size_t smem = dp_smem(a, wpb);
   if (smem > 227 * 1024) return -1;
-  if (cudaFuncSetAttribute(k_b2_dp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess)
-    return -1;
-  k_b2_dp<<<ceil_div(npl, wpb), 32 * wpb, smem, stream>>>(
-      a, npl, plist, nbr_i, nbr_s, rel, species, pair_tab, c_in, p_in, dp, ldd,
-      force_dots);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+  return with_lmax<double>(a, [&](auto sh) {
+    auto kern = k_b2_dp<decltype(sh)>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        cudaSuccess)
+      return -1;
+    kern<<<ceil_div(npl, kDpPairs), 32 * wpb, smem, stream>>>(
+        a, npl, plist, nbr_i, nbr_s, rel, species, pair_tab, c_in, p_in, dp, ldd, force_dots);
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+  });
 }
 
 // FP32 pair forces, one warp per atom: lanes take the atom's pairs (f_ij
