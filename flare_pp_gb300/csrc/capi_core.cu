@@ -117,6 +117,8 @@ int fpp_structure_create(const double *cell, const int32_t *species,
   int smax = 0;
   for (int i = 0; i < noa; i++) smax = std::max(smax, species[i] + 1);
   st.n_species_max = smax;
+  st.species_count.assign(smax, 0);
+  for (int i = 0; i < noa; i++) st.species_count[species[i]]++;
   cudaStream_t cs = (cudaStream_t)stream;
   if ((rc = st.positions.reserve(sizeof(double) * 3 * std::max(noa, 1))) != FPP_OK ||
       (rc = st.species.reserve(sizeof(int) * std::max(noa, 1))) != FPP_OK) {

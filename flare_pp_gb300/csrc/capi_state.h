@@ -110,7 +110,7 @@ struct fpp_model {
   // scalars, z / C / K blocks, second products, column sums and partials
   fpp::DevBuf kf_rows, kf_z, kf_q, kf_cols;
   fpp_structure *batch = nullptr;       // packed structure of a batched prediction
-  fpp::DevBuf batch_aoff, batch_poff, batch_sums, batch_src;
+  fpp::DevBuf batch_off, batch_sums, batch_src;
   // envs_struc workspace of the stored-derivative form (grown on demand, kept between calls)
   fpp::DevBuf es_rown, es_ndm, es_flags, es_pos, es_scan, es_plist, es_qatom, es_dmap,
       es_dp, es_sfd, es_fd;
