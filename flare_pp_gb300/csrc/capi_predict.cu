@@ -262,10 +262,17 @@ static int forward32(fpp_structure *s, const B2Args &a0, const int *pair_tab, in
   return FPP_OK;
 }
 
-// energy and the flare-order stress -(1/V) sum f_a r_b from the reduced row
+// energy and the flare-order stress -(1/V) sum f_a r_b from the reduced row, and the
+// caller's copies of the forces and atom energies (one launch for what a kernel and two
+// copies did: at a hundred atoms each costs as much)
 __global__ void k_finish(const double *__restrict__ red, double vi, double *energy,
-                         double *stress) {
-  if (threadIdx.x != 0) return;
+                         double *stress, int nf, const double *__restrict__ f,
+                         double *__restrict__ forces, int na, const double *__restrict__ ae,
+                         double *__restrict__ atom_energies) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, n = gridDim.x * blockDim.x;
+  for (int i = t; i < nf; i += n) forces[i] = f[i];
+  for (int i = t; i < na; i += n) atom_energies[i] = ae[i];
+  if (t != 0) return;
   if (energy) energy[0] = red[0];
   if (stress) {
     stress[0] = -red[1] * vi;
@@ -285,16 +292,13 @@ static int finish_outputs(fpp_structure *s, cudaStream_t st, double *energy,
     // stays asynchronous: the outputs are written in stream order, and a
     // device-side error of this call is reported by the next synchronizing
     // call on the structure (the status word is only cleared once read)
-    if (energy || stress) {
-      k_finish<<<1, 32, 0, st>>>(S.reduce_out.as<double>(), 1.0 / S.ci.volume, energy, stress);
+    const int nf = forces ? 3 * S.noa : 0, na = atom_energies ? S.noa : 0;
+    if (energy || stress || nf || na) {
+      k_finish<<<std::min(ceil_div(std::max(nf, 1), 256), 152 * 8), 256, 0, st>>>(
+          S.reduce_out.as<double>(), 1.0 / S.ci.volume, energy, stress, nf,
+          S.forces.as<double>(), forces, na, S.atom_e.as<double>(), atom_energies);
       FPP_CUDA(cudaGetLastError());
     }
-    if (forces && S.noa)
-      FPP_CUDA(cudaMemcpyAsync(forces, S.forces.ptr, sizeof(double) * 3 * S.noa,
-                               cudaMemcpyDeviceToDevice, st));
-    if (atom_energies && S.noa)
-      FPP_CUDA(cudaMemcpyAsync(atom_energies, S.atom_e.ptr, sizeof(double) * S.noa,
-                               cudaMemcpyDeviceToDevice, st));
     return FPP_OK;
   }
   // every device-to-host copy of the call, then one synchronization

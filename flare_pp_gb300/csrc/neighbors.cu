@@ -124,8 +124,14 @@ __global__ void k_wrap_bin(int noa, const double *__restrict__ pos, CellDev cd,
                            dvec4 *__restrict__ wp, float4 *__restrict__ wp32,
                            float4 *__restrict__ wp_lo,
                            float4 *__restrict__ frac, int *__restrict__ atom_bin,
-                           int *__restrict__ bin_count, DeviceStatus *st) {
+                           int *__restrict__ bin_count, int *__restrict__ bin_cursor,
+                           int nbins, int *__restrict__ flags, int *__restrict__ count_end,
+                           DeviceStatus *st) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  // what later kernels of the build count in starts at zero (a memset each before)
+  for (int b = i; b < nbins; b += gridDim.x * blockDim.x) bin_cursor[b] = 0;
+  if (i < 4) flags[i] = 0;
+  if (i == 0) *count_end = 0;
   if (i >= noa) return;
   double p[3] = {pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]};
   if (!isfinite(p[0]) || !isfinite(p[1]) || !isfinite(p[2])) {
@@ -790,18 +796,95 @@ int check_status(StructureState &st, cudaStream_t stream, const char *what) {
   return status_from_readback(st, stream, what);
 }
 
-// The pair total, the slab overflow flag and the status word into the
-// host-visible readback block (one thread).
-__global__ void k_nb_readback(const int *__restrict__ total, const int *__restrict__ flags,
-                              const DeviceStatus *__restrict__ status,
-                              HostReadback *__restrict__ rb) {
-  if (threadIdx.x != 0) return;
-  rb->total_pairs = *total;
+__device__ __forceinline__ void nb_readback(int total, const int *flags,
+                                            const DeviceStatus *status, HostReadback *rb) {
+  rb->total_pairs = total;
   rb->overflow = flags[0];
   rb->status[0] = status->code;
   rb->status[1] = status->where;
   rb->status[2] = status->info;
   rb->status[3] = status->pad;
+}
+
+// out[i] = in[0] + .. + in[i - 1] for i = 0 .. n by one block (n <= kScanItems), and the
+// readback below if rb.  A small structure's build is as long as its chain of launches:
+// one instead of three (the library scan's two, the readback); a block's eight entries
+// per thread are loaded at once, so its time is that of one pass.
+constexpr int kScanItems = 8192;
+__global__ void __launch_bounds__(1024)
+k_scan_small(int n, const int *__restrict__ in, int *__restrict__ out,
+             const int *__restrict__ flags, const DeviceStatus *__restrict__ status,
+             HostReadback *__restrict__ rb) {
+  __shared__ int warp_sum[32];
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  int v[8], sum = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const int i = 8 * t + k;
+    v[k] = i < n ? in[i] : 0;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; k++) sum += v[k];
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  if (lane == 31) warp_sum[warp] = incl;
+  __syncthreads();
+  if (warp == 0) {
+    int w = warp_sum[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += u;
+    }
+    warp_sum[lane] = w;
+  }
+  __syncthreads();
+  int run = incl - sum + (warp > 0 ? warp_sum[warp - 1] : 0);
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const int i = 8 * t + k;
+    if (i <= n) out[i] = run;
+    run += v[k];
+  }
+  // the total's own place, where n fills the block's entries
+  if (t == 1023 && n == kScanItems) out[n] = run;
+  if (rb && t == 0) nb_readback(warp_sum[31], flags, status, rb);
+}
+
+// The pair total, the slab overflow flag and the status word into the
+// host-visible readback block (one thread).
+__global__ void k_nb_readback(const int *__restrict__ total, const int *__restrict__ flags,
+                              const DeviceStatus *__restrict__ status,
+                              HostReadback *__restrict__ rb) {
+  if (threadIdx.x == 0) nb_readback(*total, flags, status, rb);
+}
+
+// Exclusive sums of n counts and their total (n + 1 entries out; in[n] is zero), with the
+// readback if rb: one block where it holds them, else the library's scan.  At 8,192
+// entries the block takes as long as the library's two launches and the readback.
+static int scan_counts(StructureState &st, int n, const int *in, int *out, HostReadback *rb,
+                       cudaStream_t stream) {
+  if (n <= kScanItems) {
+    k_scan_small<<<1, 1024, 0, stream>>>(n, in, out, st.flags.as<int>(),
+                                         st.status.as<DeviceStatus>(), rb);
+    FPP_CUDA(cudaGetLastError());
+    return FPP_OK;
+  }
+  size_t tmp = 0;
+  FPP_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp, in, out, n + 1, stream));
+  FPP_TRY(st.scan_tmp.reserve(tmp));
+  tmp = st.scan_tmp.bytes;
+  FPP_CUDA(cub::DeviceScan::ExclusiveSum(st.scan_tmp.ptr, tmp, in, out, n + 1, stream));
+  if (rb) {
+    k_nb_readback<<<1, 32, 0, stream>>>(out + n, st.flags.as<int>(),
+                                        st.status.as<DeviceStatus>(), rb);
+    FPP_CUDA(cudaGetLastError());
+  }
+  return FPP_OK;
 }
 
 // Pairs the pair buffers hold (0 before the first build; the FP64 table,
@@ -846,27 +929,19 @@ int build_neighbors(StructureState &st, cudaStream_t stream) {
   FPP_TRY(st.bin_start.reserve(sizeof(int) * (nbins + 1)));
   FPP_TRY(st.bin_cursor.reserve(sizeof(int) * nbins));
   FPP_CUDA(cudaMemsetAsync(st.bin_count.ptr, 0, sizeof(int) * (nbins + 1), stream));
-  FPP_CUDA(cudaMemsetAsync(st.bin_cursor.ptr, 0, sizeof(int) * nbins, stream));
+  FPP_TRY(st.flags.reserve(sizeof(int) * 4));
   DeviceStatus *dst = st.status.as<DeviceStatus>();
 
   const int tb = 256;
   k_wrap_bin<<<ceil_div(noa, tb), tb, 0, stream>>>(
       noa, st.positions.as<double>(), cd, st.wrapped.as<dvec4>(),
       st.wrapped32.as<float4>(), st.wrapped_lo.as<float4>(), st.frac.as<float4>(),
-      st.atom_bin.as<int>(),
-      st.bin_count.as<int>(), dst);
+      st.atom_bin.as<int>(), st.bin_count.as<int>(), st.bin_cursor.as<int>(), nbins,
+      st.flags.as<int>(), st.nbr_count.as<int>() + noa, dst);
   FPP_CUDA(cudaGetLastError());
 
-  size_t tmp_bytes = 0, t2 = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, st.bin_count.as<int>(),
-                                st.bin_start.as<int>(), nbins + 1, stream);
-  cub::DeviceScan::ExclusiveSum(nullptr, t2, st.nbr_count.as<int>(),
-                                st.nbr_offset.as<int>(), noa + 1, stream);
-  FPP_TRY(st.scan_tmp.reserve(std::max(tmp_bytes, t2)));
-  tmp_bytes = st.scan_tmp.bytes;
-  FPP_CUDA(cub::DeviceScan::ExclusiveSum(st.scan_tmp.ptr, tmp_bytes,
-                                         st.bin_count.as<int>(),
-                                         st.bin_start.as<int>(), nbins + 1, stream));
+  FPP_TRY(scan_counts(st, nbins, st.bin_count.as<int>(), st.bin_start.as<int>(), nullptr,
+                      stream));
   FPP_TRY(st.binned.reserve(sizeof(float4) * noa));
   k_bin_scatter<<<ceil_div(noa, tb), tb, 0, stream>>>(
       noa, st.atom_bin.as<int>(), st.bin_start.as<int>(), st.bin_cursor.as<int>(),
@@ -875,25 +950,17 @@ int build_neighbors(StructureState &st, cudaStream_t stream) {
 
   const int wpb = 4;  // warps per block, one atom per warp
   dim3 grid(ceil_div(noa, wpb)), block(32 * wpb);
-  FPP_CUDA(cudaMemsetAsync(st.nbr_count.as<int>() + noa, 0, sizeof(int), stream));
   // single pass into the per-atom slab
   FPP_TRY(st.slab.reserve(sizeof(long long) * (size_t)noa * kSlabCap));
-  FPP_TRY(st.flags.reserve(sizeof(int) * 4));
-  FPP_CUDA(cudaMemsetAsync(st.flags.ptr, 0, sizeof(int) * 4, stream));
   k_enum<<<ceil_div(noa, kEnumWarps), 32 * kEnumWarps, 0, stream>>>(
       noa, cd, st.wrapped.as<dvec4>(), st.wrapped32.as<float4>(), st.wrapped_lo.as<float4>(),
       st.frac.as<float4>(), st.bin_start.as<int>(), st.binned.as<float4>(),
       st.nbr_count.as<int>(),
       st.slab.as<long long>(), st.flags.as<int>());
   FPP_CUDA(cudaGetLastError());
-  tmp_bytes = st.scan_tmp.bytes;
-  FPP_CUDA(cub::DeviceScan::ExclusiveSum(st.scan_tmp.ptr, tmp_bytes,
-                                         st.nbr_count.as<int>(),
-                                         st.nbr_offset.as<int>(), noa + 1, stream));
   FPP_TRY(ensure_readback(st));
-  k_nb_readback<<<1, 32, 0, stream>>>(st.nbr_offset.as<int>() + noa, st.flags.as<int>(),
-                                      st.status.as<DeviceStatus>(), st.rb_dev);
-  FPP_CUDA(cudaGetLastError());
+  FPP_TRY(scan_counts(st, noa, st.nbr_count.as<int>(), st.nbr_offset.as<int>(), st.rb_dev,
+                      stream));
   if (!st.nb_ready) FPP_CUDA(cudaEventCreateWithFlags(&st.nb_ready, cudaEventDisableTiming));
   FPP_CUDA(cudaEventRecord(st.nb_ready, stream));
   // the compaction into the pair buffers of an earlier build, queued before
@@ -920,10 +987,8 @@ int build_neighbors(StructureState &st, cudaStream_t stream) {
                                         st.bin_start.as<int>(), st.bin_atoms.as<int>(),
                                         st.nbr_count.as<int>());
     FPP_CUDA(cudaGetLastError());
-    tmp_bytes = st.scan_tmp.bytes;
-    FPP_CUDA(cub::DeviceScan::ExclusiveSum(st.scan_tmp.ptr, tmp_bytes,
-                                           st.nbr_count.as<int>(),
-                                           st.nbr_offset.as<int>(), noa + 1, stream));
+    FPP_TRY(scan_counts(st, noa, st.nbr_count.as<int>(), st.nbr_offset.as<int>(), nullptr,
+                        stream));
     FPP_CUDA(cudaMemcpyAsync(&total, st.nbr_offset.as<int>() + noa, sizeof(int),
                              cudaMemcpyDeviceToHost, stream));
     FPP_CUDA(cudaStreamSynchronize(stream));
