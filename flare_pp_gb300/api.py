@@ -284,13 +284,17 @@ class B2(_Handle):
         dv.cumulative_type_count = [0]
         for s in range(ns):
             atoms = np.nonzero(sp == s)[0]
+            # consecutive atoms (one species, or sorted by species): slices of the
+            # arrays instead of copies of them
+            run = len(atoms) > 0 and atoms[-1] - atoms[0] + 1 == len(atoms)
+            pick = slice(atoms[0], atoms[-1] + 1) if run else atoms
             nn = cnt[atoms].astype(np.int64)
             dv.n_clusters_by_type.append(len(atoms))
             dv.cumulative_type_count.append(dv.cumulative_type_count[s] + len(atoms))
             dv.n_clusters += len(atoms)
             dv.n_neighbors_by_type.append(int(nn.sum()))
-            dv.descriptors.append(desc[atoms])
-            dv.descriptor_norms.append(norms[atoms])
+            dv.descriptors.append(desc[pick])
+            dv.descriptor_norms.append(norms[pick])
             dv.cutoff_values.append(np.ones(len(atoms)))
             dv.cutoff_dervs.append(np.zeros(3 * int(nn.sum())))
             dv.neighbor_counts.append(nn)
@@ -298,12 +302,16 @@ class B2(_Handle):
                 np.concatenate([[0], np.cumsum(nn)[:-1]]).astype(np.int64)
                 if len(atoms) else np.zeros(0, np.int64))
             dv.atom_indices.append(atoms)
-            rows = (np.concatenate([np.arange(cum[a], cum[a + 1]) for a in atoms])
-                    if len(atoms) else np.zeros(0, np.int64)).astype(np.int64)
+            if run:
+                rows = slice(cum[atoms[0]], cum[atoms[-1] + 1])
+                frows = slice(3 * rows.start, 3 * rows.stop)
+            else:
+                rows = (np.concatenate([np.arange(cum[a], cum[a + 1]) for a in atoms])
+                        if len(atoms) else np.zeros(0, np.int64)).astype(np.int64)
+                frows = (3 * rows[:, None] + np.arange(3)[None]).ravel()
             dv.neighbor_indices.append(nidx[rows].astype(np.int64))
             dv.neighbor_coordinates.append(ncoord[rows])
             if self.store_dervs:
-                frows = (3 * rows[:, None] + np.arange(3)[None]).ravel()
                 dv.descriptor_force_dervs.append(dervs[frows])
                 dv.descriptor_force_dots.append(dots[frows])
             else:
@@ -1073,14 +1081,16 @@ class SparseGP:
         n = len(structures)
         counts = [s.noa for s in structures]
         hs = (_lib.ctypes.c_void_p * max(1, n))(*[s.handle for s in structures])
-        E, F, S = np.zeros(n), np.zeros((sum(counts), 3)), np.zeros((n, 6))
-        e, f, st = np.zeros(n), np.zeros((sum(counts), 3)), np.zeros((n, 6))
+        total = None
         for m in self._models:      # the kernels' contributions add
+            e, f, st = np.zeros(n), np.zeros((sum(counts), 3)), np.zeros((n, 6))
             check(lib().fpp_predict_mapped_batched(m.handle, hs, n, PRECISIONS[precision],
                                                    ptr(e), ptr(f), ptr(st), _stream(stream)))
-            E, F, S = E + e, F + f, S + st
-        offs = np.concatenate([[0], np.cumsum(counts)])
-        return E, [F[offs[k]:offs[k + 1]] for k in range(n)], S
+            total = (e, f, st) if total is None else tuple(
+                a + b for a, b in zip(total, (e, f, st)))
+        E, F, S = total or (np.zeros(n), np.zeros((sum(counts), 3)), np.zeros((n, 6)))
+        offs = np.concatenate([[0], np.cumsum(counts)]).tolist()
+        return E, [F[a:b] for a, b in zip(offs[:-1], offs[1:])], S
 
     def center_mixed_on(self, structure, stream=None):
         """Centre the mixed-precision mapped form on this structure's mean
