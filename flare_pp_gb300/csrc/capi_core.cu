@@ -31,6 +31,12 @@ DevBuf::~DevBuf() {
   if (ptr) cudaFree(ptr);
 }
 
+void DevBuf::release() {
+  if (ptr) cudaFree(ptr);
+  ptr = nullptr;
+  bytes = 0;
+}
+
 int DevBuf::reserve(size_t n) {
   if (n <= bytes && ptr) return FPP_OK;
   if (ptr) {

@@ -1015,13 +1015,16 @@ static int envs_struc_device(fpp_model *m, fpp_structure *s, cudaStream_t st, De
   FPP_TRY(forward64(s, a, m->pair_tab.as<int>(), !gemm, st));
   double *phat = S.phat64.as<double>();
   if (gemm && m->n_sparse_total > 0) {
+    std::lock_guard<std::mutex> lock(m->kuf_mu);
     KufItem it;
     std::memset(&it, 0, sizeof(it));
     it.s = s;
     it.col_f0 = 1;
     it.q.col_s = 1 + 3ll * noa;
     FPP_TRY(kuf_gemm(m, m->kuf_work, {it}, K.as<double>(), n_out, st));
-    return ozaki_check_status(m->oz, st);
+    FPP_TRY(ozaki_check_status(m->oz, st));
+    m->kuf_work.trim();
+    return FPP_OK;
   }
   // row-ordered atom norms
   DevBuf &rown = m->es_rown;
@@ -1228,7 +1231,9 @@ int fpp_kuf_batched(fpp_model *m, fpp_structure *const *structures, int32_t n_st
   FPP_TRY(upload_pair_tab(m->pair_tab, m->pair_tab_host, st));
   // FP64 descriptors of every structure, queued without synchronization
   // (each structure keeps its own workspace), and the work lists
-  DevBuf dK, dfcol, dstruc, ditems;
+  std::lock_guard<std::mutex> lock(m->kuf_mu);
+  KufWork &work = m->kuf_work;
+  DevBuf &dK = work.K, &dfcol = work.cols, dstruc, ditems;
   FPP_TRY(dK.reserve(sizeof(double) * (size_t)nst * n_labels));
   FPP_CUDA(cudaMemsetAsync(dK.ptr, 0, sizeof(double) * (size_t)nst * n_labels, st));
   FPP_TRY(dfcol.reserve(sizeof(int) * fcol.size()));
@@ -1309,7 +1314,6 @@ int fpp_kuf_batched(fpp_model *m, fpp_structure *const *structures, int32_t n_st
     FPP_TRY(kuf_tiles(m, ka, (int)items.size(), st, &ks, &threads));
     FPP_CUDA(cudaMemsetAsync(dK.ptr, 0, sizeof(double) * (size_t)nst * n_labels, st));
   }
-  KufWork work;
   FPP_CUDA(cudaEventRecord(ev.e0, st));
   if (!batch.empty()) FPP_TRY(kuf_gemm(m, work, batch, dK.as<double>(), n_labels, st));
   if (!items.empty() &&
@@ -1326,6 +1330,7 @@ int fpp_kuf_batched(fpp_model *m, fpp_structure *const *structures, int32_t n_st
   float ms = 0.f;
   FPP_CUDA(cudaEventElapsedTime(&ms, ev.e0, ev.e1));
   m->kuf_ms = ms;
+  work.trim();
   return FPP_OK;
 }
 
@@ -1598,7 +1603,7 @@ int fpp_envs_struc(fpp_model *m, fpp_structure *s, double *kernel_mat, void *str
   FPP_TRY(model_check(m, s));
   if (!kernel_mat) return fail(FPP_ERR_INVALID, "null output");
   cudaStream_t st = (cudaStream_t)stream;
-  DevBuf K;
+  DevBuf &K = m->es_K;
   FPP_TRY(envs_struc_device(m, s, st, K));
   FPP_CUDA(cudaStreamSynchronize(st));
   const size_t n = (size_t)m->n_sparse_total * (1 + 3 * s->st.noa + 6);
@@ -1625,33 +1630,47 @@ int fpp_predict(fpp_model *m, fpp_structure *s, double *mean_efs, double *varian
     FPP_TRY(get_cublas(m, st, &h));
     const double one = 1.0, zero = 0.0;
     if (!m->has_R_inv) return fail(FPP_ERR_INVALID, "R_inv not set (fpp_model_set_R_inv)");
-    DevBuf K, alpha, mean, V, var;
+    DevBuf &K = m->es_K;
     FPP_TRY(envs_struc_device(m, s, st, K));
     std::vector<double> al(std::max(nst, 1), 0.0);
     for (auto &x : m->sp)
       for (int k = 0; k < x.n_sparse; k++) al[x.sparse_offset + k] = x.alpha[k];
-    FPP_TRY(alpha.reserve(sizeof(double) * al.size()));
-    FPP_TRY(mean.reserve(sizeof(double) * n_out));
-    FPP_TRY(V.reserve(sizeof(double) * (size_t)n_out * std::max(nst, 1)));
-    FPP_TRY(var.reserve(sizeof(double) * n_out));
-    FPP_CUDA(cudaMemcpyAsync(alpha.ptr, al.data(), sizeof(double) * al.size(), cudaMemcpyHostToDevice, st));
-    FPP_CUBLAS(cublasDgemv(h, CUBLAS_OP_N, n_out, nst, &one, K.as<double>(), n_out,
-                           alpha.as<double>(), 1, &zero, mean.as<double>(), 1));
+    // one workspace kept with the model: V and K^T (n_out x nst), alpha, mean, variance
+    const size_t n1 = std::max(nst, 1), nv = (size_t)n_out * n1;
+    FPP_TRY(m->sor.reserve(sizeof(double) * (2 * nv + n1 + 2 * (size_t)n_out)));
+    double *V = m->sor.as<double>(), *KT = V + nv, *alpha = KT + nv, *mean = alpha + n1,
+           *var = mean + n_out;
+    FPP_CUDA(cudaMemcpyAsync(alpha, al.data(), sizeof(double) * al.size(), cudaMemcpyHostToDevice, st));
+    FPP_CUBLAS(cublasDgemv(h, CUBLAS_OP_N, n_out, nst, &one, K.as<double>(), n_out, alpha, 1,
+                           &zero, mean, 1));
     // V[o][i] = sum_k K[k][o] R_inv[k][i] (predict_SOR's R_inv^T K, row o per
     // label) on the tensor cores, FP64-accurate: operands K^T and R_inv^T
-    DevBuf KT, RT;
-    FPP_TRY(KT.reserve(sizeof(double) * (size_t)n_out * std::max(nst, 1)));
-    FPP_TRY(RT.reserve(sizeof(double) * (size_t)std::max(nst, 1) * std::max(nst, 1)));
-    if (launch_transpose(nst, n_out, K.as<double>(), n_out, KT.as<double>(), nst, st) != 0 ||
-        launch_transpose(nst, nst, m->R_inv.as<double>(), nst, RT.as<double>(), nst, st) != 0)
-      return fail(FPP_ERR_CUDA, "transpose launch failed");
-    FPP_TRY(ozaki_dgemm_nt(n_out, nst, nst, KT.as<double>(), nst, RT.as<double>(), nst,
-                           V.as<double>(), nst, m->oz, st, m->R_inv_upper));
-    if (launch_row_sq(n_out, nst, V.as<double>(), nst, var.as<double>(), st) != 0)
+    if (nst > 0) {
+      if (!(m->oz_RinvT.ready && m->oz_RinvT.rows == nst && m->oz_RinvT.K == nst)) {
+        DevBuf RT;
+        FPP_TRY(RT.reserve(sizeof(double) * (size_t)nst * nst));
+        if (launch_transpose(nst, nst, m->R_inv.as<double>(), nst, RT.as<double>(), nst, st) != 0)
+          return fail(FPP_ERR_CUDA, "transpose launch failed");
+        FPP_TRY(ozaki_const(m->oz_RinvT, nst, nst, RT.as<double>(), nst, st));
+      }
+      DeviceStatus *status;
+      FPP_TRY(ozaki_status(m->oz, st, &status));
+      if (launch_transpose(nst, n_out, K.as<double>(), n_out, KT, nst, st) != 0)
+        return fail(FPP_ERR_CUDA, "transpose launch failed");
+      FPP_TRY(ozaki_split(m->oz.a, n_out, nst, KT, nst, st));
+      const OzakiProblem q{ozaki_mat(m->oz.a), ozaki_mat(m->oz_RinvT), 0, n_out, nst, V, nst,
+                           m->R_inv_upper};
+      FPP_TRY(ozaki_run(&q, 1, status, st));
+    }
+    if (launch_row_sq(n_out, nst, V, nst, var, st) != 0)
       return fail(FPP_ERR_CUDA, "variance launch failed");
+    std::vector<double> out(2 * (size_t)n_out);
+    FPP_CUDA(cudaMemcpyAsync(out.data(), mean, sizeof(double) * out.size(),
+                             cudaMemcpyDeviceToHost, st));
     FPP_TRY(ozaki_check_status(m->oz, st));
-    FPP_CUDA(cudaMemcpy(mean_efs, mean.ptr, sizeof(double) * n_out, cudaMemcpyDeviceToHost));
-    FPP_CUDA(cudaMemcpy(variance_efs, var.ptr, sizeof(double) * n_out, cudaMemcpyDeviceToHost));
+    FPP_CUDA(cudaStreamSynchronize(st));
+    std::copy(out.begin(), out.begin() + n_out, mean_efs);
+    std::copy(out.begin() + n_out, out.end(), variance_efs);
     return FPP_OK;
   }
   // mean through the adjoint

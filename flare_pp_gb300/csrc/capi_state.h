@@ -3,6 +3,7 @@
 #include <cublas_v2.h>
 #include <cuda_fp16.h>
 
+#include <mutex>
 #include <vector>
 
 #include "b2_kernels.h"
@@ -33,6 +34,17 @@ struct KufWork {
   DevBuf tables, pairs;        // structures and blocks; pairs by class
   DevBuf z_planes, z;          // atoms: digit planes, z / a / sums of t
   DevBuf planes, f, partial;   // derivative rows: digit planes, products; block sums
+  DevBuf K, cols;              // fpp_kuf_batched: the result, force columns
+  // Kept between calls (allocating and freeing it took a tenth of a call of 32 cells)
+  // up to this much, given back above it and with the model.
+  static constexpr size_t kKeep = (size_t)2 << 30;
+  void trim() {
+    if (tables.bytes + pairs.bytes + z_planes.bytes + z.bytes + planes.bytes + f.bytes +
+            partial.bytes + K.bytes + cols.bytes <= kKeep)
+      return;
+    for (DevBuf *b : {&tables, &pairs, &z_planes, &z, &planes, &f, &partial, &K, &cols})
+      b->release();
+  }
 };
 }  // namespace fpp
 
@@ -105,7 +117,9 @@ struct fpp_model {
   fpp::OzakiOperand oz_RinvT;
   fpp::OzakiOperand oz_kuf;             // digit planes of dhat by pair class (capi_kuf.cu)
   fpp::DevBuf kuf_tab;                  // its column tables
-  fpp::KufWork kuf_work;                // envs_struc workspace, kept between calls
+  fpp::KufWork kuf_work;                // Kuf and envs_struc workspace
+  std::mutex kuf_mu;                    // held while a call uses it
+  fpp::DevBuf es_K, sor;                // kernel matrix of a structure; SOR products
   // kernel-form workspaces (grown on demand, kept between calls): per-row
   // scalars, z / C / K blocks, second products, column sums and partials
   fpp::DevBuf kf_rows, kf_z, kf_q, kf_cols;

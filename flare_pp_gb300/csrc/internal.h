@@ -40,6 +40,7 @@ struct DevBuf {
   }
   ~DevBuf();
   int reserve(size_t n);  // at least n bytes; contents not preserved
+  void release();
   template <typename T> T *as() const { return static_cast<T *>(ptr); }
 };
 
