@@ -23,29 +23,37 @@
 // (their level sums could run over 1536 columns, which FP64 epilogue sums need:
 // FP64 issues 2 per clock and SM; the integer ones do not).
 //
-// What bounds it: shared memory.  An N = 128 MMA takes 64 cycles and reads 8 KB, all
-// of the SM's 128 bytes per cycle, and TMA writes there too.  So
+// What bounds it: an N = 128 MMA of one SM takes 64 cycles and reads 8 KB, all of the
+// SM's 128 bytes per cycle, and TMA writes there too.  So
+//  - a CTA pair (cluster of two, cta_group::2) takes a 256-row tile: each SM reads its own
+//    128 rows of A and half of the columns' rows of B, and half of B is loaded;
 //  - a K block's digit tiles are loaded once per group of levels and used in all its
 //    pairs: the pairs of levels L0..L1 run by ascending A digit s, whose partners
 //    t = L0-s .. L1-s are a window sliding down the B digits; A tiles live one step,
 //    B tiles four or five (24 tile loads feed 36 pairs; one A and one B tile per
-//    pair before);
-//  - two neighboring partners make one N = 256 MMA, which reads A once.
-// The issuing thread comes next: its loops are unrolled per group (376 cycles per
-// pair with the slots worked out at run time, where the pair's MMAs take 256) and
-// its tcgen05 instructions stand under elect.sync.  Measured at 4096 x 2048 x 1500:
-// 13.8 TFLOP/s FP64-equivalent with the 5-bit digits, 17.7 with these and run-time
-// slots, 26.6 unrolled, 28.9 with elect.sync and N = 256, 34.2 with integer group
-// sums in place of FP64 conversions and 32-byte accesses to C (36 pairs, one
-// launch; the MMAs alone would take 52).
+//    pair before).
+// Then come the single threads that feed the tensor cores.  The issuer's loops are
+// unrolled per group (376 cycles per pair with the slots worked out at run time, where
+// the pair's MMAs take 256), its tcgen05 instructions stand under elect.sync, and it
+// waits for a step's operands behind the first MMAs of the step before (the tensor
+// cores' queue is short: a wait between steps left them idle).  A and B have a producer
+// each (one thread took as long to issue 24 loads as the pairs take).
+// Measured at 4096 x 2048 x 1500 (36 pairs, one launch), TFLOP/s FP64-equivalent: 13.8
+// with the 5-bit digits; 17.7 with these and run-time slots; 26.6 unrolled; 28.9 with
+// elect.sync; 34.2 with integer group sums in place of FP64 conversions and 32-byte
+// accesses to C; 34.5 with two producers, 37.0 with the waits moved, 41.1 in CTA pairs
+// (pairs alone, before the producers and the waits, gave nothing).  1000 x 1050 x 1050:
+// 154 us before the last three, 117 so.  The MMAs alone would take 52; 256 tiles over 76
+// pairs fill 84 % of four rounds.
 //
-// Kernel layout (one persistent CTA per SM, 576 threads):
-//   warp 0 lane 0  TMA producer: 128B-swizzled 128 x 64 digit tiles into two
-//                  rings (A: 6 slots, B: 8 slots)
-//   warp 1         MMA issuer (one elected lane): per unit (tile, group of
-//                  levels, K chunk) the pairs of its four levels into four
-//                  128-column accumulators (all of TMEM); a level is handed to the epilogue as soon as
-//                  its last pair of the chunk is issued
+// Kernel layout (one persistent CTA per SM, 608 threads; in pairs):
+//   warps 0, 18    TMA producers (one lane): 128B-swizzled digit tiles, 128 x 64 of A and
+//                  bn / 2 x 64 of B, into two rings (A: 8 slots, B: 12); the pair's
+//                  loads are counted on the even CTA's barriers
+//   warp 1         MMA issuer (the even CTA's, one elected lane): per unit (tile, group
+//                  of levels, K chunk) the pairs of its four levels into four
+//                  accumulators of bn columns; a level is handed to both epilogues as
+//                  soon as its last pair of the chunk is issued
 //   warps 2-17     epilogue: four warps per TMEM lane quarter, each owning 32
 //                  columns of its 32 rows: tcgen05.ld, then the level's integer
 //                  into 64-bit sums held in registers over all chunks.  The
@@ -69,14 +77,17 @@ namespace fpp {
 
 namespace {
 constexpr int OBM = 128, OBN = 128, OBK = kTmaBoxK;  // OBN: most columns of a tile
-constexpr int OTILE = OBM * OBK * 2;    // bytes of one digit tile (A or B)
-constexpr int ONA = 6, ONB = 8;         // ring slots
+constexpr int OTILE = OBM * OBK * 2;    // bytes of one CTA's A digit tile
+constexpr int OBTILE = OTILE / 2;       // most bytes of its half of a B digit tile
+constexpr int ONA = 8, ONB = 12;        // ring slots
 constexpr int OLEV = 4;                 // levels per half (TMEM accumulators)
 constexpr int OTMEM_COLS = OLEV * OBN;
 constexpr int OEPI = 16;                // epilogue warps
 constexpr int OCOLS = 4 * OBN / OEPI;   // columns of an epilogue warp
-constexpr int OTHREADS = 32 * (2 + OEPI);
-constexpr int OSMEM_BYTES = (ONA + ONB) * OTILE + 1024 /*align*/ + 512 /*barriers*/;
+constexpr int OPROD_B = 2 + OEPI;       // the second producer warp
+constexpr int OTHREADS = 32 * (3 + OEPI);
+constexpr int OSMEM_BYTES =
+    ONA * OTILE + ONB * OBTILE + 1024 /*align*/ + 512 /*barriers*/;
 static_assert(OTMEM_COLS == 512, "four levels of a group fill TMEM");
 static_assert(ONB > OLEV + 1, "the live B digits of a step and a slot to fill");
 }  // namespace
@@ -94,7 +105,7 @@ struct OzakiParams {
   CUtensorMap a[kOzakiMaxGroups], b[kOzakiMaxGroups];
   OzakiGroup g[kOzakiMaxGroups];
   int n_groups, n_tiles;
-  int bn;                    // columns of a tile (a multiple of 16, 64 .. OBN)
+  int bn;                    // columns of a tile (a multiple of 32, 64 .. OBN)
   int n_levels;              // levels 0 .. n_levels - 1 (8 or 9)
   DeviceStatus *status;
 };
@@ -207,20 +218,20 @@ __device__ __forceinline__ double scale_pow2(double v, int k) {
   return v * p2(k1) * p2(k2) * p2(k - k1 - k2);
 }
 
-__global__ void __launch_bounds__(OTHREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(OTHREADS, 1)
 k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
   const int bn = p.bn;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char *gbase = smem_raw + (base - raw);
-  constexpr int kBarOff = (ONA + ONB) * OTILE;
+  constexpr int kBarOff = ONA * OTILE + ONB * OBTILE;
   constexpr int kBars = 2 * (ONA + ONB) + 2 * OLEV;
   const uint32_t bars = base + kBarOff;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(gbase + kBarOff + 8 * kBars);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   auto a_slot = [&](int s) { return base + (uint32_t)s * OTILE; };
-  const uint32_t b_bytes = (uint32_t)bn * (OBK * 2);  // a B digit tile
+  const uint32_t b_bytes = (uint32_t)bn * OBK;  // half a B digit tile (bn / 2 rows)
   auto b_slot = [&](int s) { return base + (uint32_t)ONA * OTILE + (uint32_t)s * b_bytes; };
   auto a_full = [&](int s) { return bars + 8u * s; };
   auto a_empty = [&](int s) { return bars + 8u * (ONA + s); };
@@ -231,7 +242,9 @@ k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
-  const int cid = (int)blockIdx.x, ncta = (int)gridDim.x;
+  // CTA pairs walk the tiles; the even CTA issues the pair's MMAs
+  const uint32_t rank = blockIdx.x & 1u;
+  const int cid = (int)blockIdx.x >> 1, ncta = (int)gridDim.x >> 1;
   const int ngr = level_groups(p.n_levels);
 
   if (threadIdx.x == 0) {
@@ -245,20 +258,20 @@ k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
     }
     for (int l = 0; l < OLEV; l++) {
       mbar_init(accf_bar(l), 1);
-      mbar_init(acce_bar(l), OEPI);
+      mbar_init(acce_bar(l), 2 * OEPI);  // both CTAs' epilogues (the even CTA's is used)
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
                  "r"(OTMEM_COLS)
                  : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  cluster_sync();  // both CTAs' barriers are there
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
@@ -270,68 +283,71 @@ k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
     while (gi + 1 < p.n_groups && t >= p.g[gi + 1].tile0) gi++;
     const OzakiGroup &g = p.g[gi];
     const int lt = t - g.tile0;
-    mrow = (lt / g.tiles_n) * OBM;
+    mrow = (lt / g.tiles_n) * (2 * OBM) + (int)rank * OBM;  // this CTA's rows
     n0 = (lt % g.tiles_n) * bn;
     kbt = g.kblocks;
     if (g.b_lower) kbt = min(kbt, (n0 + bn + OBK - 1) / OBK);
   };
 
-  if (warp == 0 && lane == 0) {
-    // ---------------- TMA producer ----------------
-    RingPos<ONA> ia;
-    RingPos<ONB> ib;
-    bool stop = false;
-    auto wait_slot = [&](uint32_t bar, uint32_t parity, int t) {
-      if (!mbar_wait(bar, parity)) {
-        set_status(p.status, FPP_ERR_TIMEOUT, 211, t);
-        *abort_flag = 1;
-      }
-      if (*abort_flag) stop = true;
-      return !stop;
-    };
-    for (int t = cid; t < p.n_tiles && !stop; t += ncta) {
-      int gi, mrow, n0, kbt;
-      locate(t, gi, mrow, n0, kbt);
-      const CUtensorMap *ma = &p.a[gi], *mb = &p.b[gi];
-      const int Mp = p.g[gi].Mp, Np = p.g[gi].Np, arow = p.g[gi].a_row0 + mrow;
-      const int brow = p.g[gi].b_row0 + n0;
-      for (int gr = 0; gr < ngr && !stop; gr++) {
-        const LevelGroup G(p.n_levels, gr);
-        for (int kb = 0; kb < kbt && !stop; kb++) {
-          int next = G.top();  // the next B digit to load
-          for (int s = 0; s < G.steps() && !stop; s++) {
-            {
-              const int st = ia.slot;
-              if (!wait_slot(a_empty(st), ia.parity ^ 1u, t)) break;
-              mbar_expect_tx(a_full(st), OTILE);
-              tma_load_2d(a_slot(st), ma, a_full(st), kb * OBK, s * Mp + arow);
-              ia.advance(1);
-            }
-            // the B digits first used at this step, largest first
-            for (; next >= G.lo(s) && !stop; next--) {
-              const int st = ib.slot;
-              if (!wait_slot(b_empty(st), ib.parity ^ 1u, t)) break;
-              mbar_expect_tx(b_full(st), b_bytes);
-              tma_load_2d(b_slot(st), mb, b_full(st), kb * OBK, next * Np + brow);
-              ib.advance(1);
-            }
+  if (warp == 0 || warp == OPROD_B) {
+    // ---------------- TMA producers: A digits, B digits ----------------
+    if (lane == 0) {
+      bool stop = false;
+      auto wait_slot = [&](uint32_t bar, uint32_t parity, int t) {
+        if (!mbar_wait(bar, parity)) {
+          set_status(p.status, FPP_ERR_TIMEOUT, 211, t);
+          *abort_flag = 1;
+        }
+        if (*abort_flag) stop = true;
+        return !stop;
+      };
+      auto walk = [&](auto pos, auto &&load) {  // load(next position, digit) of each K block
+        for (int t = cid; t < p.n_tiles && !stop; t += ncta) {
+          int gi, mrow, n0, kbt;
+          locate(t, gi, mrow, n0, kbt);
+          for (int gr = 0; gr < ngr && !stop; gr++) {
+            const LevelGroup G(p.n_levels, gr);
+            for (int kb = 0; kb < kbt && !stop; kb++)
+              for (int s = 0; s < G.steps() && !stop; s++) load(pos, t, gi, mrow, n0, kb, s, G);
           }
         }
+        return pos;
+      };
+      if (warp == 0) {
+        RingPos<ONA> ia = walk(RingPos<ONA>{}, [&](RingPos<ONA> &i, int t, int gi, int mrow, int,
+                                                   int kb, int s, const LevelGroup &) {
+          if (!wait_slot(a_empty(i.slot), i.parity ^ 1u, t)) return;
+          if (rank == 0) mbar_expect_tx(a_full(i.slot), 2 * OTILE);  // both CTAs' loads
+          tma_pair_load_2d(a_slot(i.slot), &p.a[gi], in_cta(a_full(i.slot), 0), kb * OBK,
+                           s * p.g[gi].Mp + p.g[gi].a_row0 + mrow);
+          i.advance(1);
+        });
+        // drain: every slot this CTA filled has been read before it exits
+        for (int d = 0; d < ONA && !*abort_flag; d++, ia.advance(1))
+          if (!mbar_wait(a_empty(ia.slot), ia.parity ^ 1u)) {
+            set_status(p.status, FPP_ERR_TIMEOUT, 215, d);
+            *abort_flag = 1;
+          }
+      } else {
+        // a group's steps use B digits top .. 0, largest first: digit top - s at turn s
+        RingPos<ONB> ib = walk(RingPos<ONB>{}, [&](RingPos<ONB> &i, int t, int gi, int, int n0,
+                                                   int kb, int s, const LevelGroup &G) {
+          if (!wait_slot(b_empty(i.slot), i.parity ^ 1u, t)) return;
+          if (rank == 0) mbar_expect_tx(b_full(i.slot), 2 * b_bytes);
+          tma_pair_load_2d(b_slot(i.slot), &p.b[gi], in_cta(b_full(i.slot), 0), kb * OBK,
+                           (G.top() - s) * p.g[gi].Np + p.g[gi].b_row0 + n0 +
+                               (int)rank * (bn / 2));
+          i.advance(1);
+        });
+        for (int d = 0; d < ONB && !*abort_flag; d++, ib.advance(1))
+          if (!mbar_wait(b_empty(ib.slot), ib.parity ^ 1u)) {
+            set_status(p.status, FPP_ERR_TIMEOUT, 216, d);
+            *abort_flag = 1;
+          }
       }
     }
-    // drain: every slot this CTA filled has been read before it exits
-    for (int d = 0; d < ONA && !*abort_flag; d++, ia.advance(1))
-      if (!mbar_wait(a_empty(ia.slot), ia.parity ^ 1u)) {
-        set_status(p.status, FPP_ERR_TIMEOUT, 215, d);
-        *abort_flag = 1;
-      }
-    for (int d = 0; d < ONB && !*abort_flag; d++, ib.advance(1))
-      if (!mbar_wait(b_empty(ib.slot), ib.parity ^ 1u)) {
-        set_status(p.status, FPP_ERR_TIMEOUT, 216, d);
-        *abort_flag = 1;
-      }
-  } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
+  } else if (warp == 1 && rank == 0) {
+    // ---------------- MMA issuer (the even CTA's) ----------------
     // ib: slot of the K block's first B digit; unit: uses of accumulator 0, of
     // the others (a group of one level leaves them out).  Everything but the
     // waits is unrolled per group of levels: with the slots and levels worked
@@ -351,14 +367,19 @@ k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
     };
     auto k_block = [&](auto lc, bool chunk_first, bool chunk_last, int t) {
       constexpr LevelGroup G = decltype(lc)::value();
-#pragma unroll
-      for (int s = 0; s < G.steps(); s++) {
-        wait_or_abort(a_full(ia.slot), ia.parity, 213, t);
+      // the A digit and the B digits first used at step s
+      auto wait_step = [&](int s, RingPos<ONA> qa) {
+        wait_or_abort(a_full(qa.slot), qa.parity, 213, t);
 #pragma unroll
         for (int d = s == 0 ? G.top() : G.lo(s - 1) - 1; d >= G.lo(s); d--) {
           const RingPos<ONB> q = ib.ahead(G.top() - d);
           wait_or_abort(b_full(q.slot), q.parity, 213, t);
         }
+      };
+      wait_step(0, ia);
+      if (__any_sync(0xffffffffu, *abort_flag)) return false;
+#pragma unroll
+      for (int s = 0; s < G.steps(); s++) {
         const bool fresh = chunk_first && s <= G.first_step(G.L1);
         if (fresh) {
           // the accumulators of the levels that start at this step
@@ -368,56 +389,37 @@ k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
               wait_or_abort(acce_bar(L - G.L0),
                             (uint32_t)((L == G.L0 ? unit : unit_rest) & 1) ^ 1u, 212, t);
         }
-        if (__any_sync(0xffffffffu, *abort_flag)) return false;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t pa = da0 + (uint64_t)(ia.slot * (OTILE >> 4));
-        // Partners two by two: B digits d and d - 1 in neighboring slots are one
-        // 256-row operand and their levels' accumulators neighboring columns, so
-        // one N = 256 MMA forms both pairs.
 #pragma unroll
-        for (int j = 0; j < OLEV; j += 2) {
+        for (int j = 0; j < OLEV; j++) {
           const int d = G.hi(s) - j;
           if (d < G.lo(s)) continue;
-          const RingPos<ONB> q0 = ib.ahead(G.top() - d);
-          const uint64_t pb = db0 + (uint64_t)(q0.slot * b_step);
+          const uint64_t pb = db0 + (uint64_t)(ib.ahead(G.top() - d).slot * b_step);
           const uint32_t acc = tmem + (uint32_t)acc_col(s + d - G.L0, bn);
-          const bool new0 = s == G.first_step(s + d), new1 = s == G.first_step(s + d - 1);
-          const uint32_t add0 = new0 && chunk_first ? 0u : 1u;
-          const uint32_t add1 = new1 && chunk_first ? 0u : 1u;
-          const bool two = d - 1 >= G.lo(s);
-          if (two && add0 == add1 && q0.slot + 1 < ONB) {
-            if (elect_one()) {
+          const uint32_t add = s == G.first_step(s + d) && chunk_first ? 0u : 1u;
+          if (elect_one()) {
 #pragma unroll
-              for (int ks = 0; ks < OBK / 16; ks++)
-                mma_f16_n(acc, pa + ks * 2, pb + ks * 2, 2 * bn, ks == 0 ? add0 : 1u);
-            }
-          } else {
-            const uint64_t pb1 = db0 + (uint64_t)(q0.ahead(1).slot * b_step);
-            if (elect_one()) {
-#pragma unroll
-              for (int ks = 0; ks < OBK / 16; ks++)
-                mma_f16_n(acc, pa + ks * 2, pb + ks * 2, bn, ks == 0 ? add0 : 1u);
-              if (two) {
-#pragma unroll
-                for (int ks = 0; ks < OBK / 16; ks++)
-                  mma_f16_n(acc + bn, pa + ks * 2, pb1 + ks * 2, bn, ks == 0 ? add1 : 1u);
-              }
-            }
+            for (int ks = 0; ks < OBK / 16; ks++)
+              mma_pair_f16(acc, pa + ks * 2, pb + ks * 2, bn, ks == 0 ? add : 1u);
           }
+          // the next step's operands, while these MMAs run: a wait costs more than
+          // the few MMAs that queue behind each other take
+          if (j == 0 && s + 1 < G.steps()) wait_step(s + 1, ia.ahead(1));
         }
         // free the slots once these MMAs read them: the A digit, and the B
         // digits without a later partner
         if (elect_one()) {
-          mma_commit(a_empty(ia.slot));
+          mma_pair_commit(a_empty(ia.slot));
 #pragma unroll
           for (int d = G.top(); d >= 0; d--) {
             const int last = G.L1 - d < G.steps() ? G.L1 - d : G.steps() - 1;
-            if (s == last) mma_commit(b_empty(ib.ahead(G.top() - d).slot));
+            if (s == last) mma_pair_commit(b_empty(ib.ahead(G.top() - d).slot));
           }
           if (chunk_last) {
 #pragma unroll
             for (int L = G.L0; L <= G.L1; L++)
-              if (s == G.last_step(L)) mma_commit(accf_bar(L - G.L0));
+              if (s == G.last_step(L)) mma_pair_commit(accf_bar(L - G.L0));
           }
         }
         __syncwarp();
@@ -451,9 +453,9 @@ k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
     }
     if (__any_sync(0xffffffffu, *abort_flag)) {  // release the epilogue
       if (elect_one())
-        for (int l = 0; l < OLEV; l++) mma_commit(accf_bar(l));
+        for (int l = 0; l < OLEV; l++) mma_pair_commit(accf_bar(l));
     }
-  } else if (warp >= 2) {
+  } else if (warp != 1) {
     // ---------------- epilogue ----------------
     const int q = warp & 3;                 // TMEM lane quarter this warp may access
     const int colh = (warp - 2) / 4;        // which OCOLS columns of the tile
@@ -502,7 +504,7 @@ k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(acce_bar(l));
+            if (lane == 0) mbar_arrive_cluster(in_cta(acce_bar(l), 0));
           }
         }
         if (stop) break;
@@ -552,9 +554,9 @@ k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  cluster_sync();  // the peer no longer reads, writes or signals this CTA's memory
   if (warp == 2) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(OTMEM_COLS)
                  : "memory");
   }
@@ -594,7 +596,7 @@ k_ozaki_split(int rows, int K, long long ldx, const double *__restrict__ X,
   if (lane == 0) exps[r] = e;
 }
 
-static int ozaki_launch_shape(int dev, int *ctas) {
+static int ozaki_launch_shape(int dev, int *pairs) {
   constexpr int kMaxDev = 64;
   static std::mutex mu;
   static int cached[kMaxDev] = {0};
@@ -604,15 +606,23 @@ static int ozaki_launch_shape(int dev, int *ctas) {
     if (cudaFuncSetAttribute(k_ozaki_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              OSMEM_BYTES) != cudaSuccess)
       return -1;
-    int sms = 0, per_sm = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ozaki_gemm, OTHREADS,
-                                                      OSMEM_BYTES) != cudaSuccess)
-      return -1;
-    if (per_sm < 1) return -1;
-    cached[dev] = sms * per_sm;
+    // resident CTA pairs (an SM without a partner in its cluster group stays idle)
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(2, 1, 1);
+    cfg.blockDim = dim3(OTHREADS, 1, 1);
+    cfg.dynamicSmemBytes = OSMEM_BYTES;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 2;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_ozaki_gemm, &cfg) != cudaSuccess || n < 1) return -1;
+    cached[dev] = n;
   }
-  *ctas = cached[dev];
+  *pairs = cached[dev];
   return 0;
 }
 
@@ -637,20 +647,20 @@ int launch_ozaki_split(int rows, int K, const double *X, long long ldx, __half *
 }
 
 // Columns of a tile for all products of a launch (the rings' slots are sized by
-// them): the cheapest count of rounds of tiles over the SMs, a tile costing about
+// them): the cheapest count of rounds of tiles over the CTA pairs, a tile costing about
 // bn + 300 (its A digits are read and its sums drained whatever bn is).  Narrower tiles
-// pay where they add no round: 16384 x 150 x 544 with two tiles of 80 columns instead
-// of 128 takes 199 us instead of 227, 1000 x 1050 x 1050 with 136 tiles of 64 instead of
-// 72 of 128 takes 154 instead of 170.
-static int tile_columns(const OzakiProblem *probs, int n, int ctas) {
+// pay where they add no round: 16384 x 150 x 544 with two tiles of 96 columns instead
+// of 128 takes 160 us instead of 176, 1000 x 1050 x 1050 with 68 tiles of 64 instead of
+// 36 of 128 takes 117 instead of 141.
+static int tile_columns(const OzakiProblem *probs, int n, int pairs) {
   int best = OBN;
   long long cost = 0;
-  for (int bn : {OBN, 96, 80, 64}) {
+  for (int bn : {OBN, 96, 64}) {
     long long tiles = 0;
     for (int k = 0; k < n; k++)
       if (probs[k].M > 0 && probs[k].N > 0)
-        tiles += (long long)ceil_div(probs[k].M, OBM) * ceil_div(probs[k].N, bn);
-    const long long c = (tiles + ctas - 1) / ctas * (bn + 300);
+        tiles += (long long)ceil_div(probs[k].M, 2 * OBM) * ceil_div(probs[k].N, bn);
+    const long long c = (tiles + pairs - 1) / pairs * (bn + 300);
     if (bn == OBN || c < cost) {
       best = bn;
       cost = c;
@@ -662,11 +672,11 @@ static int tile_columns(const OzakiProblem *probs, int n, int ctas) {
 int launch_ozaki_gemm(const OzakiProblem *probs, int n_probs, DeviceStatus *status,
                       cudaStream_t stream, int n_levels) {
   if (n_probs > kOzakiMaxGroups || (n_levels != 8 && n_levels != 9)) return -2;
-  int dev = 0, ctas = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || ozaki_launch_shape(dev, &ctas) != 0) return -1;
+  int dev = 0, pairs = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || ozaki_launch_shape(dev, &pairs) != 0) return -1;
   OzakiParams p;
   std::memset(&p, 0, sizeof(p));
-  p.bn = tile_columns(probs, n_probs, ctas);
+  p.bn = tile_columns(probs, n_probs, pairs);
   int tiles = 0;
   for (int k = 0; k < n_probs; k++) {
     const OzakiProblem &q = probs[k];
@@ -679,7 +689,7 @@ int launch_ozaki_gemm(const OzakiProblem *probs, int n_probs, DeviceStatus *stat
     const int i = p.n_groups++;
     // one map over all digit planes of an operand: rows s * rows_pad + row
     if (make_map(&p.a[i], q.a.planes, sa.k_pad, sa.rows_pad * kOzakiDigits, sa.k_pad, OBM) ||
-        make_map(&p.b[i], q.b.planes, sb.k_pad, sb.rows_pad * kOzakiDigits, sb.k_pad, p.bn))
+        make_map(&p.b[i], q.b.planes, sb.k_pad, sb.rows_pad * kOzakiDigits, sb.k_pad, p.bn / 2))
       return -3;
     OzakiGroup &g = p.g[i];
     g.M = q.M;
@@ -696,7 +706,7 @@ int launch_ozaki_gemm(const OzakiProblem *probs, int n_probs, DeviceStatus *stat
     g.eb = q.b.exps + q.b_row0;
     g.C = q.C;
     g.ldc = q.ldc;
-    tiles += ceil_div(q.M, OBM) * g.tiles_n;
+    tiles += ceil_div(q.M, 2 * OBM) * g.tiles_n;
   }
   if (tiles == 0) return 0;
   p.n_tiles = tiles;
@@ -707,7 +717,7 @@ int launch_ozaki_gemm(const OzakiProblem *probs, int n_probs, DeviceStatus *stat
   cfg.blockDim = dim3(OTHREADS, 1, 1);
   cfg.dynamicSmemBytes = OSMEM_BYTES;
   cfg.stream = stream;
-  cfg.gridDim = dim3(tiles < ctas ? tiles : ctas, 1, 1);
+  cfg.gridDim = dim3(2 * (tiles < pairs ? tiles : pairs), 1, 1);
   if (cudaLaunchKernelEx(&cfg, k_ozaki_gemm, p) != cudaSuccess) return -1;
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

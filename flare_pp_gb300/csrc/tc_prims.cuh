@@ -106,16 +106,6 @@ __host__ __device__ constexpr uint32_t idesc_f16() {
          ((uint32_t)(128 >> 4) << 24);
 }
 
-// The same with the columns N known at run time (a multiple of 16, at most 256).
-__device__ __forceinline__ void mma_f16_n(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t n,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(idesc_f16<0>() | ((n >> 3) << 17)), "r"(accumulate));
-}
-
 template <int NN>
 __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t a, uint64_t b,
                                         uint32_t accumulate) {
@@ -124,6 +114,59 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t a, uint64_t b,
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
       "l"(a), "l"(b), "r"(idesc_f16<NN>()), "r"(accumulate));
+}
+
+// ---- CTA pairs (clusters of two): one MMA over both SMs ----
+// A 256-row tile: each CTA of the pair holds its 128 rows of A, half the columns' rows of
+// B (at the same shared-memory offsets) and its 128 rows of the accumulator; the even CTA
+// issues.
+
+// n columns (a multiple of 32, at most 256); descriptors as for one CTA.
+__device__ __forceinline__ void mma_pair_f16(uint32_t tmem_d, uint64_t a, uint64_t b,
+                                             uint32_t n, uint32_t accumulate) {
+  const uint32_t idesc = (1u << 4) | ((n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
+}
+
+// Arrives on the barrier at this offset in both CTAs when the pair's MMAs are done.
+__device__ __forceinline__ void mma_pair_commit(uint32_t bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
+      " [%0], %1;" ::"r"(bar), "h"((uint16_t)3)
+      : "memory");
+}
+
+// The address of a shared-memory location in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+
+// A tile into this CTA's shared memory, its bytes counted on a barrier (a cluster
+// address) of either CTA of the pair.
+__device__ __forceinline__ void tma_pair_load_2d(uint32_t dst, const CUtensorMap *map,
+                                                 uint32_t bar, int c0, int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+
+// Arrives on a barrier of any CTA of the cluster (a cluster address).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // One lane of a converged warp (always the same one).  The compiler issues the
