@@ -11,15 +11,22 @@
 // The cross terms have their own accumulator: added into the leading one they
 // would each round against its magnitude (measured: 1.6x the force error).
 //
-// One persistent CTA per SM walks the 128 x 128 tiles of all species blocks
-// (each block of P rows against its own B), in one launch; every CTA loads
-// all four operand planes of its own tile (no clusters):
-//   warp 0 lane 0  TMA producer: 128B-swizzled K-major tiles of P_hi, P_lo,
-//                  B_hi, B_lo (64 K-columns per stage) into a 3-stage ring
-//   warp 1 lane 0  MMA issuer: 4 K=16 steps x 3 tcgen05.mma per stage,
-//                  tcgen05.commit frees the stage; the two accumulator pairs
-//                  (2 x 2 x 128 TMEM columns) alternate between tiles, so the
-//                  epilogue of one tile overlaps the MMAs of the next
+// One persistent CTA per SM, in pairs (clusters of two, cta_group::2), walks the 256 x 128
+// tiles of all species blocks (each block of P rows against its own B), in one launch.
+// Shared memory bounds it (operand reads and TMA writes against 128 bytes per cycle and
+// SM): in a pair each SM reads its 128 rows of P and half of the columns' rows of B, and
+// half of B is loaded; four stages fit instead of three.  32,768 atoms, 1500 columns:
+// 284 us with a CTA's own 128 x 128 tiles, 240 so.  (Waiting for the next stage behind
+// the first MMAs of one, which pays in gemm_ozaki.cu, costs a tenth here: the stage is
+// not there yet, and the MMAs after the wait are late.)
+//   warp 0 lane 0  TMA producer: 128B-swizzled K-major tiles of P_hi, P_lo (128 rows),
+//                  B_hi, B_lo (64 rows; 64 K-columns per stage) into a 4-stage ring, the
+//                  pair's loads counted on the even CTA's barriers
+//   warp 1         MMA issuer (the even CTA's, one elected lane): 4 K=16 steps x 3
+//                  tcgen05.mma per stage, tcgen05.commit frees the stage in both CTAs;
+//                  the two accumulator pairs (2 x 2 x 128 TMEM columns) alternate
+//                  between tiles, so the epilogue of one tile overlaps the MMAs of the
+//                  next
 //   warps 2-5      epilogue: tcgen05.ld of their 32 TMEM lanes, combine,
 //                  scale, store FP32 rows of V, then release the accumulators
 // Every mbarrier wait is bounded; a wait that runs out records
@@ -40,10 +47,10 @@
 
 namespace fpp {
 
-constexpr int BM = 128, BN = 128, BK = 64, STAGES = 3;
+constexpr int BM = 128, BN = 128, BK = 64, STAGES = 4;
 static_assert(BK == kTmaBoxK, "the tensor maps load 64-column boxes");
 constexpr int A_TILE = BM * BK * 2;  // bytes, one fp16 operand tile
-constexpr int B_TILE = BN * BK * 2;
+constexpr int B_TILE = BN / 2 * BK * 2;  // a CTA's half of the columns
 constexpr int STAGE_BYTES = 2 * A_TILE + 2 * B_TILE;
 constexpr int TMEM_COLS = 512;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
@@ -64,7 +71,7 @@ struct GroupedParams {
 };
 
 
-__global__ void __launch_bounds__(192, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
 k_split_gemm_grouped(const __grid_constant__ GroupedParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -79,10 +86,13 @@ k_split_gemm_grouped(const __grid_constant__ GroupedParams p) {
   auto accf_bar = [&](int b) { return bars + 8u * (2 * STAGES + b); };
   auto acce_bar = [&](int b) { return bars + 8u * (2 * STAGES + 2 + b); };
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
   const int n_tiles = p.tile_start[p.n_groups];
   const int kblocks = (p.K + BK - 1) / BK;
-  const int cid = (int)blockIdx.x, ncl = (int)gridDim.x;
+  // CTA pairs walk the tiles; the even CTA issues the pair's MMAs
+  const uint32_t rank = blockIdx.x & 1u;
+  const int cid = (int)blockIdx.x >> 1, ncl = (int)gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) {
@@ -91,20 +101,20 @@ k_split_gemm_grouped(const __grid_constant__ GroupedParams p) {
     }
     for (int b = 0; b < 2; b++) {
       mbar_init(accf_bar(b), 1);
-      mbar_init(acce_bar(b), 4);
+      mbar_init(acce_bar(b), 8);  // both CTAs' epilogues (the even CTA's is used)
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
                  "r"(TMEM_COLS)
                  : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  cluster_sync();  // both CTAs' barriers are there
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
@@ -115,7 +125,7 @@ k_split_gemm_grouped(const __grid_constant__ GroupedParams p) {
     g = 0;
     while (g + 1 < p.n_groups && t >= p.tile_start[g + 1]) g++;
     const int lt = t - p.tile_start[g];
-    mrow = (lt / p.tiles_n) * BM;
+    mrow = (lt / p.tiles_n) * (2 * BM) + (int)rank * BM;  // this CTA's rows
     n0 = (lt % p.tiles_n) * BN;
   };
 
@@ -136,12 +146,13 @@ k_split_gemm_grouped(const __grid_constant__ GroupedParams p) {
         }
         if (*abort_flag) break;
         const uint32_t st = base + s * STAGE_BYTES;
-        mbar_expect_tx(full_bar(s), STAGE_BYTES);
-        const int kc = kb * BK;
-        tma_load_2d(st, &p.a_hi, full_bar(s), kc, arow);
-        tma_load_2d(st + A_TILE, &p.a_lo, full_bar(s), kc, arow);
-        tma_load_2d(st + 2 * A_TILE, &p.b_hi[g], full_bar(s), kc, n0);
-        tma_load_2d(st + 2 * A_TILE + B_TILE, &p.b_lo[g], full_bar(s), kc, n0);
+        if (rank == 0) mbar_expect_tx(full_bar(s), 2 * STAGE_BYTES);  // both CTAs' loads
+        const uint32_t bar = in_cta(full_bar(s), 0);
+        const int kc = kb * BK, brow = n0 + (int)rank * (BN / 2);
+        tma_pair_load_2d(st, &p.a_hi, bar, kc, arow);
+        tma_pair_load_2d(st + 2 * A_TILE, &p.b_hi[g], bar, kc, brow);
+        tma_pair_load_2d(st + 2 * A_TILE + B_TILE, &p.b_lo[g], bar, kc, brow);
+        tma_pair_load_2d(st + A_TILE, &p.a_lo, bar, kc, arow);
       }
     }
     // drain: every stage this CTA filled has been read (no MMA completion
@@ -152,51 +163,45 @@ k_split_gemm_grouped(const __grid_constant__ GroupedParams p) {
         *abort_flag = 1;
       }
     }
-  } else if (warp == 1 && lane == 0) {
-    // ---------------- MMA issuer ----------------
+  } else if (warp == 1 && rank == 0) {
+    // ---------------- MMA issuer (the even CTA's, one elected lane) ----------------
     int it = 0, j = 0;
-    for (int t = cid; t < n_tiles; t += ncl, j++) {
-      const int buf = j & 1;
-      const uint32_t acc0 = tmem + (uint32_t)(buf * 2 * BN), acc1 = acc0 + BN;
-      if (!mbar_wait(acce_bar(buf), (uint32_t)(((j >> 1) & 1) ^ 1))) {
-        set_status(p.status, FPP_ERR_TIMEOUT, 112, t);
+    bool stop = false;
+    auto wait_or_abort = [&](uint32_t bar, uint32_t parity, int site, int t) {
+      if (!mbar_wait(bar, parity)) {
+        if (lane == 0) set_status(p.status, FPP_ERR_TIMEOUT, site, t);
         *abort_flag = 1;
       }
-      if (*abort_flag) {
-        mma_commit(accf_bar(buf));  // release the epilogue of this buffer
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      bool ok = true;
+    };
+    for (int t = cid; t < n_tiles && !stop; t += ncl, j++) {
+      const int buf = j & 1;
+      const uint32_t acc0 = tmem + (uint32_t)(buf * 2 * BN), acc1 = acc0 + BN;
+      wait_or_abort(acce_bar(buf), (uint32_t)(((j >> 1) & 1) ^ 1), 112, t);
       for (int kb = 0; kb < kblocks; kb++, it++) {
         const int s = it % STAGES;
-        const uint32_t ph = (uint32_t)((it / STAGES) & 1);
-        if (!mbar_wait(full_bar(s), ph)) {
-          set_status(p.status, FPP_ERR_TIMEOUT, 113, t);
-          *abort_flag = 1;
-          ok = false;
-          break;
-        }
+        wait_or_abort(full_bar(s), (uint32_t)((it / STAGES) & 1), 113, t);
+        stop = __any_sync(0xffffffffu, *abort_flag) != 0;
+        if (stop) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t st = base + s * STAGE_BYTES;
-        const uint32_t a_hi = st, a_lo = st + A_TILE;
-        const uint32_t b_hi = st + 2 * A_TILE;  // B_lo follows at + B_TILE
+        const uint64_t a_hi = smem_desc(st), a_lo = smem_desc(st + A_TILE);
+        const uint64_t b_hi = smem_desc(st + 2 * A_TILE);
+        const uint64_t b_lo = smem_desc(st + 2 * A_TILE + B_TILE);
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < BK / 16; ks++) {
-          const uint32_t off = ks * 32;
-          const uint32_t first = (kb > 0 || ks > 0) ? 1u : 0u;
-          // B_hi and B_lo are one 256-row operand in shared memory and acc0,
-          // acc1 adjacent TMEM columns: [acc0 | acc1] = A_hi [B_hi ; B_lo]^T
-          // in one N = 256 MMA, then acc1 += A_lo B_hi^T.  Shared-memory
-          // reads per K step fall from 24 KB to 20 KB (the operand reads and
-          // the TMA writes share the SM's shared-memory bandwidth).
-          mma_f16<2 * BN>(acc0, smem_desc(a_hi + off), smem_desc(b_hi + off), first);
-          mma_f16<BN>(acc1, smem_desc(a_lo + off), smem_desc(b_hi + off), 1u);
+          for (int ks = 0; ks < BK / 16; ks++) {
+            const uint32_t add = (kb > 0 || ks > 0) ? 1u : 0u;
+            // acc0 = A_hi B_hi^T, acc1 = A_hi B_lo^T + A_lo B_hi^T
+            mma_pair_f16(acc0, a_hi + ks * 2, b_hi + ks * 2, BN, add);
+            mma_pair_f16(acc1, a_hi + ks * 2, b_lo + ks * 2, BN, add);
+            mma_pair_f16(acc1, a_lo + ks * 2, b_hi + ks * 2, BN, 1u);
+          }
+          mma_pair_commit(empty_bar(s));  // frees the stage once these MMAs have read it
         }
-        mma_commit(empty_bar(s));  // frees the stage once these MMAs have read it
+        __syncwarp();
       }
-      mma_commit(accf_bar(buf));
-      if (!ok) break;
+      if (elect_one()) mma_pair_commit(accf_bar(buf));  // (after an abort: frees the epilogue)
+      __syncwarp();
     }
   } else if (warp >= 2) {
     // ---------------- epilogue ----------------
@@ -248,13 +253,13 @@ k_split_gemm_grouped(const __grid_constant__ GroupedParams p) {
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive(acce_bar(buf));
+      if (lane == 0) mbar_arrive_cluster(in_cta(acce_bar(buf), 0));
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  cluster_sync();  // the peer no longer reads, writes or signals this CTA's memory
   if (warp == 2) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"(TMEM_COLS)
                  : "memory");
   }
@@ -268,7 +273,7 @@ int split_gemm_smem_bytes() { return SMEM_BYTES; }
 // The shared-memory attribute and the resident CTA count are properties of a
 // device: set and measured once per device, under a lock (host threads may
 // launch on several devices).
-static int launch_shape(int dev, int *ctas) {
+static int launch_shape(int dev, int *pairs) {
   constexpr int kMaxDev = 64;
   static std::mutex mu;
   static int cached[kMaxDev] = {0};
@@ -279,15 +284,24 @@ static int launch_shape(int dev, int *ctas) {
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              SMEM_BYTES) != cudaSuccess)
       return -1;
-    int sms = 0, per_sm = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_split_gemm_grouped, 192,
-                                                      SMEM_BYTES) != cudaSuccess)
+    // resident CTA pairs
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(2, 1, 1);
+    cfg.blockDim = dim3(192, 1, 1);
+    cfg.dynamicSmemBytes = SMEM_BYTES;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = 2;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_split_gemm_grouped, &cfg) != cudaSuccess || n < 1)
       return -1;
-    if (per_sm < 1) return -1;
-    cached[dev] = sms * per_sm;
+    cached[dev] = n;
   }
-  *ctas = cached[dev];
+  *pairs = cached[dev];
   return 0;
 }
 
@@ -309,14 +323,14 @@ int launch_split_gemm_grouped(const GroupedGemmArgs &g, cudaStream_t stream) {
     if ((q.ldb * 2) % 16 != 0 || ((uintptr_t)q.b_hi | (uintptr_t)q.b_lo) % 16 != 0 ||
         g.K > q.ldb)
       return -2;
-    if (make_map(&p.b_hi[k], q.b_hi, g.K, q.b_rows, q.ldb, BN) ||
-        make_map(&p.b_lo[k], q.b_lo, g.K, q.b_rows, q.ldb, BN))
+    if (make_map(&p.b_hi[k], q.b_hi, g.K, q.b_rows, q.ldb, BN / 2) ||
+        make_map(&p.b_lo[k], q.b_lo, g.K, q.b_rows, q.ldb, BN / 2))
       return -3;
     p.row0[k] = q.row0;
     p.M[k] = q.M;
     p.scale[k] = q.out_scale;
     p.tile_start[k] = tiles;
-    tiles += ((q.M + BM - 1) / BM) * tiles_n;
+    tiles += ((q.M + 2 * BM - 1) / (2 * BM)) * tiles_n;
   }
   p.tile_start[g.n_groups] = tiles;
   p.n_groups = g.n_groups;
@@ -329,15 +343,15 @@ int launch_split_gemm_grouped(const GroupedGemmArgs &g, cudaStream_t stream) {
   if (tiles == 0) return 0;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return -1;
-  int ctas = 0;
-  if (launch_shape(dev, &ctas) != 0) return -1;
+  int pairs = 0;
+  if (launch_shape(dev, &pairs) != 0) return -1;
   // one persistent CTA per SM (the shared-memory ring admits one per SM)
   cudaLaunchConfig_t cfg;
   std::memset(&cfg, 0, sizeof(cfg));
   cfg.blockDim = dim3(192, 1, 1);
   cfg.dynamicSmemBytes = SMEM_BYTES;
   cfg.stream = stream;
-  cfg.gridDim = dim3(tiles < ctas ? tiles : ctas, 1, 1);
+  cfg.gridDim = dim3(2 * (tiles < pairs ? tiles : pairs), 1, 1);
   if (cudaLaunchKernelEx(&cfg, k_split_gemm_grouped, p) != cudaSuccess) return -1;
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -1,8 +1,8 @@
 // Device and host primitives shared by the tcgen05 GEMMs of this library
 // (gemm_tc.cu, gemm_ozaki.cu): mbarriers with bounded waits, 2D TMA loads of
 // 128B-swizzled K-major fp16 tiles, shared-memory and instruction
-// descriptors for tcgen05.mma kind::f16 with M = 128, the MMA commit, TMEM
-// loads, and the tensor-map encoder.
+// descriptors for tcgen05.mma kind::f16 over a CTA pair (M = 256), the MMA
+// commit, TMEM loads, and the tensor-map encoder.
 #pragma once
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -77,15 +77,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   }
 }
 
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map,
-                                            uint32_t bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
-      : "memory");
-}
-
 // Shared-memory matrix descriptor: K-major operand, 128B swizzle, 8-row core
 // groups 1024 B apart.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
@@ -98,30 +89,12 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
   return d;
 }
 
-// Instruction descriptor: kind::f16 with fp16 A and B, FP32 accumulate,
-// K-major A and B, M = 128, N = NN.
-template <int NN>
-__host__ __device__ constexpr uint32_t idesc_f16() {
-  return (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(NN >> 3) << 17) |
-         ((uint32_t)(128 >> 4) << 24);
-}
-
-template <int NN>
-__device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t a, uint64_t b,
-                                        uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(idesc_f16<NN>()), "r"(accumulate));
-}
-
 // ---- CTA pairs (clusters of two): one MMA over both SMs ----
 // A 256-row tile: each CTA of the pair holds its 128 rows of A, half the columns' rows of
 // B (at the same shared-memory offsets) and its 128 rows of the accumulator; the even CTA
 // issues.
 
-// n columns (a multiple of 32, at most 256); descriptors as for one CTA.
+// fp16 A and B, FP32 accumulate, K-major, n columns (a multiple of 32, at most 256).
 __device__ __forceinline__ void mma_pair_f16(uint32_t tmem_d, uint64_t a, uint64_t b,
                                              uint32_t n, uint32_t accumulate) {
   const uint32_t idesc = (1u << 4) | ((n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
@@ -182,12 +155,6 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-      : "memory");
-}
-
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
   uint32_t r[32];
   asm volatile(
@@ -218,10 +185,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 // The tensor-map encoder is a driver entry point; it is resolved through the
