@@ -222,15 +222,15 @@ __host__ __device__ inline FwdLayout<T> fwd_layout(const B2Args &a) {
 //    rounds per neighbor with a lane per (l, m) column: half the lanes idle at lmax 3);
 //  - the first chunk of 16 of a species is its sum, later ones are Kahan-folded.
 // The sums themselves run as before: neighbors in order, chunks of 16.
-// 4,394 atoms with a skin, N = 8, lmax = 3: 446 us before, 233 so; 8,192 atoms, N = 12,
-// lmax = 4: 899 and 623.
+// 4,394 atoms with a skin, N = 8, lmax = 3: 446 us before, 161 so; 8,192 atoms, N = 12,
+// lmax = 4: 899 and 619.
 template <typename SH>
 __device__ __forceinline__ void forward64_sums(const B2Args &a, int si, int beg, int end,
                                                const dvec4 *__restrict__ rel,
                                                const int *__restrict__ nbr_s, double *g_s,
                                                double *y_s, double *c_s, double *cc_s,
                                                int *list, int lane) {
-  constexpr int kSums = SH::kL1 == 5 ? 10 : 8;  // sums per lane and pass
+  constexpr int kSums = SH::kL1 == 5 ? 10 : 8;  // most sums per lane and pass
   const int N = SH::N(a), LMAX = SH::lmax(a), H = (LMAX + 1) * (LMAX + 1), NS = SH::NS(a);
   const int W = a.window, GP = (N + 3) & ~3, WS = W + 1, HP = (H + 3) & ~3;
   int *cnt_s = list + NS * W, *queue = cnt_s + NS;  // [NS], [2 W]
@@ -286,29 +286,30 @@ __device__ __forceinline__ void forward64_sums(const B2Args &a, int si, int beg,
       const int *ls = list + sp * W;
       const bool first = !((seen >> sp) & 1ull);
       seen |= 1ull << sp;
-      for (int o0 = 0; o0 < N * H; o0 += 32 * kSums) {
-        int yo[kSums], go[kSums], co[kSums];  // this lane's sums: (n, lm) of o0 + 32 j + lane
+      // one pass over the neighbors for J sums per lane, from o0 on
+      auto pass = [&](auto jc, int o0) {
+        constexpr int J = decltype(jc)::value;
+        int yo[J], go[J], co[J];  // this lane's sums: (n, lm) of o0 + 32 j + lane
 #pragma unroll
-        for (int j = 0; j < kSums; j++) {
+        for (int j = 0; j < J; j++) {
           const int o = min(o0 + 32 * j + lane, N * H - 1), n = o / H, lm = o - n * H;
           yo[j] = lm * WS;
           go[j] = n;
           co[j] = (sp * N + n) * HP + lm;
         }
         for (int k0 = 0; k0 < ns_; k0 += 16) {
-          double chunk[kSums];
+          double chunk[J];
 #pragma unroll
-          for (int j = 0; j < kSums; j++) chunk[j] = 0.0;
+          for (int j = 0; j < J; j++) chunk[j] = 0.0;
           const int k1 = min(ns_, k0 + 16);
           for (int k = k0; k < k1; k++) {
             const int b = ls[k];
             const double *yb = y_s + b, *gb = g_s + b * GP;
 #pragma unroll
-            for (int j = 0; j < kSums; j++)
-              if (o0 + 32 * j < N * H) chunk[j] = fma(gb[go[j]], yb[yo[j]], chunk[j]);
+            for (int j = 0; j < J; j++) chunk[j] = fma(gb[go[j]], yb[yo[j]], chunk[j]);
           }
 #pragma unroll
-          for (int j = 0; j < kSums; j++)
+          for (int j = 0; j < J; j++)
             if (o0 + 32 * j + lane < N * H) {
               if (first && k0 == 0) {
                 c_s[co[j]] = chunk[j];
@@ -321,6 +322,27 @@ __device__ __forceinline__ void forward64_sums(const B2Args &a, int si, int beg,
                 c_s[co[j]] = t;
               }
             }
+        }
+      };
+      // as few sums past N H as the widths allow: predicated off, their FP64
+      // instructions would cost as much as the others
+      for (int o0 = 0; o0 < N * H;) {
+        const int left = (N * H - o0 + 31) / 32;
+        if (left <= 2) {
+          pass(std::integral_constant<int, 2>{}, o0);
+          o0 += 64;
+        } else if (left <= 4) {
+          pass(std::integral_constant<int, 4>{}, o0);
+          o0 += 128;
+        } else if (left <= 6) {
+          pass(std::integral_constant<int, 6>{}, o0);
+          o0 += 192;
+        } else if (left <= 8 || kSums == 8) {
+          pass(std::integral_constant<int, 8>{}, o0);
+          o0 += 256;
+        } else {
+          pass(std::integral_constant<int, kSums>{}, o0);
+          o0 += 32 * kSums;
         }
       }
     }

@@ -17,8 +17,8 @@
 // SM); here the work per (pair, environment) on that pipe is fifteen adds of the
 // gather, and the contraction runs at the tensor cores' FP64-equivalent rate.  32 cells of
 // 8,460 atoms (354,000 pairs), N = 8, lmax = 3, two species of 150 environments each:
-// 76.7 ms by the adjoint; here 12.1 ms: GEMM 4.7, rows 3.6, descriptors 1.7, gather 1.4.
-// One cell of 256 atoms (envs_struc; stored derivatives before): 0.56 ms instead of 1.8.
+// 76.7 ms by the adjoint; here 10.4 ms: GEMM 3.8, rows 3.6, descriptors 0.9, gather 1.4.
+// One cell of 256 atoms (envs_struc; stored derivatives before): 0.50 ms instead of 1.8.
 #include <cuda_runtime.h>
 
 #include <algorithm>
