@@ -397,7 +397,7 @@ def run_ours(args):
     torch.cuda.synchronize()
     e2e_s = time.perf_counter() - t0
     e2e_value = world * noa * K / e2e_s
-    # ---- plain FP64 GPU form (same path, FP64 everywhere, cuBLAS DGEMM) ----
+    # ---- plain FP64 GPU form (same path, FP64 everywhere; contraction by digit planes) ----
     step(0, _lib.FPP_PREC_FP64)
     torch.cuda.synchronize()
     k64 = max(1, min(5, K))
@@ -562,12 +562,12 @@ def kuf_batch_leg(n_structures=256):
     rc 5.0, 1000 sparse environments drawn at random (seed 404), E, F and S
     label columns of every structure (labels are zeros: Kuf does not depend
     on them).  One fpp_kuf_batched call = the structures' FP64 descriptors
-    (queued without host synchronization) and one persistent adjoint-route
-    launch over all (structure, atom) items, tile shape from the library's
-    autotuner (cached in a file).  Reported: the Kuf kernel's CUDA-event
-    time on the second call, the whole call (host Kuf out), the tile shape,
-    and the kernel's FP64 rate from its algorithmic FLOP count against the
-    measured FP64 DGEMM rate of this GPU (1.10 TFLOP/s)."""
+    (queued without host synchronization), then per chunk of structures the
+    pairs' derivative rows, one FP64-accurate GEMM with the sparse environments
+    on the tensor cores and a gather per atom.  Reported: the Kuf kernels'
+    CUDA-event time on the second call, the whole call (host Kuf out), the
+    gather's tile, and the FP64 rate of the adjoint form's algorithmic FLOP
+    count against the measured FP64 DGEMM rate of this GPU (1.10 TFLOP/s)."""
     import flare_pp_gb300 as fg
     from flare_pp_gb300 import synth
     rc = 5.0
@@ -590,7 +590,7 @@ def kuf_batch_leg(n_structures=256):
             gp.add_specific_environments(strucs[k], atoms)
     sd, kern = gp.sparse_descriptors[0], gp.kernels[0]
     t0 = time.perf_counter()
-    gp._kuf_batched(sd, kern)                   # first call: autotune or cached tiles
+    gp._kuf_batched(sd, kern)
     first_s = time.perf_counter() - t0
     import torch
     torch.cuda.profiler.start()   # a profiler started with capture off sees this call
@@ -599,9 +599,9 @@ def kuf_batch_leg(n_structures=256):
     call_s = time.perf_counter() - t0
     torch.cuda.profiler.stop()
     ks, th, ms, items = gp.kuf_launch(len(gp._kuf_models) - 1)
-    # algorithmic FP64 FLOP of the kernel per (atom i, sparse environment k of
-    # i's species): z = dhat.phat (2 n_d), w (2 n_d), u = (W + W^T) c
-    # (2 n_rad^2 H), and per pair f = u . dc/dr (4 N H + 8 H)
+    # algorithmic FP64 FLOP per (atom i, sparse environment k of i's species), in
+    # the form that needs fewest (the adjoint's): z = dhat.phat (2 n_d), w (2 n_d),
+    # u = (W + W^T) c (2 n_rad^2 H), and per pair f = u . dc/dr (4 N H + 8 H)
     N, lmax, ns = 8, 3, 2
     H = (lmax + 1) ** 2
     nr = ns * N
@@ -618,10 +618,11 @@ def kuf_batch_leg(n_structures=256):
                         f"of 32-512 atoms, N=8 lmax=3 rc 5.0, {len(pick)} sparse)",
             "n_atoms": int(sum(len(sp) for _, sp, _ in cells)), "n_labels": int(n_labels),
             "work_items": int(items), "tiles": {"ks": ks, "threads": th},
-            "tile_source": "autotuner (cached per device and descriptor shape)",
+            "tile_source": "fixed (the gather's 32 environments by 8 atoms)",
             "kernel_ms": round(ms, 2), "call_s": round(call_s, 3),
             "first_call_s": round(first_s, 3),
-            "roofline": {"bound": "fp64", "achieved": round(achieved, 3),
+            "roofline": {"bound": "fp64 (its contraction on the tensor cores, so above 1)",
+                         "achieved": round(achieved, 3),
                          "peak": 1.10, "unit": "TFLOP/s", "frac": round(achieved / 1.10, 3),
                          "peak_source": "measured cuBLAS DGEMM rate of this GPU",
                          "algorithmic_flop": flop}}
@@ -630,9 +631,11 @@ def kuf_batch_leg(n_structures=256):
 def launches_per_step(n_species):
     # neighbors: wrap_bin, bin_scatter, enum, nb_readback, compact_geom (which
     # also links reverse pairs) and two CUB exclusive scans of two kernels each
-    # (compiled into the library); descriptors: forward; contraction: one
-    # grouped split GEMM; adjoint: wu, pair_force, gather, reduce; outputs: finish
-    return 9 + 1 + 1 + 4 + 1
+    # (compiled into the library; up to 8,192 counts one kernel per scan, which
+    # does the readback too); descriptors: forward (B3: and couple);
+    # contraction: one grouped split GEMM; adjoint: wu, pair_force, gather,
+    # reduce; outputs: finish
+    return 9 + 1 + (1 if SETTINGS["kind"] == "B3" else 0) + 1 + 4 + 1
 
 
 def oracle_check(w, positions, results):
@@ -784,7 +787,7 @@ def measure_matmul_peaks(n=8192, seconds=4.0):
     """FP64 and TF32 matmul peaks of this GPU, the way the bf16 peak is
     measured: torch.matmul of n^3 (2 n^3 FLOP), best of 10 (burst) and back to
     back for `seconds` (sustained), CUDA events.  The FP64 figures bound the
-    FP64 path (cuBLAS DGEMM contraction, training solve, uncertainties)."""
+    FP64 path (training solve, uncertainties)."""
     import torch
     dev = torch.device("cuda", 0)
     out = {}

@@ -16,7 +16,7 @@
 // Shared memory bounds it (operand reads and TMA writes against 128 bytes per cycle and
 // SM): in a pair each SM reads its 128 rows of P and half of the columns' rows of B, and
 // half of B is loaded; four stages fit instead of three.  32,768 atoms, 1500 columns:
-// 284 us with a CTA's own 128 x 128 tiles, 240 so.  (Waiting for the next stage behind
+// 284 us with a CTA's own 128 x 128 tiles, 270 so (tensor pipe 77 and 86 % busy).  (Waiting for the next stage behind
 // the first MMAs of one, which pays in gemm_ozaki.cu, costs a tenth here: the stage is
 // not there yet, and the MMAs after the wait are late.)
 //   warp 0 lane 0  TMA producer: 128B-swizzled K-major tiles of P_hi, P_lo (128 rows),

@@ -44,7 +44,7 @@ enum fpp_status {
 };
 
 enum fpp_precision {
-  FPP_PREC_FP64 = 0,  /* FP64 descriptors, FP64 contractions (cuBLAS DGEMM) */
+  FPP_PREC_FP64 = 0,  /* FP64 descriptors, FP64-accurate contractions (digit planes) */
   FPP_PREC_MIXED = 1  /* FP32 descriptors with compensated sums, tcgen05
                          contraction on split-fp16 operands, FP32 accumulate */
 };
@@ -477,9 +477,9 @@ int fpp_std_atom_compute(fpp_model *m, int32_t nlocal, int32_t nall,
 
 /* FP64-accurate C = A B^T on the fp16 tensor cores: row-major A (M x K, row
  * stride lda), B (N x K, ldb), C (M x N, ldc).  Each row of A and of B is cut
- * into 11 exact 5-bit digit planes relative to its largest entry; the level
- * sums of the digit products are exact in the FP32 accumulators and are added
- * in FP64, so every product keeps ~55 bits of each operand relative to its
+ * into 8 exact balanced 7-bit digit planes relative to its largest entry; the
+ * level sums of the digit products are exact in the FP32 accumulators and are
+ * added in 64-bit integers, then FP64, so every product keeps ~55 bits of each operand relative to its
  * row's largest entry (the error bound of an FP64 GEMM, with |a_ik| |b_jk|
  * replaced by max_k |a_ik| max_k |b_jk|).  The kernel-form GEMMs of
  * envs_struc / predict_SOR (normalized_dot_product.cpp:140-143,
