@@ -76,6 +76,7 @@ SIGNATURES = {
     "fpp_likelihood_gradient_stable": (_c_int, [_i32, _i32, _vp, _vp, _vp, _vp, _vp, _vp,
                                                 _vp, _vp, _vp, _i32, _vp, _vp, _vp]),
     "fpp_model_set_max_memory": (_c_int, [_vp, _dbl]),
+    "fpp_model_set_workspace_limits": (_c_int, [_vp, _i64, _i64, _i64]),
     "fpp_model_kuf_tiles": (_c_int, [_vp, _P(_i32), _P(_i32), _P(ctypes.c_float), _P(_i64)]),
     "fpp_model_pair_batches": (_c_int, [_vp, _P(_i32)]),
     "fpp_likelihood_gradient_stable_kernels": (_c_int, [_i32, _i32, _vp, _vp, _vp, _vp, _vp,

@@ -107,7 +107,7 @@ static int slice(fpp_model *m, KufWork &w, const KufItem *items, int n, double *
     if (m->sp[s].n_sparse > 0)
       FPP_TRY(ozaki_const(m->sp[s].oz_dhat, m->sp[s].n_sparse, nd,
                           m->sp[s].d_dhat.as<double>(), nd, st));
-  // structures in chunks of about kKufChunkBytes of rows; the digit planes and products
+  // structures in chunks of about kuf_chunk_bytes of rows; the digit planes and products
   // of a chunk are written and read once
   struct Chunk {
     int s0, s1;                      // structures
@@ -134,7 +134,7 @@ static int slice(fpp_model *m, KufWork &w, const KufItem *items, int n, double *
       const bool want_pairs = items[k].q.force_col || items[k].col_f0 >= 0 ||
                               items[k].q.col_s >= 0;
       const size_t b = want_pairs ? 3 * (size_t)S.n_pairs * rb : 0;
-      if (k > c.s0 && c.bytes + b > kKufChunkBytes) break;
+      if (k > c.s0 && c.bytes + b > m->kuf_chunk_bytes) break;
       c.bytes += b;
       KufGemmStruc &g = hs[k];
       std::memset(&g, 0, sizeof(g));
@@ -258,7 +258,7 @@ static int slice(fpp_model *m, KufWork &w, const KufItem *items, int n, double *
     return start[(size_t)(c * ns + s1) * ns] - start[(size_t)(c * ns + s0) * ns];
   };
   for (int c = 0; c < n_chunks; c++) {
-    if ((size_t)places(c, 0, ns) * 3 * rb <= 2 * kKufChunkBytes) {
+    if ((size_t)places(c, 0, ns) * 3 * rb <= 2 * m->kuf_chunk_bytes) {
       units.push_back({c, 0, ns});
       max_rows = std::max(max_rows, (size_t)places(c, 0, ns) * 3);
     } else {
@@ -294,6 +294,7 @@ static int slice(fpp_model *m, KufWork &w, const KufItem *items, int n, double *
   const int2 *dblocks = reinterpret_cast<const int2 *>(w.tables.as<char>() + at_blocks);
   const double *const *dzptr =
       reinterpret_cast<const double *const *>(w.tables.as<char>() + at_zptr);
+  int split = -1;  // the chunk whose descriptors z_planes holds
   for (const Unit &u : units) {
     const Chunk &c = chunks[u.chunk];
     ka.s0 = u.s0;
@@ -309,12 +310,15 @@ static int slice(fpp_model *m, KufWork &w, const KufItem *items, int n, double *
     for (int s = u.s0; s < u.s1; s++)
       ka.tiles[s + 1] = ka.tiles[s] + ceil_div(m->sp[s].n_sparse, 32);
     if (ka.tiles[u.s1] == 0) continue;
-    // z rows: one split of the chunk's descriptors (its species' rows only matter)
+    // z rows: one split of the chunk's descriptors, before the first of its units that
+    // runs (species without sparse environments have none)
     const int nz = c.z0[ns];
-    if (u.s0 == 0 && nz > 0 &&
-        launch_ozaki_split(nz, nd, nullptr, 0, w.z_planes.as<__half>(), zexps, st,
-                           dzptr + c.rows0) != 0)
-      return fail(FPP_ERR_CUDA, "digit-plane split launch failed");
+    if (split != u.chunk) {
+      if (nz > 0 && launch_ozaki_split(nz, nd, nullptr, 0, w.z_planes.as<__half>(), zexps, st,
+                                       dzptr + c.rows0) != 0)
+        return fail(FPP_ERR_CUDA, "digit-plane split launch failed");
+      split = u.chunk;
+    }
     if (launch_kuf_rows(ka, st) != 0)
       return fail(FPP_ERR_CUDA, "derivative rows launch failed");
     const OzakiMat zm{w.z_planes.as<__half>(), zexps, nz, nd};
@@ -349,7 +353,7 @@ int kuf_gemm(fpp_model *m, KufWork &w, const std::vector<KufItem> &items, double
   for (size_t k = 0; k < items.size();) {
     size_t e = k;
     long long pairs = 0;
-    while (e < items.size() && (e == k || (pairs + items[e].s->st.n_pairs <= (1ll << 29) &&
+    while (e < items.size() && (e == k || (pairs + items[e].s->st.n_pairs <= m->kuf_slice_pairs &&
                                            e - k < 32768)))
       pairs += items[e++].s->st.n_pairs;
     FPP_TRY(slice(m, w, items.data() + k, (int)(e - k), dK, n_labels, st));

@@ -15,11 +15,6 @@ struct KufItem {
   long long col_f0;
 };
 
-// Rows of a chunk of structures: large enough to fill the chip many times over (1 GB is
-// about 40,000 pairs at 448 columns and 150 environments, twelve rounds of GEMM tiles),
-// small enough that the workspace stays a fraction of the device.
-constexpr size_t kKufChunkBytes = (size_t)1 << 30;
-
 // Fewest sparse environments of a species for which fpp_kuf_batched takes this form.  Its
 // derivative rows and tiles cost the same for one environment as for tens, the adjoint
 // form's time is per environment: 32 cells of 8,460 atoms, N = 8, lmax = 3, two species,

@@ -478,6 +478,17 @@ int fpp_model_destroy(fpp_model *m) {
   return FPP_OK;
 }
 
+int fpp_model_set_workspace_limits(fpp_model *m, int64_t kuf_chunk_bytes,
+                                   int64_t kuf_slice_pairs, int64_t keep_bytes) {
+  if (!m) return fail(FPP_ERR_INVALID, "null argument");
+  if (kuf_slice_pairs > kKufSlicePairs)
+    return fail(FPP_ERR_CAPACITY, "more than 2^29 pairs in a slice");
+  m->kuf_chunk_bytes = kuf_chunk_bytes > 0 ? (size_t)kuf_chunk_bytes : kKufChunkBytes;
+  m->kuf_slice_pairs = kuf_slice_pairs > 0 ? (long long)kuf_slice_pairs : kKufSlicePairs;
+  m->keep_bytes = keep_bytes > 0 ? (size_t)keep_bytes : kKeepBytes;
+  return FPP_OK;
+}
+
 int fpp_model_set_sparse(fpp_model *m, int32_t species, int32_t n_sparse,
                          const double *descriptors, const double *norms,
                          const double *alpha) {
@@ -1023,7 +1034,7 @@ static int envs_struc_device(fpp_model *m, fpp_structure *s, cudaStream_t st, De
     it.q.col_s = 1 + 3ll * noa;
     FPP_TRY(kuf_gemm(m, m->kuf_work, {it}, K.as<double>(), n_out, st));
     FPP_TRY(ozaki_check_status(m->oz, st));
-    m->kuf_work.trim();
+    m->kuf_work.trim(m->keep_bytes);
     return FPP_OK;
   }
   // row-ordered atom norms
@@ -1330,7 +1341,7 @@ int fpp_kuf_batched(fpp_model *m, fpp_structure *const *structures, int32_t n_st
   float ms = 0.f;
   FPP_CUDA(cudaEventElapsedTime(&ms, ev.e0, ev.e1));
   m->kuf_ms = ms;
-  work.trim();
+  work.trim(m->keep_bytes);
   return FPP_OK;
 }
 

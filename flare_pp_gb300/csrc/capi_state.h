@@ -36,16 +36,21 @@ struct KufWork {
   DevBuf planes, f, partial;   // derivative rows: digit planes, products; block sums
   DevBuf K, cols;              // fpp_kuf_batched: the result, force columns
   // Kept between calls (allocating and freeing it took a tenth of a call of 32 cells)
-  // up to this much, given back above it and with the model.
-  static constexpr size_t kKeep = (size_t)2 << 30;
-  void trim() {
+  // up to `keep` bytes, given back above that and with the model.
+  void trim(size_t keep) {
     if (tables.bytes + pairs.bytes + z_planes.bytes + z.bytes + planes.bytes + f.bytes +
-            partial.bytes + K.bytes + cols.bytes <= kKeep)
+            partial.bytes + K.bytes + cols.bytes <= keep)
       return;
     for (DevBuf *b : {&tables, &pairs, &z_planes, &z, &planes, &f, &partial, &K, &cols})
       b->release();
   }
 };
+// Rows of a chunk of structures: large enough to fill the chip many times over (1 GB is
+// about 40,000 pairs at 448 columns and 150 environments, twelve rounds of GEMM tiles),
+// small enough that the workspace stays a fraction of the device.
+constexpr size_t kKufChunkBytes = (size_t)1 << 30;
+constexpr long long kKufSlicePairs = 1ll << 29;  // pairs of a slice, counted in an int
+constexpr size_t kKeepBytes = (size_t)2 << 30;   // workspace kept between calls
 }  // namespace fpp
 
 struct fpp_b2 {
@@ -119,6 +124,10 @@ struct fpp_model {
   fpp::DevBuf kuf_tab;                  // its column tables
   fpp::KufWork kuf_work;                // Kuf and envs_struc workspace
   std::mutex kuf_mu;                    // held while a call uses it
+  // limits of the workspaces (fpp_model_set_workspace_limits)
+  size_t kuf_chunk_bytes = fpp::kKufChunkBytes;
+  long long kuf_slice_pairs = fpp::kKufSlicePairs;
+  size_t keep_bytes = fpp::kKeepBytes;
   fpp::DevBuf es_K, sor;                // kernel matrix of a structure; SOR products
   // kernel-form workspaces (grown on demand, kept between calls): per-row
   // scalars, z / C / K blocks, second products, column sums and partials

@@ -293,6 +293,15 @@ int fpp_kuf_batched(fpp_model *m, fpp_structure *const *structures,
                     int32_t n_structures, const int32_t *label_mask,
                     const int32_t *atom_offsets, const int32_t *atoms,
                     double *kuf, int64_t n_labels, void *stream);
+/* Limits of m's device workspaces; 0 or less: the default.  kuf_chunk_bytes (1 GB): the
+ * derivative rows that fpp_kuf_batched, fpp_envs_struc and fpp_predict with variances
+ * form at a time, in whole structures (a structure of more than twice as much is taken
+ * species by species).  kuf_slice_pairs (2^29, the most): neighbor pairs of the
+ * structures that are ordered together.  keep_bytes (2 GB): workspace kept with the
+ * model between calls; a call that needed more gives it back.  Results do not depend on
+ * them.  No counterpart in the reference. */
+int fpp_model_set_workspace_limits(fpp_model *m, int64_t kuf_chunk_bytes,
+                                   int64_t kuf_slice_pairs, int64_t keep_bytes);
 /* The tile shape the last fpp_kuf_batched call on m used (sparse
  * environments per pass, threads per block), and (each may be NULL) the
  * CUDA-event time of its Kuf kernels in ms and its (structure, atom) work
