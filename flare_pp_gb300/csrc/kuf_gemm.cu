@@ -101,6 +101,8 @@ __host__ __device__ inline int sums_stride(const B2Args &a) {
 __host__ __device__ inline size_t rows_shared_doubles(const B2Args &a) {
   return (size_t)(2 * a.N + 4 * a.H) * kRowStride + 3 * kRowPairs;
 }
+// static shared memory of the kernel (m_i, m_sj, m_struc), out of the same limit
+constexpr size_t kRowStatic = 3 * sizeof(int) * kRowPairs;
 __host__ __device__ inline size_t rows_warp_doubles(const B2Args &a, int kc) {
   return (size_t)6 * sums_stride(a) * (a.lmax + 1) + ((kc + 3) & ~3);
 }
@@ -412,7 +414,7 @@ size_t kuf_rows_smem(const B2Args &a, int kc, int *warps) {
     for (int w = 8; w >= 1; w >>= 1) {
       const size_t b =
           sizeof(double) * (rows_shared_doubles(a) + w * rows_warp_doubles(a, kc));
-      if (b > cap || (cap < 200 * 1024 && w < 4)) continue;
+      if (b + kRowStatic > cap || (cap < 200 * 1024 && w < 4)) continue;
       if (warps) *warps = w;
       return b;
     }
