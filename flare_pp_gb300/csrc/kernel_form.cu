@@ -9,6 +9,8 @@
 // stress columns assembled per sparse environment.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernel_form.h"
 
@@ -178,14 +180,19 @@ int launch_envs_block(int S1, int S2, const double *Z, int ldz, const double *n1
 // then a thread per column over the chunks (a separate pass over the block and a
 // matrix-vector product with ones before: two more reads of it).
 constexpr int kColsumRows = 64;
+// rows of a chunk: a multiple of 64, so that the chunks fit a grid's y (65,535; more than 64
+// rows from 4.19 million on)
+static int colsum_rows(int rows) {
+  return kColsumRows * std::max(1, ceil_div(ceil_div(rows, kColsumRows), 65535));
+}
 __global__ void __launch_bounds__(128)
 k_envs_block_colsum(int rows, int S, double *__restrict__ Z, int ldz,
                     const double *__restrict__ rownorm, const double *__restrict__ snorm,
-                    double sig2, double power, double *__restrict__ partial) {
+                    double sig2, double power, int chunk, double *__restrict__ partial) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= S) return;
   const bool live = snorm[k] >= 1e-8;
-  const int r0 = blockIdx.y * kColsumRows, r1 = min(rows, r0 + kColsumRows);
+  const int r0 = blockIdx.y * chunk, r1 = min(rows, r0 + chunk);
   double sum = 0.0;
 #pragma unroll 8
   for (int r = r0; r < r1; r++) {
@@ -207,17 +214,16 @@ k_colsum_finish(int chunks, int S, const double *__restrict__ partial, double *_
 }
 
 size_t envs_colsum_partial(int rows, int S) {
-  return (size_t)ceil_div(rows, kColsumRows) * S;
+  return (size_t)ceil_div(rows, colsum_rows(rows)) * S;
 }
 
 int launch_envs_block_colsum(int rows, int S, double *Z, int ldz, const double *rownorm,
                              const double *snorm, double sig2, double power, double *partial,
                              double *out, cudaStream_t st) {
   if (rows <= 0 || S <= 0) return 0;
-  const int chunks = ceil_div(rows, kColsumRows), cols = ceil_div(S, 128);
-  if (chunks > 65535) return -1;
+  const int chunk = colsum_rows(rows), chunks = ceil_div(rows, chunk), cols = ceil_div(S, 128);
   k_envs_block_colsum<<<dim3(cols, chunks), 128, 0, st>>>(rows, S, Z, ldz, rownorm, snorm, sig2,
-                                                          power, partial);
+                                                          power, chunk, partial);
   k_colsum_finish<<<cols, 128, 0, st>>>(chunks, S, partial, out);
   return LAUNCH_OK;
 }
