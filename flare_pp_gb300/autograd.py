@@ -48,10 +48,17 @@ class FlareEnergy(torch.autograd.Function):
         return -grad_e * f, None, None, None
 
 
-def _plain():
-    """Whether nothing watches the autograd graph: gradients on, no tracing or
-    compilation, no functorch transform, no saved-tensor hooks."""
-    if not torch.is_grad_enabled() or torch.jit.is_tracing() or torch.compiler.is_compiling():
+def _plain(positions, n):
+    """Whether the graph would accept these positions of n atoms and nothing watches it:
+    an ordinary n x 3 FP64 CUDA tensor, gradients on, no anomaly detection (which raises
+    for NaN forces in the backward pass), no tracing or compilation, no functorch
+    transform, no saved-tensor hooks."""
+    if (type(positions) is not torch.Tensor or positions.dtype != torch.float64
+            or not positions.is_cuda or positions.shape != (n, 3)
+            or positions.layout != torch.strided or positions.is_inference()):
+        return False
+    if (not torch.is_grad_enabled() or torch.is_anomaly_enabled() or torch.jit.is_tracing()
+            or torch.compiler.is_compiling()):
         return False
     try:
         return not (torch._C._are_functorch_transforms_active()
@@ -68,7 +75,7 @@ def energy_forces_stress(gp, structure, positions, precision="mixed"):
     computes: they are returned from there unless something watches the graph
     (a backward pass through the engine costs as much host time as the whole
     evaluation of a hundred atoms)."""
-    if _plain():
+    if _plain(positions, structure.noa):
         return _evaluate(positions, gp, structure, precision)
     pos = positions.detach().requires_grad_(True)
     e = FlareEnergy.apply(pos, gp, structure, precision)
