@@ -933,7 +933,10 @@ int build_neighbors(StructureState &st, cudaStream_t stream) {
   DeviceStatus *dst = st.status.as<DeviceStatus>();
 
   const int tb = 256;
-  k_wrap_bin<<<ceil_div(noa, tb), tb, 0, stream>>>(
+  // blocks for the bins too: a few atoms in a large box have many more of them (8 atoms, 4.1
+  // million bins: 339 us per build by one block, 55 with these)
+  const int wrap_blocks = std::max(ceil_div(noa, tb), std::min(ceil_div(nbins, tb), 152 * 8));
+  k_wrap_bin<<<wrap_blocks, tb, 0, stream>>>(
       noa, st.positions.as<double>(), cd, st.wrapped.as<dvec4>(),
       st.wrapped32.as<float4>(), st.wrapped_lo.as<float4>(), st.frac.as<float4>(),
       st.atom_bin.as<int>(), st.bin_count.as<int>(), st.bin_cursor.as<int>(), nbins,
