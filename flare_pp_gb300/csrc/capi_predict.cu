@@ -1034,7 +1034,6 @@ static int envs_struc_device(fpp_model *m, fpp_structure *s, cudaStream_t st, De
     it.q.col_s = 1 + 3ll * noa;
     FPP_TRY(kuf_gemm(m, m->kuf_work, {it}, K.as<double>(), n_out, st));
     FPP_TRY(ozaki_check_status(m->oz, st));
-    m->kuf_work.trim(m->keep_bytes);
     return FPP_OK;
   }
   // row-ordered atom norms
@@ -1242,6 +1241,7 @@ int fpp_kuf_batched(fpp_model *m, fpp_structure *const *structures, int32_t n_st
   FPP_TRY(upload_pair_tab(m->pair_tab, m->pair_tab_host, st));
   // FP64 descriptors of every structure, queued without synchronization
   // (each structure keeps its own workspace), and the work lists
+  TrimOnReturn trim{m};
   std::lock_guard<std::mutex> lock(m->kuf_mu);
   KufWork &work = m->kuf_work;
   DevBuf &dK = work.K, &dfcol = work.cols, dstruc, ditems;
@@ -1341,7 +1341,6 @@ int fpp_kuf_batched(fpp_model *m, fpp_structure *const *structures, int32_t n_st
   float ms = 0.f;
   FPP_CUDA(cudaEventElapsedTime(&ms, ev.e0, ev.e1));
   m->kuf_ms = ms;
-  work.trim(m->keep_bytes);
   return FPP_OK;
 }
 
@@ -1397,6 +1396,7 @@ int fpp_local_uncertainties(fpp_model *m, fpp_structure *s, const double *L_inv,
   if (n != m->n_sparse_total)
     return fail(FPP_ERR_INVALID, "L_inv size differs from the sparse set");
   cudaStream_t st = (cudaStream_t)stream;
+  TrimOnReturn trim{m};
   StructureState &S = s->st;
   const int noa = S.noa, nd = m->n_d, ldp = round_up(nd, 64);
   if (noa == 0) return FPP_OK;
@@ -1469,6 +1469,7 @@ int fpp_predict_energy_uncertainty(fpp_model *m, fpp_structure *s, double *energ
   if (local_variances && !m->has_L_inv)
     return fail(FPP_ERR_INVALID, "L_inv not set (fpp_model_set_L_inv)");
   cudaStream_t st = (cudaStream_t)stream;
+  TrimOnReturn trim{m};
   StructureState &S = s->st;
   const int noa = S.noa, nd = m->n_d, ldp = round_up(nd, 64), n = m->n_sparse_total;
   if (noa == 0) {
@@ -1614,6 +1615,7 @@ int fpp_envs_struc(fpp_model *m, fpp_structure *s, double *kernel_mat, void *str
   FPP_TRY(model_check(m, s));
   if (!kernel_mat) return fail(FPP_ERR_INVALID, "null output");
   cudaStream_t st = (cudaStream_t)stream;
+  TrimOnReturn trim{m};
   DevBuf &K = m->es_K;
   FPP_TRY(envs_struc_device(m, s, st, K));
   FPP_CUDA(cudaStreamSynchronize(st));
@@ -1632,6 +1634,7 @@ int fpp_predict(fpp_model *m, fpp_structure *s, double *mean_efs, double *varian
     if (m->power < 1.0) return fail(FPP_ERR_UNSUPPORTED, "power < 1");
   }
   cudaStream_t st = (cudaStream_t)stream;
+  TrimOnReturn trim{m};
   StructureState &S = s->st;
   const int noa = S.noa, nd = m->n_d, ldp = round_up(nd, 64);
   const int n_out = 1 + 3 * noa + 6;

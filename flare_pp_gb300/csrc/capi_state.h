@@ -132,6 +132,19 @@ struct fpp_model {
   // kernel-form workspaces (grown on demand, kept between calls): per-row
   // scalars, z / C / K blocks, second products, column sums and partials
   fpp::DevBuf kf_rows, kf_z, kf_q, kf_cols;
+  // Given back at the end of a call that needed more than keep_bytes of them (a kernel
+  // matrix of 4000 environments and 10,000 atoms, its transpose, products and planes: 5 GB).
+  void trim() {
+    size_t n = 0;
+    std::vector<fpp::DevBuf *> all = {&es_K, &sor, &kf_rows, &kf_z, &kf_q, &kf_cols,
+                                      &oz.a.buf, &oz.b.buf};
+    for (auto &s : sp) all.push_back(&s.oz_c.buf);
+    for (fpp::DevBuf *b : all) n += b->bytes;
+    if (n > keep_bytes)
+      for (fpp::DevBuf *b : all) b->release();
+    std::lock_guard<std::mutex> lock(kuf_mu);
+    kuf_work.trim(keep_bytes);
+  }
   fpp_structure *batch = nullptr;       // packed structure of a batched prediction
   fpp::DevBuf batch_off, batch_sums, batch_src;
   // envs_struc workspace of the stored-derivative form (grown on demand, kept between calls)
@@ -141,6 +154,12 @@ struct fpp_model {
 };
 
 namespace fpp {
+// Trims the model's workspaces on every return path of a call that synchronizes (before a
+// lock of kuf_mu in the same scope).
+struct TrimOnReturn {
+  fpp_model *m;
+  ~TrimOnReturn() { m->trim(); }
+};
 // columns of the mixed form's operand (power 2 may leave columns out)
 inline int mixed_nd(const fpp_model *m) {
   return m->beta_power == 2 && !m->mixed_cols.empty() ? (int)m->mixed_cols.size() : m->n_d;
