@@ -200,7 +200,7 @@ static double pair_bytes_per_atom(const fpp_model *m, int max_neigh, int precisi
   const double ldp = (double)((m->n_d + 63) / 64 * 64);
   double per = 4.0 * (2 * sb + 2 * ldp) + 2.0 * 2 * ldp  // c, u, V, w; split operand
                + 8.0 * 8;                                // norms, energies, rows
-  if (precision == FPP_PREC_FP64) per += 8.0 * (2 * sb + 3 * ldp) + 2.0 * kOzakiDigits * ldp;
+  if (precision == FPP_PREC_FP64) per += 8.0 * (2 * sb + 2 * ldp) + 2.0 * kOzakiDigits * ldp;
   // per neighbor: FP64 and FP32 geometry, indices, pair forces, the list
   per += (double)max_neigh * (32 + 16 + 4 * 4 + 16 + 4 + (precision == FPP_PREC_FP64 ? 16 : 0));
   return per;

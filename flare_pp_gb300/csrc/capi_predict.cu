@@ -848,28 +848,41 @@ static int contract64(fpp_model *m, fpp_structure *s, const double *phat, int ld
   StructureState &S = s->st;
   const int nd = m->n_d;
   FPP_TRY(S.V64.reserve(sizeof(double) * (size_t)s->total_rows * ldp));
-  OzakiProblem q[kOzakiMaxGroups];
-  int nq = 0;
   for (int sp = 0; sp < m->n_species; sp++) {
-    if (s->n_rows[sp] == 0) continue;
     auto &M = m->sp[sp];
-    double *V = S.V64.as<double>() + (size_t)s->row_off[sp] * ldp;
-    if (!M.beta_finite) {
-      cublasHandle_t h;
-      FPP_TRY(get_cublas(m, st, &h));
-      const double one = 1.0, zero = 0.0;
-      FPP_CUBLAS(cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, nd, s->n_rows[sp], nd, &one,
-                             M.beta64.as<double>(), m->ldb,
-                             phat + (size_t)s->row_off[sp] * ldp, ldp, &zero, V, ldp));
-      continue;
-    }
-    // beta is symmetric: row n of B is column n
-    FPP_TRY(ozaki_const(M.oz_beta, nd, nd, M.beta64.as<double>(), m->ldb, st));
-    if (nq == 0) FPP_TRY(ozaki_split(S.oz_p, s->total_rows, nd, phat, ldp, st));
-    q[nq++] = OzakiProblem{ozaki_mat(S.oz_p), ozaki_mat(M.oz_beta), s->row_off[sp],
-                           s->n_rows[sp], nd, V, ldp, false};
+    if (M.beta_finite || s->n_rows[sp] == 0) continue;
+    cublasHandle_t h;
+    FPP_TRY(get_cublas(m, st, &h));
+    const double one = 1.0, zero = 0.0;
+    FPP_CUBLAS(cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, nd, s->n_rows[sp], nd, &one,
+                           M.beta64.as<double>(), m->ldb,
+                           phat + (size_t)s->row_off[sp] * ldp, ldp, &zero,
+                           S.V64.as<double>() + (size_t)s->row_off[sp] * ldp, ldp));
   }
-  return ozaki_run(q, nq, S.status.as<DeviceStatus>(), st, 9);
+  // rows in equal blocks whose planes take at most keep_bytes (all of them up to 87,000
+  // rows of 1500 descriptors): the planes are twice the size of phat
+  const size_t row_bytes = ozaki_shape(128, nd).plane_bytes / 128;
+  const int most = (int)std::min<size_t>(std::max<size_t>(m->keep_bytes / row_bytes / 128, 1) * 128,
+                                         (size_t)round_up(s->total_rows, 128));
+  const int block = round_up(ceil_div(s->total_rows, ceil_div(s->total_rows, most)), 128);
+  for (int r0 = 0; r0 < s->total_rows; r0 += block) {
+    const int r1 = std::min(s->total_rows, r0 + block);
+    OzakiProblem q[kOzakiMaxGroups];
+    int nq = 0;
+    for (int sp = 0; sp < m->n_species; sp++) {
+      auto &M = m->sp[sp];
+      const int lo = std::max(r0, s->row_off[sp]);
+      const int hi = std::min(r1, s->row_off[sp] + s->n_rows[sp]);
+      if (!M.beta_finite || lo >= hi) continue;
+      // beta is symmetric: row n of B is column n
+      FPP_TRY(ozaki_const(M.oz_beta, nd, nd, M.beta64.as<double>(), m->ldb, st));
+      if (nq == 0) FPP_TRY(ozaki_split(S.oz_p, r1 - r0, nd, phat + (size_t)r0 * ldp, ldp, st));
+      q[nq++] = OzakiProblem{ozaki_mat(S.oz_p), ozaki_mat(M.oz_beta), lo - r0, hi - lo, nd,
+                             S.V64.as<double>() + (size_t)lo * ldp, ldp, false};
+    }
+    FPP_TRY(ozaki_run(q, nq, S.status.as<DeviceStatus>(), st, 9));
+  }
+  return FPP_OK;
 }
 
 // Forward, contraction and adjoint of the mapped form; leaves atom_e, pair_f

@@ -299,7 +299,9 @@ int fpp_kuf_batched(fpp_model *m, fpp_structure *const *structures,
  * species by species).  kuf_slice_pairs (2^29, the most): neighbor pairs of the
  * structures that are ordered together.  keep_bytes (2 GB): workspace kept with the
  * model between calls; a call that needed more gives it back.  Results do not depend on
- * them.  No counterpart in the reference. */
+ * them.  keep_bytes also bounds the digit planes that an FP64 mapped evaluation of power
+ * 2 keeps with the structure: more atoms are contracted in several passes.  No counterpart
+ * in the reference. */
 int fpp_model_set_workspace_limits(fpp_model *m, int64_t kuf_chunk_bytes,
                                    int64_t kuf_slice_pairs, int64_t keep_bytes);
 /* The tile shape the last fpp_kuf_batched call on m used (sparse

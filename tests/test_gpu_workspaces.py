@@ -62,3 +62,37 @@ def test_given_back_above_the_limit(gpu_lib):
         assert free() - f0 >= held, (call.__name__, free() - f0, held)
         for w, g, a in zip(want, got, again):
             assert (np.asarray(w) == g).all() and (np.asarray(w) == a).all()
+
+
+@pytest.mark.parametrize("ns", [1, 3])
+def test_fp64_contraction_in_blocks(gpu_lib, ns):
+    """Rows of phat in blocks of 128 and of 1,024: less memory, the same bits (each row's
+    products are exact integer sums)."""
+    import torch
+    rc = 4.0
+    b = fg.B2("chebyshev", "quadratic", [0, rc], [], [ns, 8 // ns, 3])
+    b.store_dervs = False
+    rng = np.random.default_rng(9)
+    bcc = np.array([[0.0, 0.0, 0.0], [0.5, 0.5, 0.5]])
+    cd = fg.ClusterDescriptor(fg.Structure(
+        *synth.rattled(bcc, 3.0, (4, 4, 4), 0.1, rng, n_species=ns), rc, [b]).descriptors[0])
+    gp = fg.SparseGP([fg.NormalizedDotProduct(2.0, 2)], 0.01, 0.05, 0.006)
+    gp.set_model(b, cd, rng.uniform(0.5, 1.5, size=cd.n_clusters))
+    frame = synth.rattled(bcc, 3.0, (16, 16, 13), 0.1, rng, n_species=ns)
+    row = 16 * -(-b.n_descriptors // 64) * 64  # bytes of a row's planes
+    want, used = None, []
+    gp.predict_mapped(fg.Structure(*frame, rc), "fp64")  # the model's own buffers
+    for keep in (0, row * 1024, 1):
+        check(gpu_lib.fpp_model_set_workspace_limits(gp._model.handle, 0, 0, keep))
+        s = fg.Structure(*frame, rc)
+        torch.cuda.synchronize()
+        f0 = torch.cuda.mem_get_info()[0]
+        got = gp.predict_mapped(s, "fp64")
+        torch.cuda.synchronize()
+        used.append(f0 - torch.cuda.mem_get_info()[0])
+        if want is None:
+            want = got
+        for w, g in zip(want, got):
+            assert (np.asarray(w) == np.asarray(g)).all(), keep
+    planes = row * len(frame[1])
+    assert used[0] - used[1] >= planes // 2 and used[0] - used[2] >= planes // 2, (used, planes)
