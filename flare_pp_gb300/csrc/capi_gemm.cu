@@ -12,23 +12,23 @@
 namespace fpp {
 
 int ozaki_split(OzakiOperand &op, int rows, int K, const double *X, long long ldx,
-                cudaStream_t st) {
+                cudaStream_t st, const OzakiColumns *cols) {
   const OzakiShape sh = ozaki_shape(rows, K);
   // one allocation: the planes, then the row exponents
   FPP_TRY(op.buf.reserve(sh.plane_bytes + sizeof(int) * (size_t)std::max(rows, 1)));
   op.rows = rows;
   op.K = K;
   op.exps_at = sh.plane_bytes;
-  if (launch_ozaki_split(rows, K, X, ldx, op.planes(), op.exps(), st) != 0)
+  if (launch_ozaki_split(rows, K, X, ldx, op.planes(), op.exps(), st, nullptr, cols) != 0)
     return fail(FPP_ERR_CUDA, "digit-plane split launch failed");
   return FPP_OK;
 }
 
 int ozaki_const(OzakiOperand &op, int rows, int K, const double *X, long long ldx,
-                cudaStream_t st) {
+                cudaStream_t st, const OzakiColumns *cols) {
   if (op.ready && op.rows == rows && op.K == K) return FPP_OK;
   op.ready = false;
-  FPP_TRY(ozaki_split(op, rows, K, X, ldx, st));
+  FPP_TRY(ozaki_split(op, rows, K, X, ldx, st, cols));
   FPP_CUDA(cudaStreamSynchronize(st));  // later calls may run on other streams
   op.ready = true;
   return FPP_OK;

@@ -87,6 +87,7 @@ struct fpp_model {
     bool beta_finite = true;            // every entry of it
     // digit planes of the constant GEMM operands, split on first use
     fpp::OzakiOperand oz_beta, oz_dhat, oz_dhatT, oz_Linv;
+    int *beta_shift = nullptr;          // int[n_d]: its columns' powers of two (in its buffer)
     fpp::OzakiOperand oz_c;             // workspace: C (or K) rows of the species' atoms
   };
   std::vector<Species> sp;
@@ -201,9 +202,9 @@ int ozaki_check_status(OzakiWork &w, cudaStream_t st);
 // same for a constant of a model (split once; ready is reset where the matrix
 // changes), and several products in one launch.
 int ozaki_split(OzakiOperand &op, int rows, int K, const double *X, long long ldx,
-                cudaStream_t st);
+                cudaStream_t st, const OzakiColumns *cols = nullptr);
 int ozaki_const(OzakiOperand &op, int rows, int K, const double *X, long long ldx,
-                cudaStream_t st);
+                cudaStream_t st, const OzakiColumns *cols = nullptr);
 OzakiMat ozaki_mat(const OzakiOperand &op);
 int ozaki_run(const OzakiProblem *probs, int n, DeviceStatus *status, cudaStream_t st,
               int n_levels = 8);

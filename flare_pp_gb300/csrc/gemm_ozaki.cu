@@ -562,13 +562,23 @@ k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
   }
 }
 
+// The bits of v 2^k (exactly where that is a normal number; zeros, Inf and NaN as they are).
+__device__ __forceinline__ unsigned long long shift_bits(unsigned long long b, int k) {
+  const int ex = (int)((b >> 52) & 0x7ff);
+  if (ex != 0 && ex != 0x7ff && ex + k > 0 && ex + k < 0x7ff)
+    return b + ((unsigned long long)(long long)k << 52);
+  if (ex == 0x7ff || (b << 1) == 0ull) return b;
+  return (unsigned long long)__double_as_longlong(
+      scale_pow2(__longlong_as_double((long long)b), k));
+}
+
 // Digit planes of the rows of X (rows x K, leading dimension ldx; or the rows that
-// `ptr` points to): a warp per row, four entries per lane; rows >= rows and columns
-// >= K of the padded planes are zeros.
+// `ptr` points to), their columns scaled by cols: a warp per row, four entries per lane;
+// rows >= rows and columns >= K of the padded planes are zeros.
 __global__ void __launch_bounds__(256)
 k_ozaki_split(int rows, int K, long long ldx, const double *__restrict__ X,
               const double *const *__restrict__ ptr, int rows_pad, int k_pad,
-              __half *__restrict__ planes, int *__restrict__ exps) {
+              __half *__restrict__ planes, int *__restrict__ exps, const OzakiColumns cols) {
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= rows_pad) return;
   const size_t plane = (size_t)rows_pad * k_pad;
@@ -581,6 +591,9 @@ k_ozaki_split(int rows, int K, long long ldx, const double *__restrict__ X,
   }
   const double *x = ptr ? ptr[r] : X + (size_t)r * ldx;
   const bool al = (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+  const int *sh = nullptr;
+  for (int g = 0; g < cols.n; g++)
+    if (r >= cols.row0[g]) sh = cols.shift[g];
   const int e = ozaki_split_row(
       K, k_pad, plane, dst, lane, [&](int k, unsigned long long (&b)[4]) {
         if (al && k + 4 <= K) {
@@ -592,8 +605,66 @@ k_ozaki_split(int rows, int K, long long ldx, const double *__restrict__ X,
           for (int i = 0; i < 4; i++)
             b[i] = k + i < K ? (unsigned long long)__double_as_longlong(x[k + i]) : 0ull;
         }
+        if (sh) {
+          const int4 c = *reinterpret_cast<const int4 *>(sh + k);
+          b[0] = shift_bits(b[0], cols.sign * c.x);
+          b[1] = shift_bits(b[1], cols.sign * c.y);
+          b[2] = shift_bits(b[2], cols.sign * c.z);
+          b[3] = shift_bits(b[3], cols.sign * c.w);
+        }
       });
   if (lane == 0) exps[r] = e;
+}
+
+// One damped step of the equilibration of a symmetric matrix: e_out[i] = (e_i + r_i) / 2
+// with 2^r_i the largest |a_ij| 2^-e_j of row i (at its fixed point the largest
+// |a_ij| 2^(-e_i - e_j) of every row is about 1); e_in null: zeros.  A warp per row;
+// entries n .. n4 - 1 of e_out are set to zero.
+constexpr int kMaxShift = 400;
+__global__ void __launch_bounds__(128)
+k_equilibrate(int n, int n4, int lda, const double *__restrict__ a,
+              const int *__restrict__ e_in, int *__restrict__ e_out) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (i >= n) {
+    if (i < n4 && lane == 0) e_out[i] = 0;
+    return;
+  }
+  constexpr int kNone = -(1 << 20);
+  int r = kNone;
+  const double *row = a + (size_t)i * lda;
+  for (int j0 = lane; j0 < n; j0 += 32 * 16) {  // sixteen loads in flight
+    long long b[16];
+    int e[16];
+#pragma unroll
+    for (int u = 0; u < 16; u++) {
+      const int j = j0 + 32 * u;
+      b[u] = j < n ? __double_as_longlong(row[j]) : 0ll;
+      e[u] = e_in && j < n ? e_in[j] : 0;
+    }
+#pragma unroll
+    for (int u = 0; u < 16; u++) {
+      const int ex = (int)((b[u] >> 52) & 0x7ff);
+      if (ex != 0) r = max(r, ex - 1023 - e[u]);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) r = max(r, __shfl_xor_sync(0xffffffffu, r, o));
+  // a column of zeros: out of the way of its rows' largest entry
+  if (lane == 0)
+    e_out[i] = r == kNone
+                   ? -kMaxShift
+                   : max(-kMaxShift, min(kMaxShift, ((e_in ? e_in[i] : 0) + r) >> 1));
+}
+
+int launch_equilibrate(int n, const double *a, int lda, int *shift, int *tmp,
+                       cudaStream_t stream) {
+  if (n <= 0) return 0;
+  const int n4 = (n + 3) / 4 * 4;
+  // six steps: a factor that spans 2^80 is then within 2^(80 / 64) of its fixed point
+  for (int it = 0; it < 6; it++)
+    k_equilibrate<<<ceil_div(n4, 4), 128, 0, stream>>>(
+        n, n4, lda, a, it == 0 ? nullptr : (it & 1 ? tmp : shift), it & 1 ? shift : tmp);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 static int ozaki_launch_shape(int dev, int *pairs) {
@@ -635,14 +706,16 @@ OzakiShape ozaki_shape(int rows, int K) {
 }
 
 int launch_ozaki_split(int rows, int K, const double *X, long long ldx, __half *planes,
-                       int *exps, cudaStream_t stream, const double *const *row_ptr) {
+                       int *exps, cudaStream_t stream, const double *const *row_ptr,
+                       const OzakiColumns *cols) {
   if (rows <= 0) return 0;
   const OzakiShape sh = ozaki_shape(rows, K);
   const int threads = 256;
   const long long warps = sh.rows_pad;
   const int blocks = (int)((warps * 32 + threads - 1) / threads);
   k_ozaki_split<<<blocks, threads, 0, stream>>>(rows, K, ldx, X, row_ptr, sh.rows_pad,
-                                                 sh.k_pad, planes, exps);
+                                                 sh.k_pad, planes, exps,
+                                                 cols ? *cols : OzakiColumns{});
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

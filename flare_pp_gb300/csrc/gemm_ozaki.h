@@ -26,9 +26,24 @@ OzakiShape ozaki_shape(int rows, int K);
 // exponent e of each row (max |row| < 2^e; kOzakiNanRow if the row holds a
 // non-finite entry) of X (rows x K, row stride ldx, device memory).
 constexpr int kOzakiNanRow = -(1 << 30);
+// Powers of two by which the columns are scaled before the split, exactly: column k of the
+// rows from row0[g] on (up to the next group's) by 2^(sign shift[g][k]), where shift[g] (device,
+// 16-byte aligned, K entries padded to a multiple of four) is not null.  With 2^shift on one
+// operand and 2^-shift on the other the product is the same, but what counts as a row's
+// largest entry is not.
+struct OzakiColumns {
+  const int *shift[kOzakiMaxGroups] = {};
+  int row0[kOzakiMaxGroups] = {};
+  int n = 0, sign = 1;
+};
 // row_ptr (device): where each row starts, instead of X and ldx.
 int launch_ozaki_split(int rows, int K, const double *X, long long ldx, __half *planes,
-                       int *exps, cudaStream_t stream, const double *const *row_ptr = nullptr);
+                       int *exps, cudaStream_t stream, const double *const *row_ptr = nullptr,
+                       const OzakiColumns *cols = nullptr);
+// Such powers of two for a symmetric matrix (finite, n x n, row stride lda): the largest
+// |a_ij| 2^(-shift_i - shift_j) of every row about 1.  tmp: scratch of the same size.
+int launch_equilibrate(int n, const double *a, int lda, int *shift, int *tmp,
+                       cudaStream_t stream);
 
 // An operand split by launch_ozaki_split.
 struct OzakiMat {
