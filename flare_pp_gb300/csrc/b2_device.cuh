@@ -143,12 +143,10 @@ __device__ __forceinline__ double w_mixed2(const AdjArgs &g, int si, int nd, flo
       if (q0 + 32 * u < nq) {
         float dl[4];
         deltas(h[u], l[u], dl);
-        // four products, then one compensated addition
-        float sum = fmaf(2.0f, gg[u].x, v[u].x) * dl[0];
-        sum = fmaf(fmaf(2.0f, gg[u].y, v[u].y), dl[1], sum);
-        sum = fmaf(fmaf(2.0f, gg[u].z, v[u].z), dl[2], sum);
-        sum = fmaf(fmaf(2.0f, gg[u].w, v[u].w), dl[3], sum);
-        acc.add(sum);
+        acc.add(fmaf(2.0f, gg[u].x, v[u].x) * dl[0]);
+        acc.add(fmaf(2.0f, gg[u].y, v[u].y) * dl[1]);
+        acc.add(fmaf(2.0f, gg[u].z, v[u].z) * dl[2]);
+        acc.add(fmaf(2.0f, gg[u].w, v[u].w) * dl[3]);
       }
     }
   }
