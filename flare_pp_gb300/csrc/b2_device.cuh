@@ -69,6 +69,20 @@ __device__ __forceinline__ float2 norm_ff(const Acc<float> &acc, float &invf) {
   return make_float2(r0, rc);
 }
 
+// This lane's part of sum p^2 over a row in shared memory (nd a multiple of four, 16-byte
+// aligned), every square compensated.
+__device__ __forceinline__ Acc<float> sum_squares(const float *p, int nd, int lane) {
+  Acc<float> acc;
+  for (int q = lane; q < (nd >> 2); q += 32) {
+    const float4 v = reinterpret_cast<const float4 *>(p)[q];
+    acc.add(v.x * v.x);
+    acc.add(v.y * v.y);
+    acc.add(v.z * v.z);
+    acc.add(v.w * v.w);
+  }
+  return acc;
+}
+
 // The centred split operand row of one atom, delta = p / |p| - pbar scaled by 2^13
 // as fp16 value and residual (scaled by 2^11), from p in shared memory; nd a
 // multiple of four, rows 8-byte aligned: four entries per lane, 16-byte reads,

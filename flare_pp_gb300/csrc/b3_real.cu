@@ -409,13 +409,8 @@ k_b3_couple(int noa, int apb, int nr, int nd, const int *__restrict__ species,
     const int atom = a0 + at, si = species[atom];
     const size_t row = row_of_atom[atom];
     const float *pa = p_s + (size_t)at * nd;
-    Acc<float> acc;  // four squares first, then one compensated addition
-    for (int q = lane; q < (nd >> 2); q += 32) {
-      const float4 v = reinterpret_cast<const float4 *>(pa)[q];
-      acc.add(fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w))));
-    }
     float invf;
-    const float2 nrm = norm_ff(acc, invf);
+    const float2 nrm = norm_ff(sum_squares(pa, nd, lane), invf);
     if (lane == 0) reinterpret_cast<float2 *>(norm_out)[atom] = nrm;
     write_split_row(pa, nd, invf, pbar + (size_t)si * nd, phat_hi + row * ldp,
                     phat_lo + row * ldp, lane);

@@ -18,6 +18,14 @@ __global__ void k_energy(AdjArgs g, int nd, const float4 *V, const uint2 *hi, co
   if (lane == 0) out[0] = e;
 }
 
+// |p| of a row that holds 2^-13, 2^-13, 2^-13, 1 in every quad
+__global__ void k_norm(int nd, const float *p, double *out) {
+  const int lane = threadIdx.x;
+  float inv;
+  const float2 n = norm_ff(sum_squares(p, nd, lane), inv);
+  if (lane == 0) out[1] = (double)n.x + (double)n.y;
+}
+
 template <typename T> static T *upload(const std::vector<T> &v) {
   void *p = nullptr;
   if (cudaMalloc(&p, sizeof(T) * v.size()) != cudaSuccess ||
@@ -44,8 +52,11 @@ int main(int argc, char **argv) {
   k_energy<<<1, 32>>>(g, nd, reinterpret_cast<const float4 *>(upload(v)),
                       reinterpret_cast<const uint2 *>(upload(hi)),
                       reinterpret_cast<const uint2 *>(upload(lo)), out);
+  std::vector<float> p(nd, 1.220703125e-4f);  // 2^-13
+  for (int q = 0; q < quads; q++) p[4 * q + 3] = 1.0f;
+  k_norm<<<1, 32>>>(nd, upload(p), out);
   double h[2];
   if (cudaMemcpy(h, out, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess) return 2;
-  std::printf("energy %.17g\n", h[0]);
+  std::printf("energy %.17g\nnorm %.17g\n", h[0], h[1]);
   return 0;
 }

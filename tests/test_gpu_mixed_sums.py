@@ -4,7 +4,12 @@ device code).
 
 Each quad of a row adds 1 + 2^-25 + 2^-25 - 1 to an energy.  Compensated entry by entry every
 term below is a multiple of 2^-25 under 2^-25 2^24, so the sum 2^-24 quads is exact; an
-uncompensated addition within a quad gives 0."""
+uncompensated addition within a quad gives 0.
+
+A norm of quads (2^-13, 2^-13, 2^-13, 1) is sqrt(quads (1 + 3 2^-26)); its float-float sums are
+exact to 2^-46 of it and the corrected square root to the square of FP32's half unit, 2^-48:
+2^-44 of the norm.  Without compensation within a quad it errs by 2^-25.4."""
+import math
 import os
 import subprocess
 
@@ -36,3 +41,9 @@ def run(harness, quads):
 @pytest.mark.parametrize("quads", [1, 5, 32, 129, 400])
 def test_energy(harness, quads):
     assert run(harness, quads)["energy"] == quads * 2.0 ** -24
+
+
+@pytest.mark.parametrize("quads", [1, 5, 32, 129, 400])
+def test_norm(harness, quads):
+    want = math.sqrt(quads * (1 + 3 * 2.0 ** -26))
+    assert abs(run(harness, quads)["norm"] - want) <= 2.0 ** -44 * want
