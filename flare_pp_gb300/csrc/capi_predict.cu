@@ -730,7 +730,9 @@ static int set_center(fpp_model *m, const std::vector<std::vector<double>> &pbar
         gv[(size_t)s * mnd + j] = (float)acc;
         c0 += p[a] * acc;
       }
-      m->c0[s] = c0;
+      // columns that are left out are zeros, not skipped: an Inf or NaN coefficient of theirs
+      // makes the energy and the forces NaN, as in FP64
+      m->c0[s] = all || m->sp[s].beta_finite ? c0 : std::nan("");
     }
   }
   // g is used in FP32; c0 must then be consistent with the same pbar: the
