@@ -1298,7 +1298,8 @@ int fpp_kuf_batched(fpp_model *m, fpp_structure *const *structures, int32_t n_st
                            cudaMemcpyHostToDevice, st));
   int max_sparse = 0;
   for (auto &x : m->sp) max_sparse = std::max(max_sparse, x.n_sparse);
-  const bool gemm = kuf_gemm_fits(m) && max_sparse >= kKufGemmSparse;
+  const bool gemm =
+      kuf_gemm_fits(m) && max_sparse >= kuf_gemm_sparse(m->n_d, n_structures);
   std::vector<KufItem> batch;  // by one GEMM
   std::vector<int2> items;     // (structure, atom) by the adjoint
   long long n_atoms = 0;

@@ -277,9 +277,10 @@ int fpp_predict_energy_uncertainty(fpp_model *m, fpp_structure *s, double *energ
  * FP64 on the GPU.  The columns are the envs_struc values of
  * normalized_dot_product.cpp:115-210: all pairs' derivative rows times the sparse
  * environments as one FP64-accurate GEMM per chunk of structures, then a gather per
- * atom (one synchronization for the batch; sums in a fixed order).  With fewer than ten
- * sparse environments of every species, and for a structure whose rows would take more
- * than 16 GB, the adjoint route instead: one persistent launch over the (structure,
+ * atom (one synchronization for the batch; sums in a fixed order).  With few sparse
+ * environments of every species (fewer than 10 to 64, by the descriptors and the
+ * structures), and for a structure whose rows would take more than 16 GB, the adjoint
+ * route instead: one persistent launch over the (structure,
  * atom) work list, its tile shape (sparse environments per pass, threads per block)
  * autotuned once per device and descriptor shape and cached in the file
  * $FPP_TUNE_CACHE (else $HOME/.cache/flare_pp_gb300/tiles.txt), its additions into
