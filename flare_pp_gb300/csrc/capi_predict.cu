@@ -1702,8 +1702,11 @@ int fpp_predict(fpp_model *m, fpp_structure *s, double *mean_efs, double *varian
     double *V = m->sor.as<double>(), *KT = V + nv, *alpha = KT + nv, *mean = alpha + n1,
            *var = mean + n_out;
     FPP_CUDA(cudaMemcpyAsync(alpha, al.data(), sizeof(double) * al.size(), cudaMemcpyHostToDevice, st));
-    FPP_CUBLAS(cublasDgemv(h, CUBLAS_OP_N, n_out, nst, &one, K.as<double>(), n_out, alpha, 1,
-                           &zero, mean, 1));
+    // (without sparse environments cuBLAS writes nothing: a mean of zero)
+    FPP_CUDA(cudaMemsetAsync(mean, 0, sizeof(double) * n_out, st));
+    if (nst > 0)
+      FPP_CUBLAS(cublasDgemv(h, CUBLAS_OP_N, n_out, nst, &one, K.as<double>(), n_out, alpha, 1,
+                             &zero, mean, 1));
     // V[o][i] = sum_k K[k][o] R_inv[k][i] (predict_SOR's R_inv^T K, row o per
     // label) on the tensor cores, FP64-accurate: operands K^T and R_inv^T
     if (nst > 0) {
