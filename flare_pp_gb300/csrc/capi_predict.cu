@@ -559,25 +559,27 @@ static int upload_beta(fpp_model *m, int s, const std::vector<double> &B) {
   auto &sp = m->sp[s];
   std::vector<double> pad((size_t)nd * ldb, 0.0);
   bool finite = true;
+  double amax = 0;
   for (int i = 0; i < nd; i++)
     for (int j = 0; j < nd; j++) {
       const double v = B[(size_t)i * nd + j];
       pad[(size_t)i * ldb + j] = v;
       finite = finite && std::isfinite(v);
+      amax = std::max(amax, std::fabs(v));
     }
   // the mixed operand: all columns, or the listed ones (-1: padding)
   const std::vector<int> &cols = m->mixed_cols;
-  const int mnd = cols.empty() ? nd : (int)cols.size(), mld = round_up(mnd, 64);
-  std::vector<double> mix((size_t)mnd * mld, 0.0);
-  double amax = 0;
+  const int mnd = (int)cols.size(), mld = round_up(mnd, 64);
+  std::vector<double> some((size_t)mnd * mld, 0.0);
+  if (mnd) amax = 0;
   for (int i = 0; i < mnd; i++)
     for (int j = 0; j < mnd; j++) {
-      const int a = cols.empty() ? i : cols[i], b = cols.empty() ? j : cols[j];
-      if (a < 0 || b < 0) continue;
-      const double v = B[(size_t)a * nd + b];
-      mix[(size_t)i * mld + j] = v;
+      if (cols[i] < 0 || cols[j] < 0) continue;
+      const double v = B[(size_t)cols[i] * nd + cols[j]];
+      some[(size_t)i * mld + j] = v;
       amax = std::max(amax, std::fabs(v));
     }
+  const std::vector<double> &mix = mnd ? some : pad;
   sp.beta_finite = finite;
   sp.oz_beta.ready = false;
   double scale = 1.0;
