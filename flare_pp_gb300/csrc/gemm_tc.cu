@@ -118,8 +118,8 @@ k_split_gemm_grouped(const __grid_constant__ GroupedParams p) {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
 
-  // work item (one 128 x 128 tile; consecutive items share a row tile, so the
-  // CTAs running at once read each A tile from L2 rather than DRAM)
+  // work item of a CTA pair (one 256 x 128 tile; consecutive items share a row tile, so
+  // the pairs running at once read each A tile from L2 rather than DRAM)
   // -> (group, row of the operand block, first column)
   auto locate = [&](int t, int &g, int &mrow, int &n0) {
     g = 0;
