@@ -630,14 +630,15 @@ class SparseGP:
 
     def kuf_tiles(self, kernel_index=0):
         """(sparse environments per pass, threads per block) of the batched
-        Kuf launch of the last update_matrices_QR (the autotuned shape)."""
+        Kuf launch of the last update_matrices_QR (the GEMM form's gather, or the
+        adjoint form's autotuned shape)."""
         return self.kuf_launch(kernel_index)[:2]
 
     def kuf_launch(self, kernel_index=0):
         """(sparse environments per pass, threads per block, kernel ms, work
         items) of the batched Kuf launch of the last update_matrices_QR: the
-        autotuned tile shape, the CUDA-event time of the Kuf kernel alone and
-        its (structure, atom) work items."""
+        tile shape, the CUDA-event time of the Kuf kernels alone and
+        their (structure, atom) work items."""
         C = _lib.ctypes
         ks, th, ms, n = C.c_int32(), C.c_int32(), C.c_float(), C.c_int64()
         check(lib().fpp_model_kuf_tiles(self._kuf_models[kernel_index].handle, C.byref(ks),

@@ -18,9 +18,10 @@
 // index and coefficient is a compile-time constant.
 //
 // Measured at 32,000 atoms, six channels, lmax 3 (1,048,576 atoms in brackets): forward
-// 465 us (15.0 ms) in one complex kernel before, 62 + 88 us now (single bond, coupling);
-// adjoint 1240 us (40 ms) before, 281 us now, bound by issue and shared-memory latency
-// at the 12 warps per SM that its shared memory admits (28 KB of rows per three atoms);
+// 465 us (15.0 ms) in one complex kernel before, 62 + 95 us now (single bond, coupling);
+// adjoint 1240 us (40 ms) before, 279 us now, bound by latency (loads, barriers, dependent
+// multiply-adds; 43 % of the issue slots taken) at the 12 warps per SM that its registers
+// and shared memory admit (28 KB of rows per three atoms);
 // contraction 365 us (11.8 ms) before on 1904 columns, 214 us now on 1288.
 // (FP64 and lmax 0 and 4 use the complex form of b3.cuh.)
 #include <cuda_fp16.h>

@@ -724,7 +724,9 @@ int launch_ozaki_split(int rows, int K, const double *X, long long ldx, __half *
 // bn + 300 (its A digits are read and its sums drained whatever bn is).  Narrower tiles
 // pay where they add no round: 16384 x 150 x 544 with two tiles of 96 columns instead
 // of 128 takes 160 us instead of 176, 1000 x 1050 x 1050 with 68 tiles of 64 instead of
-// 36 of 128 takes 117 instead of 141.
+// 36 of 128 takes 117 instead of 141.  Over 224 shapes (M 128 to 16384, N 50 to 1500, K 144 to
+// 1500; whole calls) the choice is within 5 % of the fastest width at all but four, 13 % at
+// worst.
 static int tile_columns(const OzakiProblem *probs, int n, int pairs) {
   int best = OBN;
   long long cost = 0;

@@ -87,8 +87,9 @@ k_kuf_compact(int kc, const double *const *__restrict__ src, const int *__restri
 // per component and term with the products of c and dc).  A row waits in shared
 // memory for its largest entry, then goes out as digit planes.
 //
-// Bound by the FP64 pipe (72 % busy at 32,000 pairs, 484 us).  On the way there: bases by
-// the general recurrence 703 us; the split's digits one after the other instead of bit
+// Bound by the FP64 pipe (83 % of the active cycles at 41,600 pairs, 592 us; profiles/
+// kuf_rows_gather.txt).  On the way there, at 32,000 pairs (484 us): bases by the general
+// recurrence 703 us; the split's digits one after the other instead of bit
 // fields, and one loop over both kinds of columns, whose branch became predicated FP64
 // instructions, 664 us.
 // ---------------------------------------------------------------------------

@@ -1,6 +1,6 @@
 """FP64 mapped energies with coefficients that are large where descriptors are small (as a
 fit to scaled descriptors gives them): beta_ij = b_ij / (s_i s_j), s the mean of each
-normalised descriptor of a lattice whose small displacements make some of them 10^-8 of
+normalised descriptor of a lattice whose small displacements make some of them 10^-9 of
 the others.
 
 The energies are compared with extended-precision sums over the call's own descriptors.
@@ -8,7 +8,7 @@ With x_i = |phat_i| / s_i and |b| <= 5, the digit planes of operands scaled to t
 err by at most 2^-54 of the row's largest entry each, in K products, and the powers of two
 and the equilibration of b are within a factor of 16 of s: at most
 16 * 5 * K 2^-53 max x sum x.  (Digits relative to the largest |phat_i| and |beta_ij| err by
-up to 10^8 times as much.)  phat itself is p / |p|: 2^-52 of each product."""
+up to 10^9 times as much.)  phat itself is p / |p|: 2^-52 of each product."""
 import numpy as np
 import pytest
 
