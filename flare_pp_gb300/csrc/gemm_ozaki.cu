@@ -553,6 +553,7 @@ k_ozaki_gemm(const __grid_constant__ OzakiParams p) {
       }
     }
   }
+  if (*abort_flag) settle_in_flight();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   cluster_sync();  // the peer no longer reads, writes or signals this CTA's memory
   if (warp == 2) {

@@ -256,6 +256,7 @@ k_split_gemm_grouped(const __grid_constant__ GroupedParams p) {
       if (lane == 0) mbar_arrive_cluster(in_cta(acce_bar(buf), 0));
     }
   }
+  if (*abort_flag) settle_in_flight();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   cluster_sync();  // the peer no longer reads, writes or signals this CTA's memory
   if (warp == 2) {

@@ -77,6 +77,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   }
 }
 
+// After a wait ran out, before a CTA leaves: two milliseconds for the copies, MMAs and
+// barrier signals (a pair's go to both CTAs) that are still on their way, each of which takes
+// microseconds once issued.
+static __device__ __noinline__ void settle_in_flight() {
+  const uint64_t t0 = global_ns();
+  while (global_ns() - t0 < 2000000ull) __nanosleep(1000);
+}
+
 // Shared-memory matrix descriptor: K-major operand, 128B swizzle, 8-row core
 // groups 1024 B apart.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
